@@ -25,9 +25,11 @@ against a base address, which is what the reference planner does for its arena.
 from __future__ import annotations
 
 import abc
+import ctypes
 import dataclasses
 from collections.abc import Iterable
 
+from nano_omni_b200 import _lib
 from nano_omni_b200.core import DType, Kernel, ScratchLayout, TensorDesc, TensorKind
 from nano_omni_b200.kernels.dense_bf16 import (
     DenseBf16AttentionArguments,
@@ -184,11 +186,23 @@ class KernelSequence:
             raise ValueError(f"unsupported linear weight dtype: {weight.dtype}")
 
 
+_KEPT_PLANS = 4  # scratch addresses an operator remembers: an arena per stream, seldom more than two
+
+
+@dataclasses.dataclass(frozen=True, slots=True)
+class _Plan:
+    """The C calls of an operator against one scratch address (immutable: threads that share an operator may share it)."""
+
+    need: int
+    calls: tuple[tuple[object, tuple], ...]
+
+
 class Op(abc.ABC):
     def __init__(self, *inputs: TensorDesc, outputs: tuple[tuple[DType, tuple[int, ...]], ...]) -> None:
         self.inputs = inputs
         self.output_specs = outputs
         self.outputs: tuple[TensorDesc, ...] | None = None
+        self._plans: dict[int, _Plan] = {}
 
     def to(self, *outputs: TensorDesc):
         """Bind the outputs once; returns this operator."""
@@ -224,12 +238,33 @@ class Op(abc.ABC):
         return tuple(call.map_arguments(resolve) for call in calls)
 
     def run(self, scratch, stream: int | None = None) -> None:
-        """Submit every call on ``stream``; ``scratch`` is a CUDA uint8 tensor of at least ``prepare()[1]`` bytes."""
+        """Submit every call on ``stream``; ``scratch`` is a CUDA uint8 tensor of at least ``prepare()[1]`` bytes.
+
+        The plan is made once per scratch address and kept with the operator: its inputs, outputs and options are fixed
+        from ``to()`` on, so every later run replays the same C calls.  (Planning afresh on every run cost 60-390 us of
+        host time, more than the kernels of a small call take.)
+        """
+        base = scratch.data_ptr()
+        plan = self._plans.get(base)
+        if plan is None:
+            plan = self._plan_for(base)
+        assert scratch.numel() * scratch.element_size() >= plan.need, f"operator needs {plan.need} B of scratch"
+        stream = ctypes.c_void_p(_lib.current_stream() if stream is None else stream)
+        for function, arguments in plan.calls:
+            code = function(*arguments, stream)
+            if code != 0:
+                raise RuntimeError(f"{function.__name__}: {_lib.last_error()} (status {code})")
+
+    def _plan_for(self, base: int) -> _Plan:
         _, need = self.prepare()
-        assert scratch.numel() * scratch.element_size() >= need, f"operator needs {need} B of scratch"
-        assert scratch.data_ptr() % 256 == 0, "scratch must be 256-byte aligned"
-        for call in self.bind(scratch.data_ptr()):
-            call.submit(stream)
+        assert base % 256 == 0, "scratch must be 256-byte aligned"
+        plan = _Plan(need, tuple(call for kernel in self.bind(base) for call in kernel.recorded()))
+        plans = dict(self._plans)
+        while len(plans) >= _KEPT_PLANS:
+            del plans[next(iter(plans))]
+        plans[base] = plan
+        self._plans = plans  # replaced whole: another thread that runs this operator sees the old or the new table
+        return plan
 
     @abc.abstractmethod
     def kernels(self, scratch: ScratchLayout) -> Iterable[Kernel]:
