@@ -77,6 +77,20 @@ __device__ __forceinline__ void exp2_poly_pair(uint64_t x, float& y0, float& y1)
   y1 = __uint_as_float(__float_as_uint(p1) + (__float_as_uint(t1) << 23));
 }
 
+// The 128 accumulator columns of a warp's rows times `alpha` (each thread its row), in place.
+__device__ __forceinline__ void tmem_scale_rows(uint32_t o_addr, float alpha) {
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint32_t o[32];
+    tmem_ld32(o_addr + 32 * c, o);
+    tc_wait_ld();
+#pragma unroll
+    for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+    tmem_st32(o_addr + 32 * c, o);
+  }
+  tc_wait_st();
+}
+
 // ---- waits of the attention kernels (all 32 lanes of a converged warp call them; the result is warp-uniform)
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
   uint32_t ok;

@@ -10,17 +10,17 @@
 // (channel-major; inside every 16 tokens, stored position p holds token
 // [0,1,8,9,2,3,10,11,4,5,12,13,6,7,14,15][p]), f32 scales, output bf16 [Tq, heads*128].
 //
-// Same CTA organisation as the bf16 kernel: 256 query rows of one head per CTA (tiles A and B),
-// key tiles of 128, warps 0-3 / 4-7 softmax for A / B with one thread per row, warp 8 TMA
-// producer, warp 9 tcgen05 issuer.  QK is kind::i8 (K = 32 per MMA, 4 per tile), PV is
-// kind::f8f6f4 with P (e4m3, four keys per 32-bit TMEM column) as the TMEM operand and the
-// V tile K-major straight from TMA.  int32 scores become fp32 without a conversion
-// instruction: S + 0x4B400000 read as a float is 2^23*1.5 + S exactly.
+// CTA organisation of the bf16 kernel: 256 query rows of one head per CTA (tiles A and B), key tiles of 128, warps
+// 0-3 / 4-7 softmax for A / B with one thread per row, warp 8 TMA producer, warp 9 issues the score MMAs, warp 10 the
+// value MMAs.  QK is kind::i8 (K = 32 per MMA, 4 per tile) into ONE score buffer that A and B use in turn: it is free
+// again as soon as a tile's softmax warps hold their rows in registers, so the next scores are computed during the
+// exponentials.  PV is kind::f8f6f4 with P (e4m3, four keys per 32-bit TMEM column, two buffers per query tile) as the
+// TMEM operand and the V tile K-major straight from TMA.
+// TMEM columns: S 0-127, P_A 128-191, P_B 192-255, O_A 256-383, O_B 384-511.
+// int32 scores are converted to fp32 exactly (|S| <= 128*128*128 < 2^24) before the row maximum.
 // P is scaled by 448 / 2^3 and the running maximum is raised when it grew by more than
 // 2^3, so P never exceeds 448 (e4m3's largest finite value).
 #include <cuda.h>
-
-#include <type_traits>
 
 #include "common.cuh"
 #include "fa_common.cuh"
@@ -32,15 +32,17 @@ namespace {
 
 constexpr int kTile = 128;
 constexpr int kTileBytes = kTile * 128;  // 16 KiB: 128 rows of 128 one-byte elements
-constexpr int kStages = 6;
+constexpr int kStages = 8;
 constexpr int kThreads = 384;
 constexpr int kProducerWarp = 8;
-constexpr int kMmaWarp = 9;
+constexpr int kMmaWarp = 9;  // issues the score MMAs (S = Q K^T)
+constexpr int kPvWarp = 10;  // issues the value MMAs (O += P V)
+constexpr int kKeptScales = 8192;  // key scales (one per 64 keys) a CTA keeps in shared memory: 524288 keys
 constexpr uint32_t kTmemCols = 512;
 constexpr float kHeadroomLog2 = 3.0f;              // P <= 448 while the stale maximum lags by <= 2^3
 constexpr float kLog2PScale = 8.807354922057604f - kHeadroomLog2;  // log2(448) - 3
-constexpr uint32_t kMagicBits = 0x4B400000u;       // 12582912.0f
-constexpr float kMagic = 12582912.0f;
+
+constexpr uint32_t kColS = 0, kColP = 128, kColO = 256;  // P_t(j) at kColP + 64 t + 32 (j & 1), O_t at kColO + 128 t
 
 struct __align__(1024) Shared {
   uint8_t q[2][kTileBytes];
@@ -48,21 +50,31 @@ struct __align__(1024) Shared {
   uint64_t q_full;
   uint64_t kv_full[kStages];
   uint64_t kv_empty[kStages];
-  uint64_t s_full[2];
-  uint64_t p_full[2];
-  uint64_t o_final[2];
+  uint64_t s_full[2];      // scores of tile t are in TMEM
+  uint64_t s_taken[2];     // the softmax warps of tile t hold them in registers: the buffer is free
+  uint64_t p_full[2];      // P_t is written
+  uint64_t pv_done[2][2];  // O_t += P_t(j) V_j is complete, by parity of j: that P buffer is free, O_t may be rescaled
   uint32_t tmem_base;
   uint32_t abort;
+  float key_scale[kKeptScales];
 };
 
-// 384 threads x 168 launch registers = 64512 owned by the CTA; the split below uses exactly that.
-static_assert(256 * 224 + 128 * 56 <= 384 * 168, "setmaxnreg split exceeds the registers the CTA owns");
+// Register split after setmaxnreg: the CTA owns 384 x 168 registers; an increase beyond them would never return.
+// Every register the issuing warps can spare goes to the softmax (88 instead of 56: +4 %, 104: +8 % in time).
+constexpr int kServiceRegs = 56;
+constexpr int kSoftmaxRegs = (384 * 168 - 128 * kServiceRegs) / 256 / 8 * 8;
+static_assert(256 * kSoftmaxRegs + 128 * kServiceRegs <= 384 * 168, "setmaxnreg split exceeds the registers the CTA owns");
 
-// two e4m3 bytes: `lo` in bits 0-7, `hi` in bits 8-15
-__device__ __forceinline__ uint32_t pack_e4m3(float lo, float hi) {
-  uint16_t d;
-  asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(d) : "f"(hi), "f"(lo));
-  return d;
+// four e4m3 bytes, `a` in bits 0-7
+__device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float d) {
+  uint32_t r;
+  asm("{\n\t.reg .b16 lo, hi;\n\t"
+      "cvt.rn.satfinite.e4m3x2.f32 lo, %2, %1;\n\t"
+      "cvt.rn.satfinite.e4m3x2.f32 hi, %4, %3;\n\t"
+      "mov.b32 %0, {lo, hi};\n\t}"
+      : "=r"(r)
+      : "f"(a), "f"(b), "f"(c), "f"(d));
+  return r;
 }
 __global__ void __launch_bounds__(kThreads, 1)
 fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -87,6 +99,14 @@ fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   const int n_kv = kv_end - kv_begin;
   volatile uint32_t* abort_flag = &S.abort;
 
+  // Key scales of this CTA's keys, one per 64 keys (scales per `key_block`, 64 or 128 tokens), to shared memory: read
+  // from global memory inside the loop they cost 4 % of the kernel.
+  const int k_blocks = (num_kv_tokens + key_block - 1) / key_block;
+  const int halves_log2 = key_block == 128 ? 1 : 0;  // 64-key halves per key scale
+  const float* ks_head = key_scale + static_cast<size_t>(head) * k_blocks;
+  auto key_scale_of = [&](int half64) { return ks_head[min(half64 >> halves_log2, k_blocks - 1)]; };
+  for (int i = threadIdx.x; i < min(2 * n_kv, kKeptScales); i += kThreads) S.key_scale[i] = key_scale_of(2 * kv_begin + i);
+
   if (threadIdx.x == 0) {
     mbar_init(&S.q_full, 1);
     for (int s = 0; s < kStages; ++s) {
@@ -95,8 +115,10 @@ fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     }
     for (int t = 0; t < 2; ++t) {
       mbar_init(&S.s_full[t], 1);
+      mbar_init(&S.s_taken[t], 4);
       mbar_init(&S.p_full[t], 4);
-      mbar_init(&S.o_final[t], 1);
+      mbar_init(&S.pv_done[t][0], 1);
+      mbar_init(&S.pv_done[t][1], 1);
     }
     S.abort = 0;
     mbar_fence_init();
@@ -111,7 +133,7 @@ fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   const uint32_t tmem = S.tmem_base;
 
   if (warp >= 8) {
-    reg_dealloc<56>();
+    reg_dealloc<kServiceRegs>();
     if (warp == kProducerWarp) {
       // ------------------------------------------------------------ TMA producer
       if (lane == 0) {
@@ -146,22 +168,27 @@ fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           }
         }
       }
-    } else if (warp == kMmaWarp) {
-      // ---------------------------------------------------------- tcgen05 issuer
-      // All 32 lanes run the warp-uniform control flow; one elected lane issues (see elect_one()), one asm block per
-      // group of MMAs with ready-made 64-bit descriptors.  The waits on the probabilities are on the chain P stored ->
-      // PV -> next QK -> scores complete and poll; K / V tiles were loaded long before and their waits may sleep.
-      {
+    } else if (warp == kMmaWarp || warp == kPvWarp) {
+      // --------------------------------------------------------- tcgen05 issuers
+      // Whole warps in warp-uniform control flow, one elected lane issues a group of MMAs as one asm statement (see
+      // elect_one()).  The tensor pipe is busy less than half of the time, so the two warps issue without regard to
+      // each other.
+      // All smem operands are K-major tiles of 128 rows x 128 bytes (one swizzle atom per row).
+      const uint64_t desc = umma_smem_desc(0, 16, 1024, kSwizzle128B);
+      const uint64_t kv_desc = desc + (smem_u32(S.kv[0]) >> 4);
+      auto full_parity = [](int i) { return (uint32_t)((i / kStages) & 1); };
+      auto spin = [&](uint64_t* bar, uint32_t parity, uint32_t bit) { return warp_poll(bar, parity, abort_flag, status, bit); };
+      auto rest = [&](uint64_t* bar, uint32_t parity, uint32_t bit) { return warp_rest(bar, parity, abort_flag, status, bit); };
+      if (warp == kMmaWarp) {
         constexpr uint32_t idesc_qk = umma_idesc(kDS32, kFmtS8, kFmtS8, 0, 0, kTile, kTile);
-        constexpr uint32_t idesc_pv = umma_idesc(kDF32, kFmtE4M3, kFmtE4M3, 0, 0, kTile, 128);
-        // All three smem operands are K-major tiles of 128 rows x 128 bytes (one swizzle atom per row).
-        const uint64_t desc = umma_smem_desc(0, 16, 1024, kSwizzle128B);
         const uint64_t q_desc[2] = {desc + (smem_u32(S.q[0]) >> 4), desc + (smem_u32(S.q[1]) >> 4)};
-        const uint64_t kv_desc = desc + (smem_u32(S.kv[0]) >> 4);
-        // S_t = Q_t K^T: four MMAs of 32 channels (32 bytes of a row = 2 descriptor units), then the commits
-        auto issue_qk = [&](int t, int st, bool last_reader) {
-          const uint64_t a = q_desc[t], b = kv_desc + st * (kTileBytes >> 4);
-          const uint32_t d = tmem + t * kTile;
+        // S = Q_t K_j^T: four MMAs of 32 channels (32 bytes of a row = 2 descriptor units), then the commits
+        auto qk = [&](int t, int j, uint64_t* taken, uint32_t taken_parity) -> bool {
+          const int ik = 2 * j, sk = ik % kStages;
+          const uint64_t a = t ? q_desc[1] : q_desc[0], b = kv_desc + sk * (kTileBytes >> 4);
+          if (t == 0 && !rest(&S.kv_full[sk], full_parity(ik), kWaitTimeoutLoad)) return false;
+          if (taken && !spin(taken, taken_parity, kWaitTimeoutSoftmax)) return false;  // last: the critical hand-over
+          tc_fence_after();
           if (elect_one()) {
             asm volatile(
                 "{\n\t.reg .pred p0, p1;\n\t"
@@ -169,17 +196,29 @@ fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 "tcgen05.mma.cta_group::1.kind::i8 [%0], %2, %6, %1, p0;\n\t"
                 "tcgen05.mma.cta_group::1.kind::i8 [%0], %3, %7, %1, p1;\n\t"
                 "tcgen05.mma.cta_group::1.kind::i8 [%0], %4, %8, %1, p1;\n\t"
-                "tcgen05.mma.cta_group::1.kind::i8 [%0], %5, %9, %1, p1;\n\t}" ::"r"(d),
+                "tcgen05.mma.cta_group::1.kind::i8 [%0], %5, %9, %1, p1;\n\t}" ::"r"(tmem + kColS),
                 "r"(idesc_qk), "l"(a), "l"(a + 2), "l"(a + 4), "l"(a + 6), "l"(b), "l"(b + 2), "l"(b + 4), "l"(b + 6)
                 : "memory");
             tc_commit(&S.s_full[t]);
-            if (last_reader) tc_commit(&S.kv_empty[st]);
+            if (t == 1 || !two) tc_commit(&S.kv_empty[sk]);  // last reader of K_j
           }
+          return true;
         };
-        // O_t += P_t V: four MMAs of 32 keys (32 bytes of a V row; 8 TMEM columns of P), then the commits
-        auto issue_pv = [&](int t, int st, bool accumulate, bool last_reader, bool final) {
-          const uint64_t b = kv_desc + st * (kTileBytes >> 4);
-          const uint32_t d = tmem + 256 + t * kTile, a = tmem + t * kTile;
+        bool ok = rest(&S.q_full, 0, kWaitTimeoutLoad) && qk(0, 0, nullptr, 0);
+        for (int j = 0; ok && j < n_kv; ++j) {
+          if (two && !(ok = qk(1, j, &S.s_taken[0], j & 1))) break;
+          if (j + 1 < n_kv && !(ok = qk(0, j + 1, &S.s_taken[two ? 1 : 0], j & 1))) break;
+        }
+      } else {
+        constexpr uint32_t idesc_pv = umma_idesc(kDF32, kFmtE4M3, kFmtE4M3, 0, 0, kTile, 128);
+        // O_t += P_t(j) V_j: four MMAs of 32 keys (32 bytes of a V row; 8 columns of P), then the commits
+        auto pv = [&](int t, int j) -> bool {
+          const int iv = 2 * j + 1, sv = iv % kStages;
+          const uint64_t b = kv_desc + sv * (kTileBytes >> 4);
+          const uint32_t d = tmem + kColO + t * kTile, a = tmem + kColP + t * 64 + (j & 1) * 32;
+          if (t == 0 && !rest(&S.kv_full[sv], full_parity(iv), kWaitTimeoutLoad)) return false;
+          if (!spin(&S.p_full[t], j & 1, kWaitTimeoutSoftmax)) return false;
+          tc_fence_after();
           if (elect_one()) {
             asm volatile(
                 "{\n\t.reg .pred p0, p1;\n\t"
@@ -188,189 +227,143 @@ fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%4], %8, %1, p1;\n\t"
                 "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%5], %9, %1, p1;\n\t"
                 "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%6], %10, %1, p1;\n\t}" ::"r"(d),
-                "r"(idesc_pv), "r"(accumulate ? 1u : 0u), "r"(a), "r"(a + 8), "r"(a + 16), "r"(a + 24), "l"(b), "l"(b + 2),
+                "r"(idesc_pv), "r"(j > 0 ? 1u : 0u), "r"(a), "r"(a + 8), "r"(a + 16), "r"(a + 24), "l"(b), "l"(b + 2),
                 "l"(b + 4), "l"(b + 6)
                 : "memory");
-            if (last_reader) tc_commit(&S.kv_empty[st]);
-            if (final) tc_commit(&S.o_final[t]);
+            tc_commit(&S.pv_done[t][j & 1]);
+            if (t == 1 || !two) tc_commit(&S.kv_empty[sv]);  // last reader of V_j
           }
+          return true;
         };
-        auto full_parity = [](int i) { return (uint32_t)((i / kStages) & 1); };
-        auto rest = [&](uint64_t* bar, uint32_t parity, uint32_t bit) { return warp_rest(bar, parity, abort_flag, status, bit); };
-        auto spin = [&](uint64_t* bar, uint32_t parity, uint32_t bit) { return warp_poll(bar, parity, abort_flag, status, bit); };
-
-        bool ok = rest(&S.q_full, 0, kWaitTimeoutLoad) && rest(&S.kv_full[0], 0, kWaitTimeoutLoad);
-        if (ok) {
-          tc_fence_after();
-          issue_qk(0, 0, !two);
-          if (two) issue_qk(1, 0, true);
-        }
-        for (int j = 0; ok && j < n_kv; ++j) {
-          const int iv = 2 * j + 1, ik = 2 * j + 2;
-          const int sv = iv % kStages, sk = ik % kStages;
-          const bool more = j + 1 < n_kv;
-          if (!(ok = rest(&S.kv_full[sv], full_parity(iv), kWaitTimeoutLoad))) break;
-          if (more && !(ok = rest(&S.kv_full[sk], full_parity(ik), kWaitTimeoutLoad))) break;
-          if (!(ok = spin(&S.p_full[0], j & 1, kWaitTimeoutSoftmax))) break;
-          tc_fence_after();
-          issue_pv(0, sv, j > 0, !two, !more);
-          if (more) issue_qk(0, sk, !two);
-          if (two) {
-            if (!(ok = spin(&S.p_full[1], j & 1, kWaitTimeoutSoftmax))) break;
-            tc_fence_after();
-            issue_pv(1, sv, j > 0, true, !more);
-            if (more) issue_qk(1, sk, true);
-          }
-        }
+        bool ok = true;
+        for (int j = 0; ok && j < n_kv; ++j) ok = pv(0, j) && (!two || pv(1, j));
       }
     }
   } else {
     // ------------------------------------------------- softmax + epilogue warps
-    reg_alloc<224>();
+    reg_alloc<kSoftmaxRegs>();
+    auto poll = [&](uint64_t* bar, uint32_t parity, uint32_t bit) { return warp_poll(bar, parity, abort_flag, status, bit); };
     const int t = warp >> 2;
     if (t == 0 || two) {
       const int row = (warp & 3) * 32 + lane;
       const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-      const uint32_t s_addr = tmem + lane_base + t * kTile;
-      const uint32_t o_addr = tmem + lane_base + 256 + t * kTile;
+      const uint32_t s_addr = tmem + lane_base + kColS;
+      const uint32_t p_addr = tmem + lane_base + kColP + t * 64;
+      const uint32_t o_addr = tmem + lane_base + kColO + t * kTile;
       const int token = q0 + t * kTile + row;
-      // scales per `query_block` (32, 64 or 128) query tokens and per `key_block` (64 or 128) key tokens
+      // per-row factor: query scale of the row's block (32, 64 or 128 tokens) times log2e/sqrt(128)
       const int q_blocks = (num_query_tokens + query_block - 1) / query_block;
-      const int k_blocks = (num_kv_tokens + key_block - 1) / key_block;
-      const int per_half = key_block / 64;  // 64-key halves per key scale
-      // per-row factor: query scale of the row's block times log2e/sqrt(128)
       const float qf = query_scale[static_cast<size_t>(head) * q_blocks + min(token / query_block, q_blocks - 1)] * scale_log2;
-      const float* ks_head = key_scale + static_cast<size_t>(head) * k_blocks;
-      float m_used = 0.f, l0 = 0.f, l1 = 0.f, l2 = 0.f, l3 = 0.f;
+      float m_used = 0.f;
+      uint64_t la = 0ull, lb = 0ull;  // four partial row sums as two fp32 pairs
       bool ok = true;
       for (int j = 0; j < n_kv; ++j) {
-        // factors of the two 64-key blocks of this tile (0 for a block past the end: fully masked below)
         const int jt = kv_begin + j;  // key tile in the whole sequence
-        const float f0 = qf * ks_head[(2 * jt) / per_half];
-        const float f1 = ((2 * jt + 1) / per_half < k_blocks) ? qf * ks_head[(2 * jt + 1) / per_half] : 0.f;
-        ok = warp_poll(&S.s_full[t], j & 1, abort_flag, status, kWaitTimeoutMma);  // on the chain: poll
+        float ks0, ks1;
+        if (2 * j + 1 < kKeptScales) {
+          ks0 = S.key_scale[2 * j], ks1 = S.key_scale[2 * j + 1];
+        } else {
+          ks0 = key_scale_of(2 * jt), ks1 = key_scale_of(2 * jt + 1);
+        }
+        ok = poll(&S.s_full[t], j & 1, kWaitTimeoutMma);
         if (!ok) break;
         tc_fence_after();
         uint32_t s[128];
 #pragma unroll
         for (int cc = 0; cc < 4; ++cc) tmem_ld32(s_addr + 32 * cc, *reinterpret_cast<uint32_t(*)[32]>(&s[32 * cc]));
         tc_wait_ld();
-        // int32 -> the float 2^23*1.5 + S (exact for |S| < 2^22; |S| <= 128*128*127 here)
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&S.s_taken[t]);
+        // PV(j-2) read the P buffer of this tile: looked at early, so that the answer is there when P is stored
+        bool p_free = j < 2 || mbar_test(&S.pv_done[t][j & 1], ((j - 2) >> 1) & 1);
 #pragma unroll
-        for (int i = 0; i < 128; ++i) s[i] += kMagicBits;
+        for (int i = 0; i < 128; ++i) s[i] = __float_as_uint(static_cast<float>(static_cast<int>(s[i])));
         const int valid = num_kv_tokens - jt * kTile;  // keys of this tile that exist (>= 1)
-        float a0 = __uint_as_float(s[0]), a1 = __uint_as_float(s[64]);
-        if (valid >= kTile) {
+        if (valid < kTile) {
 #pragma unroll
-          for (int i = 1; i < 63; i += 2) {
-            a0 = max3(a0, __uint_as_float(s[i]), __uint_as_float(s[i + 1]));
-            a1 = max3(a1, __uint_as_float(s[64 + i]), __uint_as_float(s[64 + i + 1]));
-          }
-          a0 = fmaxf(a0, __uint_as_float(s[63]));
-          a1 = fmaxf(a1, __uint_as_float(s[127]));
-        } else {
-          a0 = -INFINITY, a1 = -INFINITY;
-#pragma unroll
-          for (int i = 0; i < 64; ++i) {
-            if (i < valid) a0 = fmaxf(a0, __uint_as_float(s[i]));
-            if (64 + i < valid) a1 = fmaxf(a1, __uint_as_float(s[64 + i]));
-          }
+          for (int i = 0; i < 128; ++i)
+            if (i >= valid) s[i] = 0xff800000u;  // -inf
         }
-        float mx = (a0 - kMagic) * f0;
-        if (valid > 64) mx = fmaxf(mx, (a1 - kMagic) * f1);
+        float a0 = __uint_as_float(s[0]), a1 = __uint_as_float(s[64]), a2 = __uint_as_float(s[1]), a3 = __uint_as_float(s[65]);
+#pragma unroll
+        for (int i = 2; i < 62; i += 4) {
+          a0 = max3(a0, __uint_as_float(s[i]), __uint_as_float(s[i + 1]));
+          a1 = max3(a1, __uint_as_float(s[64 + i]), __uint_as_float(s[64 + i + 1]));
+          a2 = max3(a2, __uint_as_float(s[i + 2]), __uint_as_float(s[i + 3]));
+          a3 = max3(a3, __uint_as_float(s[64 + i + 2]), __uint_as_float(s[64 + i + 3]));
+        }
+        a0 = max3(a0, a2, fmaxf(__uint_as_float(s[62]), __uint_as_float(s[63])));
+        a1 = max3(a1, a3, fmaxf(__uint_as_float(s[126]), __uint_as_float(s[127])));
+        // factors of the two 64-key halves, kept positive so that the -inf of a key past the end stays -inf under them
+        const float f0 = fmaxf(qf * ks0, 1e-30f), f1 = fmaxf(qf * ks1, 1e-30f);
+        const float mx = fmaxf(a0 * f0, a1 * f1);
         if (j == 0) {
           m_used = mx;
         } else if (__any_sync(0xffffffffu, mx > m_used + kHeadroomLog2)) {
           const float m_new = fmaxf(m_used, mx);
           const float alpha = ex2(m_used - m_new);
-          l0 *= alpha, l1 *= alpha, l2 *= alpha, l3 *= alpha;
-          // S_t(j) is complete, hence so is O_t += P_t V_{j-1}; the next PV waits for our arrival.
-#pragma unroll
-          for (int cc = 0; cc < 4; ++cc) {
-            uint32_t o[32];
-            tmem_ld32(o_addr + 32 * cc, o);
-            tc_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-            tmem_st32(o_addr + 32 * cc, o);
-          }
-          tc_wait_st();
+          const uint64_t alpha2 = pack2(alpha, alpha);
+          la = mul2(la, alpha2);
+          lb = mul2(lb, alpha2);
+          // O_t += P_t V_{j-1} must have completed; the next PV waits for our arrival on p_full.
+          ok = poll(&S.pv_done[t][(j - 1) & 1], ((j - 1) >> 1) & 1, kWaitTimeoutMma);
+          if (!ok) break;
+          p_free = true;
+          tc_fence_after();
+          tmem_scale_rows(o_addr, alpha);
           m_used = m_new;
         }
-        // x = ((2^23*1.5 + S) - 2^23*1.5) * f - (m - log2(448/8)).  The subtraction is exact; folding 2^23*1.5 * f
-        // into the constant instead would round it to that product's ulp, an error of up to 4 % in P for scales near 1.
-        const float cst = m_used - kLog2PScale;
-        uint32_t p[32];
-        if (valid >= kTile) {
-          // full tile: packed fp32 pairs; four partial row sums live in two register pairs
-          uint64_t la = pack2(l0, l1), lb = pack2(l2, l3);
-          // Folding 2^23*1.5 * f into the FMA constant saves the subtraction but rounds the constant to half an ulp of
-          // that product; taken only while this stays below 2^-11 in the exponent (0.03 % in P).  f is the same for
-          // the 32 rows of a warp (one query-scale block), so the branch does not diverge.
-          auto exponentials = [&](auto fold_tag) {
-            constexpr bool kFold = decltype(fold_tag)::value;
-            const float c0 = kFold ? fmaf(kMagic, f0, cst) : cst, c1 = kFold ? fmaf(kMagic, f1, cst) : cst;
-            const uint64_t nm2 = pack2(-kMagic, -kMagic);
+        const float cst = kLog2PScale - m_used;
+        const uint64_t f2[2] = {pack2(f0, f0), pack2(f1, f1)}, cst2 = pack2(cst, cst);
+        // Groups of 16 keys, the exponentials of a group ahead of the sums and conversions of the one before: the
+        // special-function unit does not drain while a group is packed.
+        float e[2][16];
+        auto exponentials = [&](int g) {
 #pragma unroll
-            for (int g = 0; g < 8; ++g) {  // groups of 16 keys; stored order inside a group: 0,1,8,9 | 2,3,10,11 | ...
-              const uint64_t f2 = g < 4 ? pack2(f0, f0) : pack2(f1, f1);
-              const uint64_t nc2 = g < 4 ? pack2(-c0, -c0) : pack2(-c1, -c1);
-              float e[16];
-#pragma unroll
-              for (int i = 0; i < 16; i += 2) {
-                float x0, x1;
-                uint64_t sv = pack2(__uint_as_float(s[16 * g + i]), __uint_as_float(s[16 * g + i + 1]));
-                if (!kFold) sv = add2(sv, nm2);
-                unpack2(fma2(sv, f2, nc2), x0, x1);
-                e[i] = ex2(x0);
-                e[i + 1] = ex2(x1);
-              }
-#pragma unroll
-              for (int i = 0; i < 16; i += 4) {
-                la = add2(la, pack2(e[i], e[i + 1]));
-                lb = add2(lb, pack2(e[i + 2], e[i + 3]));
-              }
-#pragma unroll
-              for (int w = 0; w < 4; ++w)
-                p[4 * g + w] = pack_e4m3(e[2 * w], e[2 * w + 1]) | (pack_e4m3(e[8 + 2 * w], e[8 + 2 * w + 1]) << 16);
-            }
-          };
-          if (fmaxf(f0, f1) * kMagic < 16384.0f) {
-            exponentials(std::true_type{});
-          } else {
-            exponentials(std::false_type{});
+          for (int i = 0; i < 16; i += 2) {
+            float x0, x1;
+            unpack2(fma2(pack2(__uint_as_float(s[16 * g + i]), __uint_as_float(s[16 * g + i + 1])), f2[g >> 2], cst2), x0, x1);
+            e[g & 1][i] = ex2(x0);
+            e[g & 1][i + 1] = ex2(x1);
           }
-          unpack2(la, l0, l1);
-          unpack2(lb, l2, l3);
-        } else {
+        };
+        exponentials(0);
+        uint32_t p[32];
 #pragma unroll
-          for (int g = 0; g < 8; ++g) {
-            float e[16];
-            const float f = g < 4 ? f0 : f1;
+        for (int g = 0; g < 8; ++g) {
+          if (g < 7) exponentials(g + 1);
+          const float* x = e[g & 1];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              float x = fmaf(__uint_as_float(s[16 * g + i]) - kMagic, f, -cst);
-              if (16 * g + i >= valid) x = -INFINITY;
-              e[i] = ex2(x);
+          for (int i = 0; i < 16; i += 4) {
+            la = add2(la, pack2(x[i], x[i + 1]));
+            lb = add2(lb, pack2(x[i + 2], x[i + 3]));
+          }
+          // stored order inside a group: 0,1,8,9 | 2,3,10,11 | ...
+#pragma unroll
+          for (int w = 0; w < 4; ++w) p[4 * g + w] = pack_e4m3x4(x[2 * w], x[2 * w + 1], x[8 + 2 * w], x[8 + 2 * w + 1]);
+          if (g == 3) {
+            if (!__all_sync(0xffffffffu, p_free)) {
+              ok = poll(&S.pv_done[t][j & 1], ((j - 2) >> 1) & 1, kWaitTimeoutMma);
+              if (!ok) break;
             }
-#pragma unroll
-            for (int i = 0; i < 16; i += 4) {
-              l0 += e[i], l1 += e[i + 1], l2 += e[i + 2], l3 += e[i + 3];
-            }
-#pragma unroll
-            for (int w = 0; w < 4; ++w)
-              p[4 * g + w] = pack_e4m3(e[2 * w], e[2 * w + 1]) | (pack_e4m3(e[8 + 2 * w], e[8 + 2 * w + 1]) << 16);
+            tc_fence_after();
+            tmem_st16(p_addr + 32 * (j & 1), p);
           }
         }
-        tmem_st32(s_addr, p);
+        if (!ok) break;
+        tmem_st16(p_addr + 32 * (j & 1) + 16, p + 16);
         tc_wait_st();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&S.p_full[t]);
       }
-      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&S.o_final[t], 0, abort_flag, status, kWaitTimeoutMma));
+      if (ok) ok = poll(&S.pv_done[t][(n_kv - 1) & 1], ((n_kv - 1) >> 1) & 1, kWaitTimeoutMma);
       if (ok) {
         tc_fence_after();
+        float l0, l1, l2, l3;
+        unpack2(la, l0, l1);
+        unpack2(lb, l2, l3);
         const float l = (l0 + l1) + (l2 + l3);
         const float inv = 1.0f / l;
         const float* vs = value_scale + head * 128;
