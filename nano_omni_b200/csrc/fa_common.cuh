@@ -91,6 +91,26 @@ __device__ __forceinline__ void tmem_scale_rows(uint32_t o_addr, float alpha) {
   tc_wait_st();
 }
 
+// The same with all loads in flight at once, for a place where a tile's scores are no longer live in registers.
+__device__ __forceinline__ void tmem_scale_rows_wide(uint32_t o_addr, float alpha) {
+  uint32_t o[4][32];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) tmem_ld32(o_addr + 32 * c, o[c]);
+  tc_wait_ld();
+  const uint64_t alpha2 = pack2(alpha, alpha);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) {
+      float x, y;
+      unpack2(mul2(pack2(__uint_as_float(o[c][i]), __uint_as_float(o[c][i + 1])), alpha2), x, y);
+      o[c][i] = __float_as_uint(x), o[c][i + 1] = __float_as_uint(y);
+    }
+    tmem_st32(o_addr + 32 * c, o[c]);
+  }
+  tc_wait_st();
+}
+
 // ---- waits of the attention kernels (all 32 lanes of a converged warp call them; the result is warp-uniform)
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
   uint32_t ok;

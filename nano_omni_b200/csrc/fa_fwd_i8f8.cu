@@ -52,7 +52,7 @@ struct __align__(1024) Shared {
   uint64_t kv_empty[kStages];
   uint64_t s_full[2];      // scores of tile t are in TMEM
   uint64_t s_taken[2];     // the softmax warps of tile t hold them in registers: the buffer is free
-  uint64_t p_full[2];      // P_t is written
+  uint64_t p_full[2][2];   // P_t(j) is written, by parity of j (the softmax may run a tile ahead of the value issuer)
   uint64_t pv_done[2][2];  // O_t += P_t(j) V_j is complete, by parity of j: that P buffer is free, O_t may be rescaled
   uint32_t tmem_base;
   uint32_t abort;
@@ -116,7 +116,8 @@ fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     for (int t = 0; t < 2; ++t) {
       mbar_init(&S.s_full[t], 1);
       mbar_init(&S.s_taken[t], 4);
-      mbar_init(&S.p_full[t], 4);
+      mbar_init(&S.p_full[t][0], 4);
+      mbar_init(&S.p_full[t][1], 4);
       mbar_init(&S.pv_done[t][0], 1);
       mbar_init(&S.pv_done[t][1], 1);
     }
@@ -217,7 +218,7 @@ fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           const uint64_t b = kv_desc + sv * (kTileBytes >> 4);
           const uint32_t d = tmem + kColO + t * kTile, a = tmem + kColP + t * 64 + (j & 1) * 32;
           if (t == 0 && !rest(&S.kv_full[sv], full_parity(iv), kWaitTimeoutLoad)) return false;
-          if (!spin(&S.p_full[t], j & 1, kWaitTimeoutSoftmax)) return false;
+          if (!spin(&S.p_full[t][j & 1], (j >> 1) & 1, kWaitTimeoutSoftmax)) return false;
           tc_fence_after();
           if (elect_one()) {
             asm volatile(
@@ -356,7 +357,7 @@ fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         tc_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&S.p_full[t]);
+        if (lane == 0) mbar_arrive(&S.p_full[t][j & 1]);
       }
       if (ok) ok = poll(&S.pv_done[t][(n_kv - 1) & 1], ((n_kv - 1) >> 1) & 1, kWaitTimeoutMma);
       if (ok) {

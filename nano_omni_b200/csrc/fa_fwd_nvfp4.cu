@@ -10,17 +10,22 @@
 //                      operands from shared memory (64-byte rows, 64-byte swizzle), scale factors copied from the
 //                      atoms to TMEM with tcgen05.cp, fp32 scores in TMEM
 //   softmax            one thread per query row; running maximum in raw q.k units raised with every key tile (exact,
-//                      as the reference does per key block: dense_nvfp4.py:250-266, sol_nvfp4.py:793-803), probabilities
-//                      p = exp2((s - m) log2e/sqrt(128) + log2(2688)), row sum of the unrounded p
+//                      as the reference does per key block: dense_nvfp4.py:250-266, sol_nvfp4.py:793-803), row sum of the
+//                      unrounded probabilities p = 2^((s - m) log2e/sqrt(128)) * 2688
 //   P -> e2m1          per 16 keys: scale = max p / 6, stored as ue4m3; codes = round(p / scale) on the e2m1 grid
-//                      (dense_nvfp4.py:255-289; arithmetic of sol_nvfp4.py:764-781); eight codes per 32-bit TMEM column,
-//                      the row's four scales of a 64-key step in one column of the row's lane quadrant
+//                      (dense_nvfp4.py:255-289; arithmetic of sol_nvfp4.py:764-781), both taken from the group's largest
+//                      score instead of from p; eight codes per 32-bit TMEM column, the row's four scales of a 64-key
+//                      step in one column of the row's lane quadrant
 //   O += P4 V4         the same block-scaled MMA with P (and its scales) read from TMEM, V K-major from shared memory
 //
 // CTA organisation as the bf16 kernel: 256 query rows of one head (tiles A and B), one score buffer used by A and B in
 // turn, warps 0-3 / 4-7 softmax for A / B, warp 8 TMA producer, warp 9 issues the score MMAs, warp 10 the value MMAs.
-// TMEM columns: S 0-127, P_A 128-143, P_B 144-159, scales of P_A 160-167, P_B 168-175, Q_A 176-183, Q_B 184-191,
-// K 192-199, V 200-207, O_A 256-383, O_B 384-511.
+// Bound by the softmax warps (the tensor pipe has 512 of about 3300 cycles per pair of tiles to do): P and its scales
+// are double-buffered and handed over once per tile, the two issuers run without order between them, O is rescaled
+// after the exponentials.  20011 tokens x 24 heads: 4.71 -> 3.48 ms; 16 % of the 64-key blocks of 32768 x 24: 3.62 ->
+// 3.23 ms (before: P divided by its scale, single buffers, two hand-overs, rescale ahead of the exponentials).
+// TMEM columns: S 0-127, P_A 128-159, P_B 160-191 (two buffers each), scales of P_A 192-207, P_B 208-223 (two buffers
+// each), of Q_A 224-231, Q_B 232-239, K 240-247, V 248-255, O_A 256-383, O_B 384-511.
 //
 // kSol: each query tile visits only the 64-key blocks that one of its two 64-row query blocks selects (mask u8
 // [query blocks, heads, key blocks] of 64-token blocks; key block 0 always attends), so tiles A and B walk lists of
@@ -40,10 +45,6 @@
 #include "tensor_map.cuh"
 #include "../../include/nano_omni_b200.h"
 
-#ifndef NOB200_PFULL_WAIT
-#define NOB200_PFULL_WAIT spin
-#endif
-
 namespace nob200 {
 namespace {
 
@@ -57,12 +58,15 @@ constexpr int kMmaWarp = 9;
 constexpr int kPvWarp = 10;
 constexpr uint32_t kTmemCols = 512;
 constexpr int kMaxTiles = 4096;  // list entries of a sol query tile: 64-key blocks (262144 keys)
-constexpr float kLog2PScale = 11.39231742277876f;  // log2(6 * 448)
+constexpr float kLog2BlockScale = 8.807354922057604f;  // log2(448): the block scale of the row maximum's group
+constexpr float kLog2Six = 2.584962500721156f;
 constexpr float kInvPScale = 1.0f / 2688.0f;
 
-constexpr uint32_t kColS = 0, kColP = 128, kColSfP = 160, kColSfQ = 176, kColSfK = 192, kColSfV = 200, kColO = 256;
+// P_t(i) at kColP + 32 t + 16 (i & 1), its scales at kColSfP + 16 t + 8 (i & 1), scales of Q_t at kColSfQ + 8 t, O_t at
+// kColO + 128 t
+constexpr uint32_t kColS = 0, kColP = 128, kColSfP = 192, kColSfQ = 224, kColSfK = 240, kColSfV = 248, kColO = 256;
 
-constexpr int kServiceRegs = 88;
+constexpr int kServiceRegs = 56;
 constexpr int kSoftmaxRegs = (384 * 168 - 128 * kServiceRegs) / 256 / 8 * 8;
 static_assert(256 * kSoftmaxRegs + 128 * kServiceRegs <= 384 * 168, "setmaxnreg split exceeds the registers the CTA owns");
 
@@ -76,12 +80,12 @@ struct __align__(1024) Shared {
   uint64_t kv_empty[kStages];
   uint64_t s_full[2];
   uint64_t s_taken[2];
-  uint64_t p_full[2][2];
-  uint64_t pv_done[2];
+  uint64_t p_full[2][2];   // P_t(i) and its scales are written, by parity of i (the softmax may run a step ahead of the
+                           // value issuer)
+  uint64_t pv_done[2][2];  // O_t += P_t(i) V is complete, by parity of i: that P buffer is free, O_t may be rescaled
   uint64_t list_ready;
   uint32_t tmem_base;
   uint32_t abort;
-  uint32_t qk_issued;
   int list_len[2];
   uint16_t list[2][kMaxTiles];
   uint8_t flags[2][kMaxTiles];  // bit (query block inside the tile): that query block selected the key block
@@ -173,11 +177,11 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       mbar_init(&S.s_taken[t], 4);
       mbar_init(&S.p_full[t][0], 4);
       mbar_init(&S.p_full[t][1], 4);
-      mbar_init(&S.pv_done[t], 1);
+      mbar_init(&S.pv_done[t][0], 1);
+      mbar_init(&S.pv_done[t][1], 1);
     }
     mbar_init(&S.list_ready, 1);
     S.abort = 0;
-    S.qk_issued = 0;
     S.list_len[0] = S.list_len[1] = 0;
     mbar_fence_init();
   }
@@ -316,7 +320,6 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       if (warp == kMmaWarp) {
         const uint64_t q_desc[2] = {desc + (smem_u32(S.q[0]) >> 4), desc + (smem_u32(S.q[1]) >> 4)};
         const uint64_t kv_desc = desc + (smem_u32(S.kv[0]) >> 4);
-        uint32_t issued = 0;
         // S = Q_t K^T with the K tile of ring unit u; `first` reader waits for the tile and copies its scales,
         // `last` reader releases the stage
         // `block`: the 64-key block of a sol entry (its K scales are rows 64 (block & 1) .. of the tile's atoms: two
@@ -344,9 +347,7 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 : "memory");
             tc_commit(&S.s_full[t]);
             if (last) tc_commit(&S.kv_empty[sk]);
-            *reinterpret_cast<volatile uint32_t*>(&S.qk_issued) = issued + 1;
           }
-          ++issued;
           return true;
         };
         ok = ok && groups > 0 && rest(&S.q_full, 0, kWaitTimeoutLoad);
@@ -376,50 +377,50 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         }
       } else {
         const uint64_t kv_desc = desc + (smem_u32(S.kv[0]) >> 4);
-        // O_t += P_t(i)[:, 64 half ...] V[...] with the V tile of ring unit u: one MMA of K = 64, after `gate`
-        // score groups were issued
-        auto pv_half = [&](int t, int i, int u, int half, bool first, bool last, uint32_t gate) -> bool {
+        // O_t += P_t(i) V with the V tile of ring unit u: one MMA of K = 64 per 64 keys.  `first` reader waits for the
+        // tile and copies its scales ahead of the MMAs (same pipe, in order), `last` reader releases the stage.
+        auto pv = [&](int t, int i, int u, bool first, bool last) -> bool {
           const int iv = 2 * u + 1, sv = iv % kStages;
-          const uint64_t b = kv_desc + sv * (kTileBytes >> 4) + half * 2;  // 64 keys = 32 bytes of a channel's row
-          const uint32_t accumulate = (i > 0 || half > 0) ? 1u : 0u;
-          if (gate > static_cast<uint32_t>(groups)) gate = groups;
-          if (half == 0 && !rest(&S.kv_full[sv], full_parity(iv), kWaitTimeoutLoad)) return false;
-          if (!NOB200_PFULL_WAIT(&S.p_full[t][half], i & 1, kWaitTimeoutSoftmax)) return false;
-          if (!warp_wait_counter(&S.qk_issued, gate, abort_flag, status, kWaitTimeoutMma)) return false;
+          const uint64_t b = kv_desc + sv * (kTileBytes >> 4);  // 64 keys = 32 bytes of a channel's row
+          const uint32_t d = tmem + kColO + t * kTile, a = tmem + kColP + 32 * t + 16 * (i & 1);
+          const uint32_t sf = tmem + kColSfP + 16 * t + 8 * (i & 1);
+          if (first && !rest(&S.kv_full[sv], full_parity(iv), kWaitTimeoutLoad)) return false;
+          if (!spin(&S.p_full[t][i & 1], (i >> 1) & 1, kWaitTimeoutSoftmax)) return false;
           tc_fence_after();
           if (elect_one()) {
-            if (first && half == 0) {  // the value tile's scales, ahead of its first MMA
+            if (first) {
               cp_scale_atom(tmem + kColSfV, smem_u32(S.kv_sf[sv]));
               if (!kSol) cp_scale_atom(tmem + kColSfV + 4, smem_u32(S.kv_sf[sv]) + 512);
             }
-            asm volatile(
-                "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], [%1], %2, %3, [%5], [%6], p;\n\t}" ::"r"(
-                    tmem + kColO + t * kTile),
-                "r"(tmem + kColP + 16 * t + 8 * half), "l"(b), "r"(kIdesc), "r"(accumulate),
-                "r"(tmem + kColSfP + 8 * t + 4 * half), "r"(tmem + kColSfV + 4 * half)
-                : "memory");
-            if (kSol || half == 1) {
-              tc_commit(&S.pv_done[t]);
-              if (last) tc_commit(&S.kv_empty[sv]);
+            if (kSol) {  // an entry is 64 keys: one MMA
+              asm volatile(
+                  "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                  "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], [%1], %2, %3, [%5], [%6], p;\n\t}" ::"r"(d),
+                  "r"(a), "l"(b), "r"(kIdesc), "r"(i > 0 ? 1u : 0u), "r"(sf), "r"(tmem + kColSfV)
+                  : "memory");
+            } else {
+              asm volatile(
+                  "{\n\t.reg .pred p0, p1;\n\tsetp.ne.b32 p0, %4, 0;\n\tsetp.eq.b32 p1, 0, 0;\n\t"
+                  "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], [%1], %2, %3, [%5], [%6], p0;\n\t"
+                  "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], [%7], %8, %3, [%9], [%10], p1;\n\t}" ::"r"(d),
+                  "r"(a), "l"(b), "r"(kIdesc), "r"(i > 0 ? 1u : 0u), "r"(sf), "r"(tmem + kColSfV), "r"(a + 8), "l"(b + 2),
+                  "r"(sf + 4), "r"(tmem + kColSfV + 4)
+                  : "memory");
             }
+            tc_commit(&S.pv_done[t][i & 1]);
+            if (last) tc_commit(&S.kv_empty[sv]);
           }
           return true;
         };
         if (kSol) {
-          // a group's value MMAs wait until the next score group is in the pipe (the one its score take released)
           int next[2] = {0, 0};
           for (int g = 0; ok && g < groups; ++g) {
             const int t = next_tile(next), i = next[t]++;
-            ok = pv_half(t, i, g, 0, true, true, g + 2);  // an entry is 64 keys: one MMA
-          }
-        } else if (n_b > 0) {
-          for (int i = 0; ok && i < n_a; ++i) {
-            ok = pv_half(0, i, i, 0, true, false, 2 * i + 3) && pv_half(0, i, i, 1, true, false, 2 * i + 4) &&
-                 pv_half(1, i, i, 0, false, true, 2 * i + 4) && pv_half(1, i, i, 1, false, true, 2 * i + 5);
+            ok = pv(t, i, g, true, true);
           }
         } else {
-          for (int i = 0; ok && i < n_a; ++i) ok = pv_half(0, i, i, 0, true, true, i + 2) && pv_half(0, i, i, 1, true, true, i + 2);
+          const bool shared = n_b > 0;
+          for (int i = 0; ok && i < n_a; ++i) ok = pv(0, i, i, true, !shared) && (!shared || pv(1, i, i, false, true));
         }
       }
     }
@@ -432,12 +433,12 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       const int row = (warp & 3) * 32 + lane;
       const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
       const uint32_t s_addr = tmem + lane_base + kColS;
-      const uint32_t p_addr = tmem + lane_base + kColP + 16 * t;
-      const uint32_t sf_addr = tmem + lane_base + kColSfP + 8 * t + (warp & 3);  // the row's lane quadrant reads this column
+      const uint32_t p_addr = tmem + lane_base + kColP + 32 * t;
+      const uint32_t sf_addr = tmem + lane_base + kColSfP + 16 * t + (warp & 3);  // the row's lane quadrant reads this column
       const uint32_t o_addr = tmem + lane_base + kColO + t * kTile;
       const int quarter = (warp & 3) >> 1;  // 64-row query block inside the tile
       float m_run = -INFINITY;  // raw q.k units
-      float l0 = 0.f, l1 = 0.f, l2 = 0.f, l3 = 0.f;
+      uint64_t la = 0ull;  // two partial row sums
       bool ok = wait_list(kWaitTimeoutLoad);
       const int n = ok ? tile_count(t) : 0;
       for (int i = 0; i < n; ++i) {
@@ -453,6 +454,8 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&S.s_taken[t]);
+        // PV(i-2) read the P buffer of this tile: looked at early, so that the answer is there when P is stored
+        const bool p_free = i < 2 || mbar_test(&S.pv_done[t][i & 1], ((i - 2) >> 1) & 1);
         // keys that do not exist or that this row's query block did not select count as -inf
         int hi = selected ? kKeys : 0;
         const int valid = P.num_kv_tokens - kt * kKeys;
@@ -462,7 +465,8 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           for (int e = 0; e < kKeys; ++e)
             if (e >= hi) s[e] = 0xff800000u;
         }
-        bool pv_waited = i == 0;
+        bool raise = false;
+        float alpha = 1.f;
         uint32_t pw[kKeys / 8], sfw[kKeys / 64];
         if (hi <= 0) {
           // nothing of this tile for this warp's rows (uniform: a warp lies inside one query block)
@@ -471,98 +475,91 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 #pragma unroll
           for (int c = 0; c < kKeys / 64; ++c) sfw[c] = 0u;
         } else {
-          float mx0 = __uint_as_float(s[0]), mx1 = __uint_as_float(s[1]);
-          float mx2 = __uint_as_float(s[2]), mx3 = __uint_as_float(s[3]);
-#pragma unroll
-          for (int e = 4; e < kKeys - 4; e += 8) {
-            mx0 = max3(mx0, __uint_as_float(s[e]), __uint_as_float(s[e + 1]));
-            mx1 = max3(mx1, __uint_as_float(s[e + 2]), __uint_as_float(s[e + 3]));
-            mx2 = max3(mx2, __uint_as_float(s[e + 4]), __uint_as_float(s[e + 5]));
-            mx3 = max3(mx3, __uint_as_float(s[e + 6]), __uint_as_float(s[e + 7]));
-          }
-          mx0 = max3(mx0, __uint_as_float(s[kKeys - 4]), __uint_as_float(s[kKeys - 3]));
-          mx1 = max3(mx1, __uint_as_float(s[kKeys - 2]), __uint_as_float(s[kKeys - 1]));
-          const float m_new = fmaxf(m_run, fmaxf(max3(mx0, mx1, mx2), mx3));
-          if (i > 0 && __any_sync(0xffffffffu, m_new > m_run)) {
-            // exact running maximum: the accumulated numerator and sum move to the new reference
-            const float alpha = ex2((m_run - m_new) * P.scale_log2);
-            l0 *= alpha, l1 *= alpha, l2 *= alpha, l3 *= alpha;
-            ok = poll(&S.pv_done[t], (i - 1) & 1, kWaitTimeoutMma);
-            if (!ok) break;
-            pv_waited = true;
-            tc_fence_after();
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              uint32_t o[32];
-              tmem_ld32(o_addr + 32 * c, o);
-              tc_wait_ld();
-#pragma unroll
-              for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
-              tmem_st32(o_addr + 32 * c, o);
-            }
-            tc_wait_st();
-          }
-          m_run = m_new;
-          const float bias = kLog2PScale - m_run * P.scale_log2;
-          const uint64_t scale2 = pack2(P.scale_log2, P.scale_log2), bias2 = pack2(bias, bias);
-          uint64_t la = pack2(l0, l1), lb = pack2(l2, l3);
+          // Maxima of the groups of 16 keys, floored at a finite value so that a group without keys gives zero codes and a
+          // zero scale; they serve the running maximum and the quantisation both.
+          float gmax[kKeys / 16];
 #pragma unroll
           for (int g = 0; g < kKeys / 16; ++g) {
-            float p[16];
+            auto sc = [&](int e) { return __uint_as_float(s[16 * g + e]); };
+            const float a0 = max3(sc(0), sc(1), sc(2)), a1 = max3(sc(3), sc(4), sc(5)), a2 = max3(sc(6), sc(7), sc(8));
+            const float a3 = max3(sc(9), sc(10), sc(11)), a4 = max3(sc(12), sc(13), sc(14));
+            gmax[g] = max3(max3(a0, a1, a2), max3(a3, a4, sc(15)), -1e30f);
+          }
+          float m_new = fmaxf(m_run, gmax[0]);
+#pragma unroll
+          for (int g = 1; g < kKeys / 16 - 1; g += 2) m_new = max3(m_new, gmax[g], gmax[g + 1]);
+          m_new = fmaxf(m_new, gmax[kKeys / 16 - 1]);
+          // exact running maximum: the accumulated numerator and sum move to the new reference
+          raise = i > 0 && __any_sync(0xffffffffu, m_new > m_run);
+          if (raise) {
+            alpha = ex2((m_run - m_new) * P.scale_log2);
+            const uint64_t alpha2 = pack2(alpha, alpha);
+            la = mul2(la, alpha2);
+          }
+          m_run = m_new;
+          // A group's codes are p / (its maximum / 6) = 2^(x - x_max) * 6 with x the scaled score: one exponential
+          // straight onto the code grid (one multiply-add per pair and no reciprocal, no division of p), and the block
+          // scale is 2^(x_max - m) * 448 <= 448.  It equals dividing p by the unrounded scale up to fp32 rounding: a code
+          // moves only when p / scale sits within that of a rounding boundary of the e2m1 grid.
+          const float bias = kLog2BlockScale - m_run * P.scale_log2;
+          const uint64_t scale2 = pack2(P.scale_log2, P.scale_log2);
+          float y[2][16];
+          auto exponentials = [&](int g) {
+            const float c = fmaf(-gmax[g], P.scale_log2, kLog2Six);
+            const uint64_t c2 = pack2(c, c);
 #pragma unroll
             for (int e = 0; e < 16; e += 2) {
               float x0, x1;
-              unpack2(fma2(pack2(__uint_as_float(s[16 * g + e]), __uint_as_float(s[16 * g + e + 1])), scale2, bias2), x0, x1);
-              p[e] = ex2(x0);
-              p[e + 1] = ex2(x1);
+              unpack2(fma2(pack2(__uint_as_float(s[16 * g + e]), __uint_as_float(s[16 * g + e + 1])), scale2, c2), x0, x1);
+              y[g & 1][e] = ex2(x0);
+              y[g & 1][e + 1] = ex2(x1);
             }
+          };
+          exponentials(0);
 #pragma unroll
-            for (int e = 0; e < 16; e += 4) {
-              la = add2(la, pack2(p[e], p[e + 1]));
-              lb = add2(lb, pack2(p[e + 2], p[e + 3]));
-            }
-            float a0 = max3(p[0], p[1], p[2]), a1 = max3(p[3], p[4], p[5]), a2 = max3(p[6], p[7], p[8]);
-            float a3 = max3(p[9], p[10], p[11]), a4 = max3(p[12], p[13], p[14]);
-            const float gmax = fmaxf(max3(a0, a1, a2), max3(a3, a4, p[15]));
-            // block scale max/6 (at most 448 because p <= 2688), the codes are p over the unrounded scale.  The
-            // reciprocal is the MUFU approximation (1 ulp): it moves a code only when p / scale sits within an ulp
-            // of a rounding boundary of the e2m1 grid.
-            const float bs = gmax * (1.0f / 6.0f);
-            float inv;
-            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(bs));
-            inv = bs > 0.f ? inv : 0.f;
-            const uint64_t inv2 = pack2(inv, inv);
-#pragma unroll
-            for (int e = 0; e < 16; e += 2) unpack2(mul2(pack2(p[e], p[e + 1]), inv2), p[e], p[e + 1]);
-            pw[2 * g] = pack_e2m1x8(p);
-            pw[2 * g + 1] = pack_e2m1x8(p + 8);
+          for (int g = 0; g < kKeys / 16; ++g) {
+            const float bs = ex2(fmaf(gmax[g], P.scale_log2, bias));
+            if (g + 1 < kKeys / 16) exponentials(g + 1);
+            const float* c = y[g & 1];
+            uint64_t sum = add2(add2(pack2(c[0], c[1]), pack2(c[2], c[3])), add2(pack2(c[4], c[5]), pack2(c[6], c[7])));
+            sum = add2(sum, add2(add2(pack2(c[8], c[9]), pack2(c[10], c[11])), add2(pack2(c[12], c[13]), pack2(c[14], c[15]))));
+            la = fma2(sum, pack2(bs, bs), la);  // the unrounded probabilities' sum: p = code value x unrounded scale
+            pw[2 * g] = pack_e2m1x8(c);
+            pw[2 * g + 1] = pack_e2m1x8(c + 8);
             const uint32_t byte = pack_e4m3x2(bs, 0.f) & 0xffu;
             if ((g & 3) == 0) sfw[g >> 2] = 0u;
             sfw[g >> 2] |= byte << (8 * (g & 3));
           }
-          unpack2(la, l0, l1);
-          unpack2(lb, l2, l3);
         }
-        if (!pv_waited) {
-          // the previous tile's value MMAs still read P_t and its scales until this completes
-          ok = poll(&S.pv_done[t], (i - 1) & 1, kWaitTimeoutMma);
+        if (!__all_sync(0xffffffffu, p_free)) {
+          ok = poll(&S.pv_done[t][i & 1], ((i - 2) >> 1) & 1, kWaitTimeoutMma);
           if (!ok) break;
-          tc_fence_after();
         }
+        tc_fence_after();
 #pragma unroll
         for (int half = 0; half < kKeys / 64; ++half) {
-          tmem_st8(p_addr + 8 * half, pw + 8 * half);
-          tmem_st1(sf_addr + 4 * half, sfw[half]);
-          tc_wait_st();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&S.p_full[t][half]);
+          tmem_st8(p_addr + 16 * (i & 1) + 8 * half, pw + 8 * half);
+          tmem_st1(sf_addr + 8 * (i & 1) + 4 * half, sfw[half]);
         }
+        tc_wait_st();
+        if (raise) {
+          // O_t moves to the new maximum: after the exponentials, when the scores' registers are free and PV(i-1) is long
+          // complete, and before the arrival that lets PV(i) start
+          ok = poll(&S.pv_done[t][(i - 1) & 1], ((i - 1) >> 1) & 1, kWaitTimeoutMma);
+          if (!ok) break;
+          tc_fence_after();
+          tmem_scale_rows_wide(o_addr, alpha);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&S.p_full[t][i & 1]);
       }
-      if (ok && n > 0) ok = poll(&S.pv_done[t], (n - 1) & 1, kWaitTimeoutMma);
+      if (ok && n > 0) ok = poll(&S.pv_done[t][(n - 1) & 1], ((n - 1) >> 1) & 1, kWaitTimeoutMma);
       if (ok && n > 0) {
         tc_fence_after();
-        const float l = (l0 + l1) + (l2 + l3);
+        float l0, l1;
+        unpack2(la, l0, l1);
+        const float l = l0 + l1;
         const int token = q0 + t * kTile + row;
         const bool store = token < P.num_query_tokens && NOB_CHECK(head + P.head_offset < P.total_heads, status);
         const size_t at = (static_cast<size_t>(store ? token : 0) * P.total_heads + head + P.head_offset);
