@@ -58,6 +58,27 @@ int nob200_dense_bf16_attention_d128_splitkv(int num_tokens, int head_offset, co
                                              int kv_splits, void* workspace, size_t workspace_bytes, void* stream);
 
 /*
+ * The three dense kernels by units: `unit_rows` (128 or 256) query rows of one head, numbered head by head, one CTA each.
+ * The key tiles of the last `tail_units` units are divided into kv_splits shares each (0: of all units), the units before
+ * them run whole, so that a launch of 3.5 waves of 148 CTAs ends after 3.5 waves; 128 rows double the units of a small
+ * call.  Shares are kept in fp32 until the merge.  workspace: nob200_key_split_workspace_bytes() bytes.
+ */
+size_t nob200_key_split_workspace_bytes(int num_query_tokens, int heads, int unit_rows, int kv_splits, int tail_units);
+int nob200_dense_bf16_attention_d128_units(int num_tokens, int head_offset, const void* query, const void* key,
+                                          const void* value, void* output, int heads, int total_heads, int unit_rows, int kv_splits,
+                                          int tail_units, void* workspace, size_t workspace_bytes, void* stream);
+int nob200_dense_int8_fp8_d128_units(int num_kv_tokens, int num_query_tokens, const void* query, const void* key,
+                                    const void* value, const void* query_scale, const void* key_scale,
+                                    const void* value_scale, void* output, int heads, int query_block, int key_block,
+                                    int unit_rows, int kv_splits, int tail_units, void* workspace, size_t workspace_bytes, void* stream);
+int nob200_dense_nvfp4_attention_d128_units(int num_query_tokens, int num_kv_tokens, int head_offset, const void* query,
+                                           const void* key, const void* value, const void* query_scales,
+                                           const void* key_scales, const void* value_scales, float query_global,
+                                           float key_global, float value_global, void* output, int heads,
+                                           int total_heads, int unit_rows, int kv_splits, int tail_units, void* workspace,
+                                           size_t workspace_bytes, void* stream);
+
+/*
  * The same attention with the head->sequence reshard of the multi-GPU path fused into its epilogue
  * (no counterpart in the reference, which is single-GPU): this rank holds all `num_tokens` tokens of `heads`
  * heads; output row `token` belongs to rank token / (num_tokens / world) and is written straight into

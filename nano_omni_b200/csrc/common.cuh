@@ -37,6 +37,25 @@ uint32_t* status_word_device_ptr();  // address of the file-scope status word
 
 }  // namespace nob200
 
+#ifdef __CUDACC__
+namespace nob200 {
+// Launches a kernel whose first statement is pdl_wait(): its CTAs may be brought onto the SMs while the kernel before it
+// in the stream drains (programmatic dependent launch), which takes the launch latency (2-3 us) off the path.
+template <typename... Params, typename... Args>
+int launch_pdl(const char* what, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, void* stream, Args&&... args) {
+  cudaLaunchAttribute attribute = {};
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid, config.blockDim = block, config.dynamicSmemBytes = smem;
+  config.stream = static_cast<cudaStream_t>(stream);
+  config.attrs = &attribute, config.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+  return check_launch(what);
+}
+}  // namespace nob200
+#endif
+
 #define NOB_REQUIRE(cond, ...)                                        \
   do {                                                                \
     if (!(cond)) return nob200::fail(nob200::kInvalidArgument, __VA_ARGS__); \
@@ -68,6 +87,12 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
   return t;
 }
+
+// ---- programmatic dependent launch.  A kernel launched by launch_pdl() starts with pdl_wait(), in every thread: it
+// returns when the kernels before it in the stream have completed and their writes are visible.  pdl_release() lets the
+// next kernel of the stream be scheduled from the moment every CTA has called it (or exited); it orders no memory.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {

@@ -198,9 +198,70 @@ __device__ __forceinline__ bool route_open(const OutRoute& route, const uint32_t
   return (word & kWaitTimeoutPeer) == 0;
 }
 
-// Merge of key-split shares (normalised bf16 partial outputs [split][token][head][128] and their log-sum-exp in log2
-// units) into the routed output; defined beside the bf16 attention kernel.
-int launch_merge_splits(const __nv_bfloat16* partial_out, const float* partial_lse, const OutRoute& route, int num_tokens,
-                        int heads, int total_heads, int head_offset, int splits, void* stream);
+// How the units of a dense launch - `unit_rows` query rows of one head, numbered head by head - become CTAs.  256 rows
+// are two query tiles that share their K / V tiles and overlap each other's phases; 128 rows (one tile, 0.72 of the
+// time per key tile) double the units of a small call.  The first
+// `full_units` are one CTA each; the key tiles of the rest are divided over `splits` CTAs, whose normalised partial
+// results and log-sum-exps (log2 units) fa_merge_splits_kernel joins.  Dividing only the units of the last wave lets a
+// launch end on all SMs together at the price of a few partial rows: 518 units on 148 SMs are 3.5 waves, not 4.
+struct KeySplit {
+  int unit_rows = 256, q_tiles = 0, full_units = 0, splits = 1;
+  long long tail_base = 0;  // row (head * tokens + token) of the first divided unit
+  long long tail_rows = 0;  // rows of all divided units
+  void* partial = nullptr;  // [splits][tail_rows][128], f32 or bf16
+  float* lse = nullptr;     // [splits][tail_rows]
+  bool partial_f32 = false;
+
+  struct Share {
+    int head, q_tile, kv_begin, kv_end, piece;  // piece < 0: the whole unit
+  };
+  // A copy read back from shared memory: head, query tile and piece are needed before and after the key loop, and kept
+  // in registers across it they would be spilled inside it.
+  static __device__ __forceinline__ Share reload(const Share& kept) {
+    const volatile Share& v = kept;
+    return Share{v.head, v.q_tile, v.kv_begin, v.kv_end, v.piece};
+  }
+  __device__ __forceinline__ Share share(int block, int n_kv_total) const {
+    Share r{0, 0, 0, n_kv_total, -1};
+    int unit = block;
+    if (block >= full_units) {
+      const int k = (block - full_units) / splits;
+      r.piece = block - full_units - k * splits;
+      unit = full_units + k;
+      r.kv_begin = static_cast<int>(static_cast<long long>(n_kv_total) * r.piece / splits);
+      r.kv_end = static_cast<int>(static_cast<long long>(n_kv_total) * (r.piece + 1) / splits);
+    }
+    r.head = unit / q_tiles;
+    r.q_tile = unit - r.head * q_tiles;
+    return r;
+  }
+  __device__ __forceinline__ size_t partial_row(int piece, int head, int token, int num_tokens) const {
+    return static_cast<size_t>(piece * tail_rows + (static_cast<long long>(head) * num_tokens + token - tail_base));
+  }
+  // 32 normalised channels of a partial row, from channel `c0` on
+  __device__ __forceinline__ void store(size_t row, int c0, const float (&v)[32]) const {
+    if (partial_f32) {
+      float4* dst = reinterpret_cast<float4*>(static_cast<float*>(partial) + row * 128 + c0);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    } else {
+      uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(partial) + row * 128 + c0);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        dst[i] = make_uint4(pack_bf16(v[8 * i], v[8 * i + 1]), pack_bf16(v[8 * i + 2], v[8 * i + 3]),
+                            pack_bf16(v[8 * i + 4], v[8 * i + 5]), pack_bf16(v[8 * i + 6], v[8 * i + 7]));
+    }
+  }
+};
+
+// The split of a launch: `tail_units` 0 divides every unit.  Checks the arguments and the workspace.
+int make_key_split(KeySplit* split, const char* name, int num_query_tokens, int num_kv_tokens, int heads, int unit_rows,
+                   int kv_splits, int tail_units, bool partial_f32, void* workspace, size_t workspace_bytes);
+inline int key_split_blocks(const KeySplit& s, int heads) {
+  return s.full_units + (s.q_tiles * heads - s.full_units) * s.splits;
+}
+// Joins the shares of the divided units into the routed output; defined beside the bf16 attention kernel.
+int launch_merge_splits(const KeySplit& split, const OutRoute& route, int num_tokens, int total_heads, int head_offset,
+                        void* stream);
 
 }  // namespace nob200

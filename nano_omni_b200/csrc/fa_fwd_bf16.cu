@@ -59,6 +59,7 @@ struct __align__(1024) Shared {
   uint64_t s_taken[2];    // the softmax warps of tile t hold them in registers: the buffer is free
   uint64_t p_full[2][2];  // a 64-key half of P_t is written
   uint64_t pv_done[2];    // O_t += P_t V_j has completed: P_t may be overwritten, O_t may be rescaled
+  KeySplit::Share share;
   uint32_t tmem_base;
   uint32_t abort;
   uint32_t qk_issued;     // score MMA groups issued so far (written by the score issuer, polled by the value issuer)
@@ -80,7 +81,7 @@ constexpr uint32_t kColS = 0, kColP = 128, kColO = 256;  // TMEM columns; P_t at
 __device__ long long g_trace[12][64][8];
 #define TRACE(role, j, k)                                                         \
   do {                                                                            \
-    if (blockIdx.x == 1 && blockIdx.y == 0 && (j) < 64) g_trace[role][j][k] = clock64(); \
+    if (blockIdx.x == 1 && (j) < 64) g_trace[role][j][k] = clock64(); \
   } while (0)
 #else
 #define TRACE(role, j, k) \
@@ -98,22 +99,19 @@ template <int POLY, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 fa_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                    const __grid_constant__ CUtensorMap map_v, const OutRoute out, int num_tokens,
-                   int total_heads, int head_offset, float scale_log2, uint32_t* status,
-                   __nv_bfloat16* __restrict__ partial_out, float* __restrict__ partial_lse) {
+                   int total_heads, int head_offset, float scale_log2, uint32_t* status, const KeySplit split) {
   extern __shared__ uint8_t smem_raw[];
   Shared& S = *reinterpret_cast<Shared*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int head = blockIdx.y;
-  const int q0 = blockIdx.x * (2 * kTile);
-  const bool two = q0 + kTile < num_tokens;  // second tile holds at least one row
-  // gridDim.z > 1: this CTA covers only a contiguous share of the key tiles and writes a normalised
-  // partial result with its log-sum-exp; a second kernel merges the shares.
   const int n_kv_total = (num_tokens + kTile - 1) / kTile;
-  const int kv_begin = static_cast<int>(static_cast<long long>(n_kv_total) * blockIdx.z / gridDim.z);
-  const int kv_end = static_cast<int>(static_cast<long long>(n_kv_total) * (blockIdx.z + 1) / gridDim.z);
-  const int n_kv = kv_end - kv_begin;
+  const KeySplit::Share share = split.share(blockIdx.x, n_kv_total);
+  const int head = share.head;
+  const int q0 = share.q_tile * split.unit_rows;
+  const bool two = split.unit_rows > kTile && q0 + kTile < num_tokens;  // second tile holds at least one row
+  const int kv_begin = share.kv_begin;
+  const int n_kv = share.kv_end - kv_begin;
   volatile uint32_t* abort_flag = &S.abort;
 
   if (threadIdx.x == 0) {
@@ -129,6 +127,7 @@ fa_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       mbar_init(&S.p_full[t][1], 4);
       mbar_init(&S.pv_done[t], 1);
     }
+    S.share = share;
     S.abort = 0;
     S.qk_issued = 0;
     mbar_fence_init();
@@ -141,6 +140,7 @@ fa_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = S.tmem_base;
+  pdl_release();  // the merge of the shares may be scheduled behind the last CTAs
 
   if (warp >= 8) {
    reg_dealloc<kServiceRegs>();
@@ -302,7 +302,6 @@ fa_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     auto poll = [&](uint64_t* bar, uint32_t parity, uint32_t bit) { return warp_poll(bar, parity, abort_flag, status, bit); };
     const int t = warp >> 2;
     if (t == 0 || two) {
-      const int row = (warp & 3) * 32 + lane;
       const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
       const uint32_t s_addr = tmem + lane_base + kColS;
       const uint32_t p_addr = tmem + lane_base + kColP + t * 64;
@@ -427,15 +426,19 @@ fa_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         unpack2(lb, l2, l3);
         const float l = (l0 + l1) + (l2 + l3);
         const float inv = 1.0f / l;
-        const int token = q0 + t * kTile + row;
-        __nv_bfloat16* dst = out.row(token < num_tokens ? token : 0, total_heads, head + head_offset);
+        const KeySplit::Share at_end = KeySplit::reload(S.share);
+        const int head = at_end.head, q0 = at_end.q_tile * split.unit_rows;
+        const int token = q0 + t * kTile + (warp & 3) * 32 + lane;
+        const bool divided = at_end.piece >= 0;
         bool store = token < num_tokens;
-        if (gridDim.z > 1) {
-          const size_t at = (static_cast<size_t>(blockIdx.z) * num_tokens + token) * gridDim.y + head;
-          dst = partial_out + at * 128;
-          store = store && NOB_CHECK(at < static_cast<size_t>(gridDim.z) * num_tokens * gridDim.y, status);
-          if (store) partial_lse[at] = m_used + log2f(l);
+        __nv_bfloat16* dst = nullptr;
+        size_t row_at = 0;
+        if (divided) {
+          row_at = split.partial_row(at_end.piece, head, store ? token : q0, num_tokens);
+          store = store && NOB_CHECK(row_at < static_cast<size_t>(split.splits) * split.tail_rows, status);
+          if (store) split.lse[row_at] = m_used + log2f(l);
         } else {
+          dst = out.row(store ? token : 0, total_heads, head + head_offset);
           store = store && route_open(out, status);
           store = store && NOB_CHECK(head + head_offset < total_heads &&
                                          (out.tokens_per_rank == 0 ||
@@ -448,14 +451,17 @@ fa_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           tmem_ld32(o_addr + 32 * c, o);
           tc_wait_ld();
           if (store) {
+            float r[32];
 #pragma unroll
-            for (int i = 0; i < 32; i += 8) {
-              uint4 v;
-              v.x = pack_bf16(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
-              v.y = pack_bf16(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
-              v.z = pack_bf16(__uint_as_float(o[i + 4]) * inv, __uint_as_float(o[i + 5]) * inv);
-              v.w = pack_bf16(__uint_as_float(o[i + 6]) * inv, __uint_as_float(o[i + 7]) * inv);
-              *reinterpret_cast<uint4*>(dst + 32 * c + i) = v;
+            for (int i = 0; i < 32; ++i) r[i] = __uint_as_float(o[i]) * inv;
+            if (divided) {
+              split.store(row_at, 32 * c, r);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 32; i += 8)
+                *reinterpret_cast<uint4*>(dst + 32 * c + i) =
+                    make_uint4(pack_bf16(r[i], r[i + 1]), pack_bf16(r[i + 2], r[i + 3]), pack_bf16(r[i + 4], r[i + 5]),
+                               pack_bf16(r[i + 6], r[i + 7]));
             }
           }
         }
@@ -468,32 +474,41 @@ fa_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   if (warp == kProducerWarp) tmem_dealloc(tmem, kTmemCols);
 }
 
-// Merge of split-KV shares: out = sum_z w_z * partial_z with w_z = 2^(lse_z - max lse) / sum of those.
+// Merge of key shares: out = sum_z w_z * partial_z with w_z = 2^(lse_z - max lse) / sum of those.  A thread owns eight
+// channels of a row.
+template <bool kF32>
 __global__ void __launch_bounds__(256)
-fa_merge_splits_kernel(const __nv_bfloat16* __restrict__ partial_out, const float* __restrict__ partial_lse,
-                       const OutRoute out, int num_tokens, int heads, int total_heads, int head_offset,
-                       int splits, const uint32_t* status) {
-  const long long item = blockIdx.x * 256ll + threadIdx.x;  // (token, head, 8-channel piece)
-  const long long total = static_cast<long long>(num_tokens) * heads * 16;
-  if (item >= total || !route_open(out, status)) return;
+fa_merge_splits_kernel(const KeySplit split, const OutRoute out, int num_tokens, int total_heads, int head_offset,
+                       const uint32_t* status) {
+  pdl_wait();
+  const long long item = blockIdx.x * 256ll + threadIdx.x;  // (row, 8-channel piece)
+  if (item >= split.tail_rows * 16 || !route_open(out, status)) return;
   const int piece = static_cast<int>(item & 15);
-  const long long th = item >> 4;  // token * heads + head
-  const int head = static_cast<int>(th % heads);
-  const long long token = th / heads;
-  const size_t share = static_cast<size_t>(num_tokens) * heads;
+  const long long row = item >> 4;
+  const int head = static_cast<int>((split.tail_base + row) / num_tokens);
+  const int token = static_cast<int>((split.tail_base + row) - static_cast<long long>(head) * num_tokens);
   float mx = -INFINITY;
-  for (int z = 0; z < splits; ++z) mx = fmaxf(mx, partial_lse[z * share + th]);
+  for (int z = 0; z < split.splits; ++z) mx = fmaxf(mx, split.lse[z * split.tail_rows + row]);
   float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   float wsum = 0.f;
-  for (int z = 0; z < splits; ++z) {
-    const float w = exp2f(partial_lse[z * share + th] - mx);
+  for (int z = 0; z < split.splits; ++z) {
+    const size_t at = static_cast<size_t>(z * split.tail_rows + row);
+    const float w = exp2f(split.lse[at] - mx);
     wsum += w;
-    const uint4 raw = *reinterpret_cast<const uint4*>(partial_out + (z * share + th) * 128 + piece * 8);
-    const uint32_t r[4] = {raw.x, raw.y, raw.z, raw.w};
+    if (kF32) {
+      const float4* src = reinterpret_cast<const float4*>(static_cast<const float*>(split.partial) + at * 128 + piece * 8);
+      const float4 x = src[0], y = src[1];
+      const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      acc[2 * i] += w * __uint_as_float(r[i] << 16);
-      acc[2 * i + 1] += w * __uint_as_float(r[i] & 0xffff0000u);
+      for (int i = 0; i < 8; ++i) acc[i] += w * v[i];
+    } else {
+      const uint4 raw = *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(split.partial) + at * 128 + piece * 8);
+      const uint32_t r[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        acc[2 * i] += w * __uint_as_float(r[i] << 16);
+        acc[2 * i + 1] += w * __uint_as_float(r[i] & 0xffff0000u);
+      }
     }
   }
   const float inv = 1.0f / wsum;
@@ -502,32 +517,27 @@ fa_merge_splits_kernel(const __nv_bfloat16* __restrict__ partial_out, const floa
   v.y = pack_bf16(acc[2] * inv, acc[3] * inv);
   v.z = pack_bf16(acc[4] * inv, acc[5] * inv);
   v.w = pack_bf16(acc[6] * inv, acc[7] * inv);
-  *reinterpret_cast<uint4*>(out.row(static_cast<int>(token), total_heads, head + head_offset) + piece * 8) = v;
+  *reinterpret_cast<uint4*>(out.row(token, total_heads, head + head_offset) + piece * 8) = v;
 }
 
 int launch_dense_bf16(int num_tokens, int head_offset, const void* query, const void* key, const void* value,
-                      const OutRoute& route, int heads, int total_heads, int kv_splits, void* workspace,
-                      size_t workspace_bytes, void* stream) {
+                      const OutRoute& route, int heads, int total_heads, int unit_rows, int kv_splits,
+                      int tail_units, bool partial_f32, void* workspace, size_t workspace_bytes, void* stream) {
   const char* name = "dense_bf16_attention_d128";
   NOB_REQUIRE(num_tokens > 0 && heads > 0 && total_heads > 0, "%s: sizes must be positive", name);
   NOB_REQUIRE(head_offset >= 0 && head_offset <= total_heads - heads, "%s: head_offset %d outside [0, %d]", name,
               head_offset, total_heads - heads);
   NOB_REQUIRE(query && key && value && route.peer[0], "%s: NULL tensor", name);
-  NOB_REQUIRE(heads <= 65535, "%s: heads %d exceeds grid limit", name, heads);
-  const int n_kv = (num_tokens + kTile - 1) / kTile;
-  NOB_REQUIRE(kv_splits >= 1 && kv_splits <= 64 && kv_splits <= n_kv, "%s: kv_splits %d outside [1, min(64, %d)]",
-              name, kv_splits, n_kv);
-  const size_t share = static_cast<size_t>(num_tokens) * heads;
-  const size_t partial_bytes = (static_cast<size_t>(kv_splits) * share * 128 * 2 + 255) / 256 * 256;
-  const size_t need = kv_splits > 1 ? partial_bytes + static_cast<size_t>(kv_splits) * share * 4 : 0;
-  NOB_REQUIRE(need == 0 || (workspace && workspace_bytes >= need), "%s: %zu B of workspace required for %d key splits, %zu B given",
-              name, need, kv_splits, workspace_bytes);
+  KeySplit split;
+  int rc;
+  if ((rc = make_key_split(&split, name, num_tokens, num_tokens, heads, unit_rows, kv_splits, tail_units,
+                           partial_f32, workspace, workspace_bytes)))
+    return rc;
   uint32_t* status = status_word_device_ptr();
   if (!status) return fail(kCudaError, "%s: no current CUDA device", name);
 
   CUtensorMap mq, mk, mv;
   const uint64_t head_stride = 128 * 2, token_stride = static_cast<uint64_t>(heads) * 128 * 2;
-  int rc;
   if ((rc = make_tensor_map_3d(&mq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, query, 128, heads, num_tokens, head_stride,
                                token_stride, 64, 1, kTile)))
     return rc;
@@ -545,32 +555,51 @@ int launch_dense_bf16(int num_tokens, int head_offset, const void* query, const 
   if (err != cudaSuccess)
     return fail(kCudaError, "%s: cannot reserve %zu B of shared memory: %s", name, smem, cudaGetErrorString(err));
   const float scale_log2 = 0.08838834764831845f * 1.4426950408889634f;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  __nv_bfloat16* partial_out = static_cast<__nv_bfloat16*>(workspace);
-  float* partial_lse = kv_splits > 1 ? reinterpret_cast<float*>(static_cast<char*>(workspace) + partial_bytes) : nullptr;
-  dim3 grid((num_tokens + 2 * kTile - 1) / (2 * kTile), heads, kv_splits);
-  kernel<<<grid, kThreads, smem, s>>>(mq, mk, mv, route, num_tokens, total_heads, head_offset, scale_log2, status,
-                                      partial_out, partial_lse);
+  kernel<<<key_split_blocks(split, heads), kThreads, smem, static_cast<cudaStream_t>(stream)>>>(
+      mq, mk, mv, route, num_tokens, total_heads, head_offset, scale_log2, status, split);
   if ((rc = check_launch(name))) return rc;
-  if (kv_splits > 1) {
-    const long long items = static_cast<long long>(share) * 16;
-    fa_merge_splits_kernel<<<static_cast<unsigned>((items + 255) / 256), 256, 0, s>>>(
-        partial_out, partial_lse, route, num_tokens, heads, total_heads, head_offset, kv_splits, status);
-    rc = check_launch("dense_bf16_attention_d128(merge)");
-  }
-  return rc;
+  return split.tail_rows ? launch_merge_splits(split, route, num_tokens, total_heads, head_offset, stream) : kOk;
 }
 
 }  // namespace
 
-int launch_merge_splits(const __nv_bfloat16* partial_out, const float* partial_lse, const OutRoute& route, int num_tokens,
-                        int heads, int total_heads, int head_offset, int splits, void* stream) {
-  const long long items = static_cast<long long>(num_tokens) * heads * 16;
+int make_key_split(KeySplit* split, const char* name, int num_query_tokens, int num_kv_tokens, int heads, int unit_rows,
+                   int kv_splits, int tail_units, bool partial_f32, void* workspace, size_t workspace_bytes) {
+  const int n_kv = (num_kv_tokens + kTile - 1) / kTile;
+  NOB_REQUIRE(unit_rows == kTile || unit_rows == 2 * kTile, "%s: unit_rows must be 128 or 256 (got %d)", name, unit_rows);
+  NOB_REQUIRE(kv_splits >= 1 && kv_splits <= 64 && kv_splits <= n_kv, "%s: kv_splits %d outside [1, min(64, %d)]",
+              name, kv_splits, n_kv);
+  const int q_tiles = (num_query_tokens + unit_rows - 1) / unit_rows;
+  const long long units = static_cast<long long>(q_tiles) * heads;
+  NOB_REQUIRE(units * kv_splits <= 0x7fffffffll, "%s: %lld units x %d key splits exceed the grid limit", name, units, kv_splits);
+  NOB_REQUIRE(tail_units >= 0 && tail_units <= units, "%s: tail_units %d outside [0, %lld]", name, tail_units, units);
+  split->unit_rows = unit_rows;
+  split->q_tiles = q_tiles;
+  split->splits = kv_splits;
+  split->full_units = static_cast<int>(kv_splits == 1 ? units : tail_units ? units - tail_units : 0);
+  split->partial_f32 = partial_f32;
+  if (kv_splits == 1) return kOk;
+  const int head = split->full_units / q_tiles;
+  split->tail_base = static_cast<long long>(head) * num_query_tokens + static_cast<long long>(split->full_units - head * q_tiles) * unit_rows;
+  split->tail_rows = static_cast<long long>(heads) * num_query_tokens - split->tail_base;
+  const size_t rows = static_cast<size_t>(kv_splits) * split->tail_rows;
+  const size_t partial_bytes = (rows * 128 * (partial_f32 ? 4 : 2) + 255) / 256 * 256;
+  const size_t need = partial_bytes + rows * 4;
+  NOB_REQUIRE(workspace && workspace_bytes >= need, "%s: %zu B of workspace required for %d key splits, %zu B given", name,
+              need, kv_splits, workspace_bytes);
+  split->partial = workspace;
+  split->lse = reinterpret_cast<float*>(static_cast<char*>(workspace) + partial_bytes);
+  return kOk;
+}
+
+int launch_merge_splits(const KeySplit& split, const OutRoute& route, int num_tokens, int total_heads, int head_offset,
+                        void* stream) {
+  const long long blocks = (split.tail_rows * 16 + 255) / 256;
   uint32_t* status = status_word_device_ptr();
   if (!status) return fail(kCudaError, "attention(merge of key splits): no current CUDA device");
-  fa_merge_splits_kernel<<<static_cast<unsigned>((items + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      partial_out, partial_lse, route, num_tokens, heads, total_heads, head_offset, splits, status);
-  return check_launch("attention(merge of key splits)");
+  auto kernel = split.partial_f32 ? fa_merge_splits_kernel<true> : fa_merge_splits_kernel<false>;
+  return launch_pdl("attention(merge of key splits)", kernel, static_cast<unsigned>(blocks), 256, 0, stream, split, route,
+                    num_tokens, total_heads, head_offset, static_cast<const uint32_t*>(status));
 }
 
 }  // namespace nob200
@@ -586,8 +615,8 @@ extern "C" int nob200_dense_bf16_attention_d128(int num_tokens, int head_offset,
                                                 void* stream) {
   nob200::OutRoute route = {};
   route.peer[0] = static_cast<__nv_bfloat16*>(output);
-  return nob200::launch_dense_bf16(num_tokens, head_offset, query, key, value, route, heads, total_heads, 1, nullptr, 0,
-                                   stream);
+  return nob200::launch_dense_bf16(num_tokens, head_offset, query, key, value, route, heads, total_heads, 2 * nob200::kTile, 1, 0, false,
+                                   nullptr, 0, stream);
 }
 
 extern "C" size_t nob200_dense_bf16_attention_d128_splitkv_workspace_bytes(int num_tokens, int heads, int kv_splits) {
@@ -602,8 +631,31 @@ extern "C" int nob200_dense_bf16_attention_d128_splitkv(int num_tokens, int head
                                                         size_t workspace_bytes, void* stream) {
   nob200::OutRoute route = {};
   route.peer[0] = static_cast<__nv_bfloat16*>(output);
-  return nob200::launch_dense_bf16(num_tokens, head_offset, query, key, value, route, heads, total_heads, kv_splits,
-                                   workspace, workspace_bytes, stream);
+  return nob200::launch_dense_bf16(num_tokens, head_offset, query, key, value, route, heads, total_heads, 2 * nob200::kTile,
+                                   kv_splits, 0, false, workspace, workspace_bytes, stream);
+}
+
+extern "C" size_t nob200_key_split_workspace_bytes(int num_query_tokens, int heads, int unit_rows, int kv_splits,
+                                                   int tail_units) {
+  nob200::KeySplit split;
+  if (num_query_tokens <= 0 || heads <= 0 || kv_splits <= 1) return 0;
+  // a pointer and a size that pass every check: only the rows are of interest
+  char any;
+  if (nob200::make_key_split(&split, "key_split", num_query_tokens, 0x7fffff00, heads, unit_rows, kv_splits, tail_units,
+                             true, &any, ~size_t{0}))
+    return 0;
+  const size_t rows = static_cast<size_t>(kv_splits) * split.tail_rows;
+  return (rows * 512 + 255) / 256 * 256 + rows * 4;
+}
+
+extern "C" int nob200_dense_bf16_attention_d128_units(int num_tokens, int head_offset, const void* query, const void* key,
+                                                     const void* value, void* output, int heads, int total_heads,
+                                                     int unit_rows, int kv_splits, int tail_units, void* workspace,
+                                                     size_t workspace_bytes, void* stream) {
+  nob200::OutRoute route = {};
+  route.peer[0] = static_cast<__nv_bfloat16*>(output);
+  return nob200::launch_dense_bf16(num_tokens, head_offset, query, key, value, route, heads, total_heads, unit_rows,
+                                   kv_splits, tail_units, true, workspace, workspace_bytes, stream);
 }
 
 extern "C" int nob200_dense_bf16_attention_d128_scatter(int num_tokens, int head_offset, const void* query,
@@ -622,6 +674,6 @@ extern "C" int nob200_dense_bf16_attention_d128_scatter(int num_tokens, int head
     route.peer[r] = static_cast<__nv_bfloat16*>(peer_outputs[r]);
   }
   route.tokens_per_rank = num_tokens / world;
-  return launch_dense_bf16(num_tokens, head_offset, query, key, value, route, heads, total_heads, kv_splits, workspace,
-                           workspace_bytes, stream);
+  return launch_dense_bf16(num_tokens, head_offset, query, key, value, route, heads, total_heads, 2 * kTile, kv_splits, 0,
+                           false, workspace, workspace_bytes, stream);
 }

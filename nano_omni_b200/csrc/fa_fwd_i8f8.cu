@@ -81,22 +81,19 @@ fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                    const __grid_constant__ CUtensorMap map_v, const float* __restrict__ query_scale,
                    const float* __restrict__ key_scale, const float* __restrict__ value_scale,
                    __nv_bfloat16* __restrict__ out, int num_query_tokens, int num_kv_tokens, int heads,
-                   float scale_log2, uint32_t* status, int query_block, int key_block,
-                   __nv_bfloat16* __restrict__ partial_out, float* __restrict__ partial_lse) {
+                   float scale_log2, uint32_t* status, int query_block, int key_block, const KeySplit split) {
   extern __shared__ uint8_t smem_raw[];
   Shared& S = *reinterpret_cast<Shared*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int head = blockIdx.y;
-  const int q0 = blockIdx.x * (2 * kTile);
-  const bool two = q0 + kTile < num_query_tokens;
-  // gridDim.z > 1: this CTA covers a contiguous share of the key tiles and writes a normalised partial result with
-  // its log-sum-exp; fa_merge_splits_kernel (fa_fwd_bf16.cu) merges the shares.
   const int n_kv_total = (num_kv_tokens + kTile - 1) / kTile;
-  const int kv_begin = static_cast<int>(static_cast<long long>(n_kv_total) * blockIdx.z / gridDim.z);
-  const int kv_end = static_cast<int>(static_cast<long long>(n_kv_total) * (blockIdx.z + 1) / gridDim.z);
-  const int n_kv = kv_end - kv_begin;
+  const KeySplit::Share share = split.share(blockIdx.x, n_kv_total);
+  const int head = share.head;
+  const int q0 = share.q_tile * split.unit_rows;
+  const bool two = split.unit_rows > kTile && q0 + kTile < num_query_tokens;
+  const int kv_begin = share.kv_begin;
+  const int n_kv = share.kv_end - kv_begin;
   volatile uint32_t* abort_flag = &S.abort;
 
   // Key scales of this CTA's keys, one per 64 keys (scales per `key_block`, 64 or 128 tokens), to shared memory: read
@@ -132,6 +129,7 @@ fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = S.tmem_base;
+  pdl_release();  // the merge of the shares may be scheduled behind the last CTAs
 
   if (warp >= 8) {
     reg_dealloc<kServiceRegs>();
@@ -368,33 +366,33 @@ fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         const float l = (l0 + l1) + (l2 + l3);
         const float inv = 1.0f / l;
         const float* vs = value_scale + head * 128;
-        __nv_bfloat16* dst = out + (static_cast<size_t>(token) * heads + head) * 128;
-        if (gridDim.z > 1) {
-          const size_t at = (static_cast<size_t>(blockIdx.z) * num_query_tokens + token) * heads + head;
-          dst = partial_out + at * 128;
+        const bool divided = share.piece >= 0;
+        bool store = token < num_query_tokens && NOB_CHECK(head < heads, status);
+        __nv_bfloat16* dst = out + (static_cast<size_t>(store ? token : 0) * heads + head) * 128;
+        size_t row_at = 0;
+        if (divided) {
           // the probability scale 448/8 is common to all shares and cancels in the merge
-          if (token < num_query_tokens &&
-              NOB_CHECK(at < static_cast<size_t>(gridDim.z) * num_query_tokens * heads, status))
-            partial_lse[at] = m_used + log2f(l);
+          row_at = split.partial_row(share.piece, head, store ? token : q0, num_query_tokens);
+          store = store && NOB_CHECK(row_at < static_cast<size_t>(split.splits) * split.tail_rows, status);
+          if (store) split.lse[row_at] = m_used + log2f(l);
         }
-        const bool store = token < num_query_tokens && NOB_CHECK(head < heads, status);
 #pragma unroll
         for (int cc = 0; cc < 4; ++cc) {
           uint32_t o[32];
           tmem_ld32(o_addr + 32 * cc, o);
           tc_wait_ld();
           if (store) {
+            float r[32];
 #pragma unroll
-            for (int i = 0; i < 32; i += 8) {
-              float r[8];
+            for (int i = 0; i < 32; ++i) r[i] = __uint_as_float(o[i]) * vs[32 * cc + i] * inv;
+            if (divided) {
+              split.store(row_at, 32 * cc, r);
+            } else {
 #pragma unroll
-              for (int k = 0; k < 8; ++k) r[k] = __uint_as_float(o[i + k]) * vs[32 * cc + i + k] * inv;
-              uint4 v;
-              v.x = pack_bf16(r[0], r[1]);
-              v.y = pack_bf16(r[2], r[3]);
-              v.z = pack_bf16(r[4], r[5]);
-              v.w = pack_bf16(r[6], r[7]);
-              *reinterpret_cast<uint4*>(dst + 32 * cc + i) = v;
+              for (int i = 0; i < 32; i += 8)
+                *reinterpret_cast<uint4*>(dst + 32 * cc + i) =
+                    make_uint4(pack_bf16(r[i], r[i + 1]), pack_bf16(r[i + 2], r[i + 3]), pack_bf16(r[i + 4], r[i + 5]),
+                               pack_bf16(r[i + 6], r[i + 7]));
             }
           }
         }
@@ -407,37 +405,22 @@ fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   if (warp == kProducerWarp) tmem_dealloc(tmem, kTmemCols);
 }
 
-}  // namespace
-}  // namespace nob200
-
-extern "C" int nob200_dense_int8_fp8_d128(int num_kv_tokens, int num_query_tokens, const void* query, const void* key,
-                                          const void* value, const void* query_scale, const void* key_scale,
-                                          const void* value_scale, void* output, int heads, void* stream) {
-  return nob200_dense_int8_fp8_d128_blocks(num_kv_tokens, num_query_tokens, query, key, value, query_scale, key_scale,
-                                           value_scale, output, heads, 32, 64, stream);
-}
-
-extern "C" int nob200_dense_int8_fp8_d128_splitkv(int num_kv_tokens, int num_query_tokens, const void* query,
-                                                  const void* key, const void* value, const void* query_scale,
-                                                  const void* key_scale, const void* value_scale, void* output,
-                                                  int heads, int query_block, int key_block, int kv_splits,
-                                                  void* workspace, size_t workspace_bytes, void* stream) {
-  using namespace nob200;
+int launch_dense_int8_fp8(int num_kv_tokens, int num_query_tokens, const void* query, const void* key, const void* value,
+                          const void* query_scale, const void* key_scale, const void* value_scale, void* output, int heads,
+                          int query_block, int key_block, int unit_rows, int kv_splits, int tail_units,
+                          bool partial_f32, void* workspace, size_t workspace_bytes, void* stream) {
   NOB_REQUIRE(num_kv_tokens > 0 && num_query_tokens > 0 && heads > 0, "dense_int8_fp8_d128: sizes must be positive");
   NOB_REQUIRE(query && key && value && query_scale && key_scale && value_scale && output,
               "dense_int8_fp8_d128: NULL tensor");
-  NOB_REQUIRE(heads <= 65535, "dense_int8_fp8_d128: heads %d exceeds grid limit", heads);
   NOB_REQUIRE(query_block == 32 || query_block == 64 || query_block == 128,
               "dense_int8_fp8_d128: query scale block must be 32, 64 or 128 tokens (got %d)", query_block);
   NOB_REQUIRE(key_block == 64 || key_block == 128, "dense_int8_fp8_d128: key scale block must be 64 or 128 tokens (got %d)",
               key_block);
-  const int n_kv = (num_kv_tokens + kTile - 1) / kTile;
-  NOB_REQUIRE(kv_splits >= 1 && kv_splits <= 64 && kv_splits <= n_kv,
-              "dense_int8_fp8_d128: kv_splits %d outside [1, min(64, %d)]", kv_splits, n_kv);
-  const size_t need = nob200_dense_bf16_attention_d128_splitkv_workspace_bytes(num_query_tokens, heads, kv_splits);
-  NOB_REQUIRE(need == 0 || (workspace && workspace_bytes >= need),
-              "dense_int8_fp8_d128: %zu B of workspace required for %d key splits, %zu B given", need, kv_splits,
-              workspace_bytes);
+  KeySplit split;
+  int rc;
+  if ((rc = make_key_split(&split, "dense_int8_fp8_d128", num_query_tokens, num_kv_tokens, heads, unit_rows,
+                           kv_splits, tail_units, partial_f32, workspace, workspace_bytes)))
+    return rc;
   uint32_t* status = status_word_device_ptr();
   if (!status) return fail(kCudaError, "dense_int8_fp8_d128: no current CUDA device");
   const uint64_t q_rows = (static_cast<uint64_t>(num_query_tokens) + query_block - 1) / query_block * query_block;
@@ -445,7 +428,6 @@ extern "C" int nob200_dense_int8_fp8_d128_splitkv(int num_kv_tokens, int num_que
   const uint64_t v_cols = (static_cast<uint64_t>(num_kv_tokens) + 63) / 64 * 64;  // the value quantiser pads to 64
 
   CUtensorMap mq, mk, mv;
-  int rc;
   // Q, K: [heads][rows][128 bytes]; V: [heads][128 channels][v_cols bytes]
   if ((rc = make_tensor_map_3d(&mq, CU_TENSOR_MAP_DATA_TYPE_UINT8, query, 128, q_rows, heads, 128, q_rows * 128, 128,
                                kTile, 1)))
@@ -464,28 +446,52 @@ extern "C" int nob200_dense_int8_fp8_d128_splitkv(int num_kv_tokens, int num_que
     return fail(kCudaError, "dense_int8_fp8_d128: cannot reserve %zu B of shared memory: %s", smem,
                 cudaGetErrorString(err));
   const float scale_log2 = 0.08838834764831845f * 1.4426950408889634f;
-  const size_t share = static_cast<size_t>(num_query_tokens) * heads;
-  const size_t partial_bytes = (static_cast<size_t>(kv_splits) * share * 128 * 2 + 255) / 256 * 256;
-  __nv_bfloat16* partial_out = static_cast<__nv_bfloat16*>(workspace);
-  float* partial_lse = kv_splits > 1 ? reinterpret_cast<float*>(static_cast<char*>(workspace) + partial_bytes) : nullptr;
-  dim3 grid((num_query_tokens + 2 * kTile - 1) / (2 * kTile), heads, kv_splits);
-  fa_fwd_i8f8_kernel<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(
+  fa_fwd_i8f8_kernel<<<key_split_blocks(split, heads), kThreads, smem, static_cast<cudaStream_t>(stream)>>>(
       mq, mk, mv, static_cast<const float*>(query_scale), static_cast<const float*>(key_scale),
       static_cast<const float*>(value_scale), static_cast<__nv_bfloat16*>(output), num_query_tokens, num_kv_tokens,
-      heads, scale_log2, status, query_block, key_block, partial_out, partial_lse);
+      heads, scale_log2, status, query_block, key_block, split);
   if ((rc = check_launch("dense_int8_fp8_d128"))) return rc;
-  if (kv_splits > 1) {
-    OutRoute route = {};
-    route.peer[0] = static_cast<__nv_bfloat16*>(output);
-    rc = launch_merge_splits(partial_out, partial_lse, route, num_query_tokens, heads, heads, 0, kv_splits, stream);
-  }
-  return rc;
+  if (!split.tail_rows) return kOk;
+  OutRoute route = {};
+  route.peer[0] = static_cast<__nv_bfloat16*>(output);
+  return launch_merge_splits(split, route, num_query_tokens, heads, 0, stream);
+}
+
+}  // namespace
+}  // namespace nob200
+
+extern "C" int nob200_dense_int8_fp8_d128(int num_kv_tokens, int num_query_tokens, const void* query, const void* key,
+                                          const void* value, const void* query_scale, const void* key_scale,
+                                          const void* value_scale, void* output, int heads, void* stream) {
+  return nob200::launch_dense_int8_fp8(num_kv_tokens, num_query_tokens, query, key, value, query_scale, key_scale,
+                                       value_scale, output, heads, 32, 64, 2 * nob200::kTile, 1, 0, false, nullptr, 0, stream);
+}
+
+extern "C" int nob200_dense_int8_fp8_d128_splitkv(int num_kv_tokens, int num_query_tokens, const void* query,
+                                                  const void* key, const void* value, const void* query_scale,
+                                                  const void* key_scale, const void* value_scale, void* output,
+                                                  int heads, int query_block, int key_block, int kv_splits,
+                                                  void* workspace, size_t workspace_bytes, void* stream) {
+  return nob200::launch_dense_int8_fp8(num_kv_tokens, num_query_tokens, query, key, value, query_scale, key_scale,
+                                       value_scale, output, heads, query_block, key_block, 2 * nob200::kTile, kv_splits, 0,
+                                       false, workspace,
+                                       workspace_bytes, stream);
+}
+
+extern "C" int nob200_dense_int8_fp8_d128_units(int num_kv_tokens, int num_query_tokens, const void* query,
+                                               const void* key, const void* value, const void* query_scale,
+                                               const void* key_scale, const void* value_scale, void* output, int heads,
+                                               int query_block, int key_block, int unit_rows, int kv_splits, int tail_units,
+                                               void* workspace, size_t workspace_bytes, void* stream) {
+  return nob200::launch_dense_int8_fp8(num_kv_tokens, num_query_tokens, query, key, value, query_scale, key_scale,
+                                       value_scale, output, heads, query_block, key_block, unit_rows, kv_splits, tail_units, true,
+                                       workspace, workspace_bytes, stream);
 }
 
 extern "C" int nob200_dense_int8_fp8_d128_blocks(int num_kv_tokens, int num_query_tokens, const void* query,
                                                  const void* key, const void* value, const void* query_scale,
                                                  const void* key_scale, const void* value_scale, void* output,
                                                  int heads, int query_block, int key_block, void* stream) {
-  return nob200_dense_int8_fp8_d128_splitkv(num_kv_tokens, num_query_tokens, query, key, value, query_scale, key_scale,
-                                            value_scale, output, heads, query_block, key_block, 1, nullptr, 0, stream);
+  return nob200::launch_dense_int8_fp8(num_kv_tokens, num_query_tokens, query, key, value, query_scale, key_scale,
+                                       value_scale, output, heads, query_block, key_block, 2 * nob200::kTile, 1, 0, false, nullptr, 0, stream);
 }

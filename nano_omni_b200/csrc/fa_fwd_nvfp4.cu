@@ -84,6 +84,7 @@ struct __align__(1024) Shared {
                            // value issuer)
   uint64_t pv_done[2][2];  // O_t += P_t(i) V is complete, by parity of i: that P buffer is free, O_t may be rescaled
   uint64_t list_ready;
+  KeySplit::Share share;
   uint32_t tmem_base;
   uint32_t abort;
   int list_len[2];
@@ -148,20 +149,23 @@ constexpr uint32_t kIdesc = idesc_for(128);
 template <bool kSol>
 __global__ void __launch_bounds__(kThreads, 1)
 fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                    const __grid_constant__ CUtensorMap map_v, const Params P) {
+                    const __grid_constant__ CUtensorMap map_v, const Params P, const KeySplit split) {
   extern __shared__ uint8_t smem_raw[];
   Shared& S = *reinterpret_cast<Shared*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int head = blockIdx.y;
-  const int q0 = blockIdx.x * (2 * kTile);
-  const bool two = q0 + kTile < P.num_query_tokens;
+  const int n_kv_total = (P.num_kv_tokens + kTile - 1) / kTile;
+  const KeySplit::Share share =
+      kSol ? KeySplit::Share{(int)blockIdx.y, (int)blockIdx.x, 0, 0, -1} : split.share(blockIdx.x, n_kv_total);
+  const int head = share.head;
+  const int unit_rows = kSol ? 2 * kTile : split.unit_rows;
+  const int q0 = share.q_tile * unit_rows;
+  const bool two = unit_rows > kTile && q0 + kTile < P.num_query_tokens;
   // Dense: a step is a key tile of 128.  Sol: a step is one 64-key routing block of the tile's list, so that no MMA,
   // load or exponential is spent on a neighbour block nobody selected; K and V still arrive as 128-key tiles that
   // start at the block's first token, and the block-scaled MMAs read their first 64 keys.
   constexpr int kKeys = kSol ? 64 : kTile;
-  const int n_kv_total = (P.num_kv_tokens + kTile - 1) / kTile;
   const int q_row_blocks = (P.num_query_tokens + kTile - 1) / kTile;  // 128-row blocks of the padded operands
   volatile uint32_t* abort_flag = &S.abort;
   uint32_t* status = P.status;
@@ -181,6 +185,7 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       mbar_init(&S.pv_done[t][1], 1);
     }
     mbar_init(&S.list_ready, 1);
+    S.share = share;
     S.abort = 0;
     S.list_len[0] = S.list_len[1] = 0;
     mbar_fence_init();
@@ -193,10 +198,11 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = S.tmem_base;
+  pdl_release();  // the merge of the shares may be scheduled behind the last CTAs
 
-  // key tiles of query tile t: all of them (dense; both tiles share each K / V tile), or the tile's own list
-  auto tile_count = [&](int t) { return kSol ? S.list_len[t] : n_kv_total; };
-  auto tile_at = [&](int t, int i) { return kSol ? static_cast<int>(S.list[t][i]) : i; };
+  // key tiles of query tile t: those of the CTA's share (dense; both tiles share each K / V tile), or the tile's own list
+  auto tile_count = [&](int t) { return kSol ? S.list_len[t] : share.kv_end - share.kv_begin; };
+  auto tile_at = [&](int t, int i) { return kSol ? static_cast<int>(S.list[t][i]) : share.kv_begin + i; };
   auto wait_list = [&](uint32_t bit) -> bool {
     if (!kSol) return true;
     return __all_sync(0xffffffffu, mbar_wait(&S.list_ready, 0, abort_flag, status, bit));
@@ -259,7 +265,7 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         int next[2] = {0, 0};
         int issued = 0;
         for (int u = 0; u < units; ++u) {
-          int kt = u;
+          int kt = share.kv_begin + u;
           if (kSol) {
             const int t = (next[0] < n_a && (next[0] <= next[1] || next[1] >= n_b)) ? 0 : 1;
             kt = tile_at(t, next[t]++);
@@ -560,11 +566,15 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         float l0, l1;
         unpack2(la, l0, l1);
         const float l = l0 + l1;
+        const KeySplit::Share at_end = KeySplit::reload(S.share);
+        const int head = at_end.head, q0 = at_end.q_tile * (kSol ? 2 * kTile : split.unit_rows), row = (warp & 3) * 32 + lane;
         const int token = q0 + t * kTile + row;
-        const bool store = token < P.num_query_tokens && NOB_CHECK(head + P.head_offset < P.total_heads, status);
+        const bool divided = !kSol && at_end.piece >= 0;
+        bool store = token < P.num_query_tokens && NOB_CHECK(head + P.head_offset < P.total_heads, status);
         const size_t at = (static_cast<size_t>(store ? token : 0) * P.total_heads + head + P.head_offset);
         __nv_bfloat16* dst = P.out + at * 128;
         float factor;
+        size_t row_at = 0;
         if (kSol) {
           factor = kInvPScale * P.out_scale;
           if (store) {
@@ -573,6 +583,12 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           }
         } else {
           factor = P.out_scale / l;
+          if (divided) {
+            // the probability scale 2688 is common to all shares and cancels in the merge
+            row_at = split.partial_row(at_end.piece, head, store ? token : q0, P.num_query_tokens);
+            store = store && NOB_CHECK(row_at < static_cast<size_t>(split.splits) * split.tail_rows, status);
+            if (store) split.lse[row_at] = m_run * P.scale_log2 + log2f(l);
+          }
         }
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -580,14 +596,17 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           tmem_ld32(o_addr + 32 * c, o);
           tc_wait_ld();
           if (store) {
+            float r[32];
 #pragma unroll
-            for (int e = 0; e < 32; e += 8) {
-              uint4 v;
-              v.x = pack_bf16(__uint_as_float(o[e]) * factor, __uint_as_float(o[e + 1]) * factor);
-              v.y = pack_bf16(__uint_as_float(o[e + 2]) * factor, __uint_as_float(o[e + 3]) * factor);
-              v.z = pack_bf16(__uint_as_float(o[e + 4]) * factor, __uint_as_float(o[e + 5]) * factor);
-              v.w = pack_bf16(__uint_as_float(o[e + 6]) * factor, __uint_as_float(o[e + 7]) * factor);
-              *reinterpret_cast<uint4*>(dst + 32 * c + e) = v;
+            for (int e = 0; e < 32; ++e) r[e] = __uint_as_float(o[e]) * factor;
+            if (divided) {
+              split.store(row_at, 32 * c, r);
+            } else {
+#pragma unroll
+              for (int e = 0; e < 32; e += 8)
+                *reinterpret_cast<uint4*>(dst + 32 * c + e) =
+                    make_uint4(pack_bf16(r[e], r[e + 1]), pack_bf16(r[e + 2], r[e + 3]), pack_bf16(r[e + 4], r[e + 5]),
+                               pack_bf16(r[e + 6], r[e + 7]));
             }
           }
         }
@@ -603,7 +622,8 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 int launch_nvfp4(bool sol, const char* name, int num_query_tokens, int num_kv_tokens, int head_offset, const void* query,
                  const void* key, const void* value, const void* query_scales, const void* key_scales,
                  const void* value_scales, float query_global, float key_global, float value_global,
-                 const void* selected, void* output, void* state, int heads, int total_heads, void* stream) {
+                 const void* selected, void* output, void* state, int heads, int total_heads, int unit_rows, int kv_splits,
+                 int tail_units, void* workspace, size_t workspace_bytes, void* stream) {
   NOB_REQUIRE(num_query_tokens > 0 && num_kv_tokens > 0 && heads > 0 && total_heads > 0, "%s: sizes must be positive", name);
   NOB_REQUIRE(head_offset >= 0 && head_offset <= total_heads - heads, "%s: head_offset %d outside [0, %d]", name,
               head_offset, total_heads - heads);
@@ -613,13 +633,17 @@ int launch_nvfp4(bool sol, const char* name, int num_query_tokens, int num_kv_to
   NOB_REQUIRE(query_global > 0.f && key_global > 0.f && value_global > 0.f, "%s: global scales must be positive", name);
   NOB_REQUIRE(!sol || (num_kv_tokens + 63) / 64 <= kMaxTiles, "%s: %d key tokens exceed the %d this kernel lists", name,
               num_kv_tokens, kMaxTiles * 64);
+  KeySplit split;
+  int rc;
+  if (!sol && (rc = make_key_split(&split, name, num_query_tokens, num_kv_tokens, heads, unit_rows, kv_splits, tail_units,
+                                   true, workspace, workspace_bytes)))
+    return rc;
   uint32_t* status = status_word_device_ptr();
   if (!status) return fail(kCudaError, "%s: no current CUDA device", name);
   const uint64_t q_rows = (static_cast<uint64_t>(num_query_tokens) + 127) / 128 * 128;
   const uint64_t k_rows = (static_cast<uint64_t>(num_kv_tokens) + 127) / 128 * 128;
 
   CUtensorMap mq, mk, mv;
-  int rc;
   // Q, K: [heads][rows][64 bytes]; V: [heads][128 channels][k_rows / 2 bytes]
   if ((rc = make_tensor_map_3d(&mq, CU_TENSOR_MAP_DATA_TYPE_UINT8, query, 64, q_rows, heads, 64, q_rows * 64, 64, kTile, 1,
                                CU_TENSOR_MAP_SWIZZLE_64B)))
@@ -649,9 +673,12 @@ int launch_nvfp4(bool sol, const char* name, int num_query_tokens, int num_kv_to
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (err != cudaSuccess)
     return fail(kCudaError, "%s: cannot reserve %zu B of shared memory: %s", name, smem, cudaGetErrorString(err));
-  dim3 grid((num_query_tokens + 2 * kTile - 1) / (2 * kTile), heads);
-  kernel<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(mq, mk, mv, params);
-  return check_launch(name);
+  const dim3 grid = sol ? dim3((num_query_tokens + 2 * kTile - 1) / (2 * kTile), heads) : dim3(key_split_blocks(split, heads));
+  kernel<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(mq, mk, mv, params, split);
+  if ((rc = check_launch(name)) || !split.tail_rows) return rc;
+  OutRoute route = {};
+  route.peer[0] = static_cast<__nv_bfloat16*>(output);
+  return launch_merge_splits(split, route, num_query_tokens, total_heads, head_offset, stream);
 }
 
 }  // namespace
@@ -670,7 +697,7 @@ extern "C" int nob200_dense_nvfp4_attention_d128(int num_query_tokens, int num_k
   (void)workspace, (void)workspace_bytes;
   return launch_nvfp4(false, "dense_nvfp4_attention_d128", num_query_tokens, num_kv_tokens, head_offset, query, key, value,
                       query_scales, key_scales, value_scales, 1.0f, 1.0f, 1.0f, nullptr, output, nullptr, heads,
-                      total_heads, stream);
+                      total_heads, 2 * kTile, 1, 0, nullptr, 0, stream);
 }
 
 extern "C" int nob200_dense_nvfp4_attention_d128_global(int num_query_tokens, int num_kv_tokens, int head_offset,
@@ -682,7 +709,19 @@ extern "C" int nob200_dense_nvfp4_attention_d128_global(int num_query_tokens, in
   (void)workspace, (void)workspace_bytes;
   return launch_nvfp4(false, "dense_nvfp4_attention_d128", num_query_tokens, num_kv_tokens, head_offset, query, key, value,
                       query_scales, key_scales, value_scales, query_global, key_global, value_global, nullptr, output,
-                      nullptr, heads, total_heads, stream);
+                      nullptr, heads, total_heads, 2 * kTile, 1, 0, nullptr, 0, stream);
+}
+
+extern "C" int nob200_dense_nvfp4_attention_d128_units(int num_query_tokens, int num_kv_tokens, int head_offset,
+                                                      const void* query, const void* key, const void* value,
+                                                      const void* query_scales, const void* key_scales,
+                                                      const void* value_scales, float query_global, float key_global,
+                                                      float value_global, void* output, int heads, int total_heads,
+                                                      int unit_rows, int kv_splits, int tail_units, void* workspace,
+                                                      size_t workspace_bytes, void* stream) {
+  return launch_nvfp4(false, "dense_nvfp4_attention_d128", num_query_tokens, num_kv_tokens, head_offset, query, key, value,
+                      query_scales, key_scales, value_scales, query_global, key_global, value_global, nullptr, output,
+                      nullptr, heads, total_heads, unit_rows, kv_splits, tail_units, workspace, workspace_bytes, stream);
 }
 
 extern "C" int nob200_sol_nvfp4_attention_d128(int num_query_tokens, int num_kv_tokens, int head_offset,
@@ -694,5 +733,5 @@ extern "C" int nob200_sol_nvfp4_attention_d128(int num_query_tokens, int num_kv_
   (void)workspace, (void)workspace_bytes;
   return launch_nvfp4(true, "sol_nvfp4_attention_d128", num_query_tokens, num_kv_tokens, head_offset, query, key, value,
                       query_scales, key_scales, value_scales, 1.0f, 1.0f, 1.0f, selected, output, state, heads,
-                      total_heads, stream);
+                      total_heads, 2 * kTile, 1, 0, nullptr, 0, stream);
 }

@@ -12,7 +12,7 @@ from __future__ import annotations
 
 import ctypes
 import dataclasses
-from typing import Literal
+from typing import Literal, NamedTuple
 
 from pydantic import Field
 
@@ -32,6 +32,9 @@ class DenseBf16AttentionConfig(Config):
     threads: Literal[64, 128, 256, 384] = 384
     # key tiles divided over this many CTAs per (256 query rows, head); > 1 needs `workspace`
     kv_splits: int = Field(default=1, ge=1, le=64)
+    # > 0: only the last so many units (`query_rows` rows of one head) have their keys divided, the others run whole
+    tail_units: int = Field(default=0, ge=0)
+    query_rows: Literal[128, 256] = 256
 
 
 def choose_kv_splits(num_tokens: int, heads: int, sm_count: int = 148, num_kv_tokens: int | None = None) -> int:
@@ -63,6 +66,57 @@ def splitkv_workspace_bytes(num_tokens: int, heads: int, kv_splits: int) -> int:
         return 0
     share = num_tokens * heads
     return (kv_splits * share * 256 + 255) // 256 * 256 + kv_splits * share * 4
+
+
+class UnitPlan(NamedTuple):
+    """How a dense launch becomes CTAs: rows per unit, key shares of the last ``tail_units`` units."""
+
+    query_rows: int
+    kv_splits: int
+    tail_units: int
+
+
+def plan_units(num_tokens: int, heads: int, num_kv_tokens: int | None = None, sm_count: int = 148) -> UnitPlan:
+    """Units and key shares of a dense launch, so that its last wave of CTAs fills the SMs.
+
+    A unit is 256 (or 128) query rows of one head on one SM.  The units past the last full wave, or those and one wave
+    more, may have their keys divided.  Times are counted in key tiles of a 256-row unit (1.6 us): a 128-row unit
+    takes 0.72 of one per key tile; a CTA costs 4 beside its tiles (launch, first loads, pipeline fill, epilogue: 6-7
+    us), the merge 2.5 and 0.025 per 256-row share (fp32 rows written and read through L2).  The plain launch (256 rows,
+    no shares) stays unless the estimate falls by 2 %.
+    """
+    tiles = -(-(num_tokens if num_kv_tokens is None else num_kv_tokens) // 128)
+    best, plan = None, UnitPlan(256, 1, 0)
+    for rows, step in ((256, 1.0), (128, 0.72)):
+        units = -(-num_tokens // rows) * heads
+        if rows == 128 and units >= sm_count:
+            continue  # one query tile per SM at a time: only where SMs are left over anyway
+        waves, rest = divmod(units, sm_count)
+        whole = (waves + (rest > 0)) * (tiles * step + 4)
+        if best is None:
+            best = 0.98 * whole
+        elif whole < best:
+            best, plan = whole, UnitPlan(rows, 1, 0)
+        for tail in (rest, rest + sm_count):
+            if not 0 < tail <= units:
+                continue
+            for splits in range(2, min(24, tiles // 4) + 1):
+                rounds = -(-tail * splits // sm_count)
+                cost = (units - tail) // sm_count * (tiles * step + 4) + rounds * (-(-tiles // splits) * step + 4)
+                cost += 2.5 + 0.025 * tail * splits * rows / 256
+                if cost < best:
+                    best, plan = cost, UnitPlan(rows, splits, tail)
+    return plan
+
+
+def key_share_workspace_bytes(num_tokens: int, heads: int, plan: UnitPlan) -> int:
+    """Scratch of the fp32 shares of the last ``tail_units`` units (0: of all units)."""
+    if plan.kv_splits <= 1:
+        return 0
+    q_tiles = -(-num_tokens // plan.query_rows)
+    head, tile = divmod(q_tiles * heads - plan.tail_units if plan.tail_units else 0, q_tiles)
+    rows = plan.kv_splits * ((heads - head) * num_tokens - tile * plan.query_rows)
+    return (rows * 512 + 255) // 256 * 256 + rows * 4
 
 
 @dataclasses.dataclass(frozen=True, slots=True)
@@ -125,16 +179,22 @@ class DenseBf16AttentionKernel(
 
     def compile(self) -> None:
         if self.compiled is None:
-            self.compiled = (_lib.symbol(type(self).symbol), _lib.symbol(type(self).symbol + "_splitkv"))
+            name = type(self).symbol
+            self.compiled = (_lib.symbol(name), _lib.symbol(name + "_splitkv"), _lib.symbol(name + "_units"))
 
     def _launch(self, function, stream: int) -> int:
         a, w = self.arguments, self.workload
-        plain, split = function
-        splits = self.config.kv_splits
-        if splits > 1:
-            need = splitkv_workspace_bytes(w.num_tokens, w.heads, splits)
-            assert a.workspace is not None and a.workspace.num_bytes >= need, "kv_splits > 1 needs workspace"
-            return split(
+        plain, split, by_units = function
+        c = self.config
+        plan = UnitPlan(c.query_rows, c.kv_splits, c.tail_units)
+        units = plan.tail_units > 0 or plan.query_rows != 256
+        if units or plan.kv_splits > 1:
+            if units:
+                need = key_share_workspace_bytes(w.num_tokens, w.heads, plan)
+            else:
+                need = splitkv_workspace_bytes(w.num_tokens, w.heads, plan.kv_splits)
+            assert need == 0 or (a.workspace is not None and a.workspace.num_bytes >= need), "kv_splits > 1 needs workspace"
+            return (by_units if units else split)(
                 ctypes.c_int(w.num_tokens),
                 ctypes.c_int(a.head_offset),
                 _lib.ptr(a.query),
@@ -143,9 +203,9 @@ class DenseBf16AttentionKernel(
                 _lib.ptr(a.output),
                 ctypes.c_int(w.heads),
                 ctypes.c_int(w.total_heads),
-                ctypes.c_int(splits),
+                *((ctypes.c_int(x) for x in plan) if units else (ctypes.c_int(plan.kv_splits),)),
                 _lib.ptr(a.workspace),
-                ctypes.c_size_t(a.workspace.num_bytes),
+                ctypes.c_size_t(a.workspace.num_bytes if a.workspace is not None else 0),
                 ctypes.c_void_p(stream),
             )
         function = plain

@@ -21,7 +21,7 @@ from pydantic import Field
 
 from nano_omni_b200 import _lib
 from nano_omni_b200.core import Arguments, Config, DType, Kernel, MmaType, TensorDesc, Workload, require_tensor
-from nano_omni_b200.kernels.dense_bf16 import splitkv_workspace_bytes
+from nano_omni_b200.kernels.dense_bf16 import UnitPlan, key_share_workspace_bytes, splitkv_workspace_bytes
 
 
 class DenseInt8Fp8AttentionWorkload(Workload):
@@ -38,6 +38,9 @@ class DenseInt8Fp8AttentionConfig(Config):
     threads: Literal[64, 128, 256, 384] = 384
     # key tiles divided over this many CTAs per (256 query rows, head); > 1 needs `workspace`
     kv_splits: int = Field(default=1, ge=1, le=64)
+    # > 0: only the last so many units (`query_rows` rows of one head) have their keys divided, the others run whole
+    tail_units: int = Field(default=0, ge=0)
+    query_rows: Literal[128, 256] = 256
 
 
 @dataclasses.dataclass(frozen=True, slots=True)
@@ -123,13 +126,22 @@ class DenseInt8Fp8AttentionKernel(
         count = 2 * arguments.heads * arguments.num_query_tokens * arguments.num_kv_tokens * 128
         return {MmaType.I8I8I32: count, MmaType.F8F8F32: count}
 
+    def compile(self) -> None:
+        if self.compiled is None:
+            self.compiled = (_lib.symbol(type(self).symbol), _lib.symbol("nob200_dense_int8_fp8_d128_units"))
+
     def _launch(self, function, stream: int) -> int:
         a = self.arguments
-        splits = self.config.kv_splits
-        if splits > 1:
-            need = splitkv_workspace_bytes(a.num_query_tokens, a.heads, splits)
-            assert a.workspace is not None and a.workspace.num_bytes >= need, "kv_splits > 1 needs workspace"
-        return function(
+        split, by_units = function
+        c = self.config
+        plan = UnitPlan(c.query_rows, c.kv_splits, c.tail_units)
+        units = plan.tail_units > 0 or plan.query_rows != 256
+        if units:
+            need = key_share_workspace_bytes(a.num_query_tokens, a.heads, plan)
+        else:
+            need = splitkv_workspace_bytes(a.num_query_tokens, a.heads, plan.kv_splits)
+        assert need == 0 or (a.workspace is not None and a.workspace.num_bytes >= need), "kv_splits > 1 needs workspace"
+        return (by_units if units else split)(
             ctypes.c_int(a.num_kv_tokens),
             ctypes.c_int(a.num_query_tokens),
             _lib.ptr(a.query),
@@ -142,8 +154,8 @@ class DenseInt8Fp8AttentionKernel(
             ctypes.c_int(a.heads),
             ctypes.c_int(a.query_block),
             ctypes.c_int(a.key_block),
-            ctypes.c_int(splits),
-            _lib.ptr(a.workspace) if splits > 1 else ctypes.c_void_p(0),
-            ctypes.c_size_t(a.workspace.num_bytes if splits > 1 else 0),
+            *((ctypes.c_int(x) for x in plan) if units else (ctypes.c_int(plan.kv_splits),)),
+            _lib.ptr(a.workspace) if need else ctypes.c_void_p(0),
+            ctypes.c_size_t(a.workspace.num_bytes if need else 0),
             ctypes.c_void_p(stream),
         )

@@ -12,11 +12,13 @@ from __future__ import annotations
 
 import ctypes
 import dataclasses
+from typing import Literal
 
 from pydantic import Field
 
 from nano_omni_b200 import _lib
 from nano_omni_b200.core import Arguments, Config, DType, Kernel, MmaType, TensorDesc, Workload, require_tensor
+from nano_omni_b200.kernels.dense_bf16 import UnitPlan, key_share_workspace_bytes
 
 
 class DenseNvfp4Workload(Workload):
@@ -30,6 +32,10 @@ class DenseNvfp4Config(Config):
     tile_query_tokens: int = 128
     tile_kv_tokens: int = 128
     threads: int = 384
+    # keys of the last `tail_units` units (`query_rows` rows of one head; 0: all) over so many CTAs; > 1 needs `workspace`
+    kv_splits: int = Field(default=1, ge=1, le=64)
+    tail_units: int = Field(default=0, ge=0)
+    query_rows: Literal[128, 256] = 256
 
 
 @dataclasses.dataclass(frozen=True, slots=True)
@@ -123,9 +129,19 @@ class DenseNvfp4Kernel(Kernel[DenseNvfp4Arguments, DenseNvfp4Workload, DenseNvfp
         workload = cls.make_workload(arguments)
         return {MmaType.F4F4F32: 4 * workload.heads * workload.num_query_tokens * workload.num_kv_tokens * 128}
 
+    def compile(self) -> None:
+        if self.compiled is None:
+            self.compiled = (_lib.symbol(type(self).symbol), _lib.symbol("nob200_dense_nvfp4_attention_d128_units"))
+
     def _launch(self, function, stream: int) -> int:
         a, w = self.arguments, self.workload
-        return function(
+        plain, by_units = function
+        c = self.config
+        plan = UnitPlan(c.query_rows, c.kv_splits, c.tail_units)
+        units = plan.kv_splits > 1 or plan.query_rows != 256
+        need = key_share_workspace_bytes(w.num_query_tokens, w.heads, plan)
+        assert need == 0 or (a.workspace is not None and a.workspace.num_bytes >= need), "kv_splits > 1 needs workspace"
+        return (by_units if units else plain)(
             ctypes.c_int(w.num_query_tokens),
             ctypes.c_int(w.num_kv_tokens),
             ctypes.c_int(a.head_offset),
@@ -141,7 +157,8 @@ class DenseNvfp4Kernel(Kernel[DenseNvfp4Arguments, DenseNvfp4Workload, DenseNvfp
             _lib.ptr(a.output),
             ctypes.c_int(w.heads),
             ctypes.c_int(w.total_heads),
-            ctypes.c_void_p(0),
-            ctypes.c_size_t(0),
+            *((ctypes.c_int(x) for x in plan) if units else ()),
+            _lib.ptr(a.workspace) if need else ctypes.c_void_p(0),
+            ctypes.c_size_t(a.workspace.num_bytes if need else 0),
             ctypes.c_void_p(stream),
         )

@@ -35,7 +35,9 @@ from nano_omni_b200.kernels.dense_bf16 import (
     DenseBf16AttentionArguments,
     DenseBf16AttentionConfig,
     DenseBf16AttentionKernel,
-    choose_kv_splits,
+    UnitPlan,
+    key_share_workspace_bytes,
+    plan_units,
     splitkv_workspace_bytes,
 )
 from nano_omni_b200.kernels.dense_int8_fp8 import (
@@ -43,7 +45,7 @@ from nano_omni_b200.kernels.dense_int8_fp8 import (
     DenseInt8Fp8AttentionConfig,
     DenseInt8Fp8AttentionKernel,
 )
-from nano_omni_b200.kernels.dense_nvfp4 import DenseNvfp4Arguments, DenseNvfp4Kernel, DenseNvfp4Workload
+from nano_omni_b200.kernels.dense_nvfp4 import DenseNvfp4Arguments, DenseNvfp4Config, DenseNvfp4Kernel
 from nano_omni_b200.kernels.matmul import (
     ConvRotInt8Arguments,
     ConvRotInt8Kernel,
@@ -355,24 +357,36 @@ class _SliceAttention(Op):
 
 
 class DenseBf16Attention(_SliceAttention):
-    """One launch; key splits (and their workspace) chosen for the slice when it leaves SMs idle."""
+    """One launch; the keys of its last units are divided (``plan_units``) when they would leave SMs idle."""
 
     def __init__(self, query, key, value, *, total_heads: int, head_offset: int = 0, kv_splits: int | None = None,
                  rotation: Rotation | None = None):  # fmt: skip
         super().__init__(query, key, value, total_heads=total_heads, head_offset=head_offset, rotation=rotation)
-        self.kv_splits = kv_splits if kv_splits is not None else choose_kv_splits(self.rows, self.heads)
+        # an explicit count divides the keys of every unit
+        self.units = UnitPlan(256, kv_splits, 0) if kv_splits is not None else plan_units(self.rows, self.heads)
+        self.kv_splits = self.units.kv_splits
 
     def kernels(self, scratch: ScratchLayout) -> list[Kernel]:
         sequence = KernelSequence(scratch)
         query, key, value = (t.view(self.head_shape) for t in self.prepared_inputs(sequence))
-        need = splitkv_workspace_bytes(self.rows, self.heads, self.kv_splits)
+        if self.units.tail_units:
+            need = key_share_workspace_bytes(self.rows, self.heads, self.units)
+        else:
+            need = splitkv_workspace_bytes(self.rows, self.heads, self.kv_splits)
         workspace = sequence.temporary("splitkv", DType.U8, (need,)) if need else None
         sequence.emit(
             DenseBf16AttentionKernel,
             DenseBf16AttentionArguments(query, key, value, self.bound_outputs[0], self.head_offset, workspace),
-            DenseBf16AttentionConfig(kv_splits=self.kv_splits),
+            DenseBf16AttentionConfig(**self.units._asdict()),
         )
         return sequence.calls
+
+
+def _units(sequence: KernelSequence, rows: int, heads: int, kv_rows: int) -> tuple[dict, TensorDesc | None]:
+    """Config fields of a dense launch's units and key shares, and the scratch of the shares."""
+    plan = plan_units(rows, heads, kv_rows)
+    need = key_share_workspace_bytes(rows, heads, plan)
+    return plan._asdict(), sequence.temporary("splitkv", DType.U8, (need,)) if need else None
 
 
 def _quantise_key_value_int8(sequence: KernelSequence, key, value, rows: int, heads: int, outputs=None, rotated=False):
@@ -454,12 +468,14 @@ class DenseInt8Fp8Attention(Op):
             sequence, query, mean, self.rows, self.heads, self.rotation, rotated=self.hadamard
         )
         blocks = (128, 128) if self.hadamard else (32, 64)
+        units, workspace = _units(sequence, self.rows, self.heads, self.rows)
         sequence.emit(
             DenseInt8Fp8AttentionKernel,
             DenseInt8Fp8AttentionArguments(
                 query_i8, key_i8, value_fp8, query_scale, key_scale, value_scale, self.bound_outputs[0],
-                self.rows, self.heads, self.rows, *blocks,
+                self.rows, self.heads, self.rows, *blocks, workspace,
             ),
+            DenseInt8Fp8AttentionConfig(**units),
         )
         return sequence.calls
 
@@ -510,17 +526,15 @@ class QuerySlice(Op):
         # queries are not centred, so the statistics slot only needs a valid [1, width] tensor
         unused = sequence.temporary("query.statistics", DType.F32, (1, self.heads * 128))
         query_i8, query_scale = _quantise_query_int8(sequence, query, unused, self.rows, self.heads, self.rotation)
-        # a slice of queries is few CTAs: divide the keys when that fills the last wave of SMs better
-        splits = choose_kv_splits(self.rows, self.heads, num_kv_tokens=self.total_tokens)
-        need = splitkv_workspace_bytes(self.rows, self.heads, splits)
-        workspace = sequence.temporary("splitkv", DType.U8, (need,)) if need else None
+        # a slice of queries is few CTAs: the keys of its last units are divided
+        units, workspace = _units(sequence, self.rows, self.heads, self.total_tokens)
         sequence.emit(
             DenseInt8Fp8AttentionKernel,
             DenseInt8Fp8AttentionArguments(
                 query_i8, key_i8, value_fp8, query_scale, key_scale, value_scale, self.bound_outputs[0],
                 self.total_tokens, self.heads, self.rows, workspace=workspace,
             ),
-            DenseInt8Fp8AttentionConfig(kv_splits=splits),
+            DenseInt8Fp8AttentionConfig(**units),
         )
         return sequence.calls
 
@@ -564,12 +578,14 @@ class DenseNvfp4Attention(_SliceAttention):
         sequence = KernelSequence(scratch)
         query, key, value = self.prepared_inputs(sequence)
         _, operands = _prepare_nvfp4(sequence, query, key, value, self.rows, self.heads, self.global_scales)
+        units, workspace = _units(sequence, self.rows, self.heads, self.rows)
         sequence.emit(
             DenseNvfp4Kernel,
             DenseNvfp4Arguments(
-                *operands, self.bound_outputs[0], self.rows, self.rows, self.head_offset, None,
+                *operands, self.bound_outputs[0], self.rows, self.rows, self.head_offset, workspace,
                 self.global_scales or (1.0, 1.0, 1.0),
             ),
+            DenseNvfp4Config(**units),
         )
         if self.global_scales:
             attended = self.bound_outputs[0]
