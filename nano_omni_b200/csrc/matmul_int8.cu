@@ -11,36 +11,54 @@
 // The BF16 form replaces matmul_bf16 (src/nano_omni/kernels/matmul/matmul_bf16.py:29-160, ref_program :183-207):
 // bf16 operands, fp32 accumulation, value = acc * output_scale, then the same bias / residual / SiLU / multiply.
 //
-// Persistent CTAs, one per SM, walk the output tiles of 128 x 256 (N fastest, so that the CTAs in flight share A
-// panels in L2).  Warp 0: TMA producer, K in chunks of 128 bytes through a 4-stage ring (A 16 KiB + B 32 KiB per
-// stage, 128-byte swizzle, no multicast).  Warp 1: tcgen05 issuer, kind::i8 MMAs of 128 x 256 x 32 (kind::f16 MMAs of
-// 128 x 256 x 16 for bf16: the same 32 bytes of K per instruction) into one of two
-// 256-column 32-bit accumulators in TMEM, so that the MMAs of the next tile run while warps 2-9 drain the previous
-// one: a thread owns one row of one 128-column half, requests its residual / multiply operands, reads 64 columns
-// with tcgen05.ld and applies the epilogue in the ref_program's order with separately rounded fp32 operations.
-// Every wait is bounded.
+// Organisation.  Persistent PAIRS of CTAs (clusters of two) walk output tiles of 256 x BN, N fastest, so that the pairs
+// in flight share A panels in L2.  `tcgen05.mma.cta_group::2` multiplies a tile on both SMs at once: CTA r holds rows
+// 128 r .. of A and rows BN/2 r .. of B in its shared memory and gets rows 128 r .. of the accumulator in its TMEM.  A
+// stage of 128 bytes of K is thus 16 + BN/16 KiB per SM and 2 BN cycles of tensor work; one CTA per tile (128 x 256)
+// needed 48 KiB for 512 cycles, more than the 64 bytes per cycle that an SM reads from L2, and waited for its loads.
+//   warp 0    TMA producer (each CTA its own halves; all copies report to the leader CTA's barrier), 5-stage ring,
+//             128-byte swizzle, no multicast
+//   warp 1    of the leader issues kind::i8 MMAs of 256 x BN x 32 (kind::f16, 256 x BN x 16 for bf16: the same 32 bytes
+//             of K) into one of two 256-column accumulators; its commits release the stage in both CTAs
+//   warps 2-9 drain the other accumulator, a row per thread and 32 columns per step, the epilogue in the ref_program's
+//             order with separately rounded fp32 operations.  The residual arrives by TMA two steps ahead and the
+//             result leaves by TMA, both through the warp's own staging tiles of 32 x 32: a thread per row touches 32
+//             different lines per instruction, and that bounded the products with a short K (LoRA updates).
+// int8 15104 x 5376 x 7168 395 -> 347 us (2 N M K at the measured rate: 346), the rank-64 pair beside it 175 -> 144 us,
+// bf16 512 x 7168 x 5376 42 -> 36 us.
+// BN is 64 .. 256, chosen per shape by tile_width().  Every wait is bounded.
 #include <cuda.h>
 
+#include <atomic>
+
 #include "common.cuh"
+#include "fa_common.cuh"
 #include "tensor_map.cuh"
 #include "../../include/nano_omni_b200.h"
 
 namespace nob200 {
 namespace {
 
-constexpr int kBM = 128, kBN = 256, kBK = 128;  // bytes along K: 128 int8 or 64 bf16 elements
-constexpr int kStages = 4;
-constexpr int kABytes = kBM * kBK, kBBytes = kBN * kBK;
+constexpr int kBM = 256, kBK = 128;  // rows of a tile (both CTAs); bytes along K: 128 int8 or 64 bf16 elements
+constexpr int kMaxBN = 256, kMinBN = 64;
+constexpr int kStages = 5;
+constexpr int kABytes = kBM / 2 * kBK, kBBytes = kMaxBN / 2 * kBK;  // per CTA
 constexpr int kThreads = 320;  // producer, issuer, eight epilogue warps (two per TMEM lane quarter)
+constexpr int kEpilogueWarps = 8;
+constexpr int kStep = 32;         // columns per epilogue step
+constexpr int kStagingTiles = 4;  // per epilogue warp: [32 rows][64 bytes], 64-byte swizzle
+constexpr int kStagingBytes = 32 * kStep * 2;
 constexpr uint32_t kTmemCols = 512;
 
 struct __align__(1024) GemmShared {
   uint8_t a[kStages][kABytes];
   uint8_t b[kStages][kBBytes];
-  uint64_t full[kStages];
+  uint8_t staging[kEpilogueWarps][kStagingTiles][kStagingBytes];
+  uint64_t full[kStages];  // the leader's; counts the bytes of both CTAs
   uint64_t empty[kStages];
   uint64_t acc_full[2];
-  uint64_t acc_empty[2];
+  uint64_t acc_empty[2];  // the leader's; sixteen warps arrive
+  uint64_t residual_full[kEpilogueWarps][kStagingTiles];
   uint32_t tmem_base;
   uint32_t abort;
 };
@@ -53,6 +71,7 @@ struct GemmParams {
   const __nv_bfloat16* multiply;
   __nv_bfloat16* output;
   int m, n, k, use_silu;  // k in bytes of a row
+  int bn;                 // columns of a tile, a multiple of 32
   float output_scale;     // bf16 form only
   uint32_t* status;
 };
@@ -60,17 +79,88 @@ struct GemmParams {
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 
+// ---- CTA pairs
+__device__ __forceinline__ uint32_t pair_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void pair_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// address of the leader CTA's copy of a shared-memory object
+__device__ __forceinline__ uint32_t leader_address(const void* p) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(smem_u32(p)));
+  return r;
+}
+__device__ __forceinline__ void leader_arrive(uint32_t leader_bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(leader_bar) : "memory");
+}
+// a copy into this CTA's shared memory that reports to a barrier of either CTA of the pair
+__device__ __forceinline__ void tma_load_pair(void* dst, const void* tmap, uint32_t bar, int c0, int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
+      "l"(tmap), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+__device__ __forceinline__ void tma_store_3d(const void* tmap, const void* src, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(tmap),
+               "r"(smem_u32(src)), "r"(c0), "r"(c1), "r"(c2)
+               : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+// until at most PENDING of this thread's latest stores still read their source
+template <int PENDING>
+__device__ __forceinline__ void tma_store_wait_read() {
+  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(PENDING) : "memory");
+}
+// the commit arrives at the barrier of the same offset in both CTAs
+__device__ __forceinline__ void commit_pair(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+          smem_u32(bar)),
+      "h"(static_cast<uint16_t>(3))
+      : "memory");
+}
+// D[tmem of both] (+)= A * B over 128 bytes of K: four MMAs, 32 bytes apart in both operands
 template <bool BF16>
-__global__ void __launch_bounds__(kThreads, 1)
+__device__ __forceinline__ void mma_pair_chunk(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+#define NOB_MMA4(KIND)                                                                    \
+  asm volatile(                                                                           \
+      "{\n\t.reg .pred p0, p1;\n\t"                                                       \
+      "setp.ne.b32 p0, %2, 0;\n\tsetp.eq.b32 p1, 0, 0;\n\t"                               \
+      "tcgen05.mma.cta_group::2.kind::" KIND " [%0], %3, %7, %1, p0;\n\t"                 \
+      "tcgen05.mma.cta_group::2.kind::" KIND " [%0], %4, %8, %1, p1;\n\t"                 \
+      "tcgen05.mma.cta_group::2.kind::" KIND " [%0], %5, %9, %1, p1;\n\t"                 \
+      "tcgen05.mma.cta_group::2.kind::" KIND " [%0], %6, %10, %1, p1;\n\t}" ::"r"(d),     \
+      "r"(idesc), "r"(accumulate), "l"(a), "l"(a + 2), "l"(a + 4), "l"(a + 6), "l"(b), "l"(b + 2), "l"(b + 4), \
+      "l"(b + 6)                                                                          \
+      : "memory")
+  if constexpr (BF16) {
+    NOB_MMA4("f16");
+  } else {
+    NOB_MMA4("i8");
+  }
+#undef NOB_MMA4
+}
+
+template <bool BF16>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                   const GemmParams P) {
+              const __grid_constant__ CUtensorMap map_residual, const __grid_constant__ CUtensorMap map_output,
+              const GemmParams P) {
   extern __shared__ uint8_t smem_raw[];
   GemmShared& S = *reinterpret_cast<GemmShared*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = static_cast<int>(pair_rank());
   volatile uint32_t* abort_flag = &S.abort;
   uint32_t* status = P.status;
-  const int m_tiles = (P.m + kBM - 1) / kBM, n_tiles = (P.n + kBN - 1) / kBN;
+  const int bn = P.bn;
+  const int m_tiles = (P.m + kBM - 1) / kBM, n_tiles = (P.n + bn - 1) / bn;
   const int num_tiles = m_tiles * n_tiles;
+  const int first_tile = blockIdx.x >> 1, tile_stride = gridDim.x >> 1;
   const int k_chunks = (P.k + kBK - 1) / kBK;
 
   if (threadIdx.x == 0) {
@@ -80,17 +170,24 @@ matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&S.acc_full[b], 1);
-      mbar_init(&S.acc_empty[b], 8);
+      mbar_init(&S.acc_empty[b], 2 * kEpilogueWarps);
     }
+    for (int w = 0; w < kEpilogueWarps; ++w)
+      for (int i = 0; i < kStagingTiles; ++i) mbar_init(&S.residual_full[w][i], 1);
     S.abort = 0;
     mbar_fence_init();
   }
   if (warp == 0) {
-    tmem_alloc(&S.tmem_base, kTmemCols);
-    tmem_relinquish();
+    __syncwarp();
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&S.tmem_base)),
+                 "r"(kTmemCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
+  __syncwarp();
+  pair_sync();  // the peer's barriers exist before anything reports to them
   tc_fence_after();
   const uint32_t tmem = S.tmem_base;
 
@@ -99,166 +196,208 @@ matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
     if (lane == 0) {
       tma_prefetch_desc(&map_a);
       tma_prefetch_desc(&map_b);
+      const uint32_t stage_bytes = static_cast<uint32_t>(kABytes + bn / 2 * kBK);
       int issued = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
-        const int m0 = (tile / n_tiles) * kBM, n0 = (tile % n_tiles) * kBN;
+      for (int tile = first_tile; ok && tile < num_tiles; tile += tile_stride) {
+        const int m0 = (tile / n_tiles) * kBM + rank * (kBM / 2), n0 = (tile % n_tiles) * bn + rank * (bn / 2);
         for (int kc = 0; kc < k_chunks; ++kc, ++issued) {
           const int st = issued % kStages;
           if (issued >= kStages) {
             ok = mbar_wait(&S.empty[st], ((issued / kStages) - 1) & 1, abort_flag, status, kWaitTimeoutRing);
             if (!ok) break;
           }
-          mbar_expect_tx(&S.full[st], kABytes + kBBytes);
+          // the phase cannot complete before the leader's arrival, so the follower's bytes may come first
+          if (rank == 0) mbar_expect_tx(&S.full[st], 2 * stage_bytes);
+          const uint32_t bar = leader_address(&S.full[st]);
           constexpr int kElementsPerChunk = BF16 ? kBK / 2 : kBK;
-          tma_load_3d(S.a[st], &map_a, &S.full[st], kc * kElementsPerChunk, m0, 0);
-          tma_load_3d(S.b[st], &map_b, &S.full[st], kc * kElementsPerChunk, n0, 0);
+          tma_load_pair(S.a[st], &map_a, bar, kc * kElementsPerChunk, m0, 0);
+          tma_load_pair(S.b[st], &map_b, bar, kc * kElementsPerChunk, n0, 0);
         }
       }
-      if (*abort_flag) {  // gave up: let the copies in flight land before the CTA exits
-        for (int i = (issued > kStages ? issued - kStages : 0); i < issued; ++i) {
-          uint64_t* bar = &S.full[i % kStages];
-          const uint32_t parity = (i / kStages) & 1;
-          for (int spin = 0; spin < (1 << 16) && !mbar_try_wait(bar, parity); ++spin) {
-          }
-        }
-      }
+      // the last commits have reported here before this CTA's barriers go away
+      for (int i = issued > kStages ? issued - kStages : 0; ok && i < issued; ++i)
+        ok = mbar_wait(&S.empty[i % kStages], (i / kStages) & 1, abort_flag, status, kWaitTimeoutRing);
     }
   } else if (warp == 1) {
-    // ---------------------------------------------------------- tcgen05 issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = BF16 ? umma_idesc(kDF32, kFmtBF16, kFmtBF16, 0, 0, kBM, kBN)
-                                      : umma_idesc(kDS32, kFmtS8, kFmtS8, 0, 0, kBM, kBN);
+    // ------------------------------------------ tcgen05 issuer, the leader's: warp-uniform flow, one elected lane
+    if (rank == 0) {
+      const uint32_t idesc = BF16 ? umma_idesc(kDF32, kFmtBF16, kFmtBF16, 0, 0, kBM, bn)
+                                  : umma_idesc(kDS32, kFmtS8, kFmtS8, 0, 0, kBM, bn);
       const uint64_t desc = umma_smem_desc(0, 16, 1024, kSwizzle128B);
       const uint64_t a0 = desc + (smem_u32(S.a[0]) >> 4), b0 = desc + (smem_u32(S.b[0]) >> 4);
       int taken = 0, round = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x, ++round) {
+      for (int tile = first_tile; ok && tile < num_tiles; tile += tile_stride, ++round) {
         const int buf = round & 1;
-        if (round >= 2) {  // the epilogue must have drained this accumulator (its (round / 2)-th use)
-          ok = mbar_wait(&S.acc_empty[buf], ((round >> 1) - 1) & 1, abort_flag, status, kWaitTimeoutSoftmax);
+        if (round >= 2) {  // both CTAs' epilogues must have drained this accumulator (its (round / 2)-th use)
+          ok = warp_rest(&S.acc_empty[buf], ((round >> 1) - 1) & 1, abort_flag, status, kWaitTimeoutSoftmax);
           if (!ok) break;
           tc_fence_after();
         }
-        const uint32_t d = tmem + buf * kBN;
+        const uint32_t d = tmem + buf * kMaxBN;
         for (int kc = 0; kc < k_chunks; ++kc, ++taken) {
           const int st = taken % kStages;
-          ok = mbar_wait(&S.full[st], (taken / kStages) & 1, abort_flag, status, kWaitTimeoutLoad);
+          ok = warp_rest(&S.full[st], (taken / kStages) & 1, abort_flag, status, kWaitTimeoutLoad);
           if (!ok) break;
           tc_fence_after();
-          const uint64_t a = a0 + st * (kABytes >> 4), b = b0 + st * (kBBytes >> 4);
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_ss<BF16 ? 0 : 1>(d, a + 2 * kk, b + 2 * kk, idesc, (kc > 0 || kk > 0) ? 1u : 0u);
-          tc_commit(&S.empty[st]);
+          if (elect_one()) {
+            mma_pair_chunk<BF16>(d, a0 + st * (kABytes >> 4), b0 + st * (kBBytes >> 4), idesc, kc > 0 ? 1u : 0u);
+            commit_pair(&S.empty[st]);
+            if (kc + 1 == k_chunks) commit_pair(&S.acc_full[buf]);
+          }
+          __syncwarp();
         }
-        if (ok) tc_commit(&S.acc_full[buf]);
       }
     }
   } else {
     // ------------------------------------------------------------- epilogue warps
-    const int quarter = warp & 3;         // TMEM lanes [32 quarter, 32 quarter + 32)
-    const int column_half = (warp - 2) >> 2;  // warps 2-5 drain columns 0-127 of the tile, warps 6-9 columns 128-255
-    const int row_in_tile = quarter * 32 + lane;
+    const int quarter = warp & 3;        // TMEM lanes [32 quarter, 32 quarter + 32)
+    const int group = (warp - 2) >> 2;   // steps group, group + 2, ... of a tile
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
+    uint8_t(*staging)[kStagingBytes] = S.staging[warp - 2];
+    uint64_t* residual_full = S.residual_full[warp - 2];
+    const int steps = bn / kStep;
+    const int row_in_tile = rank * (kBM / 2) + quarter * 32;  // of the warp's first row
+    int used = 0;  // steps that lie inside the output: number `used` works in staging tile used % kStagingTiles
+    // residual tiles requested so far, and the step the next request looks at
+    int requested = 0, next_tile = first_tile, next_c = group;
+    auto request = [&]() {
+      while (next_tile < num_tiles) {
+        const int row0 = (next_tile / n_tiles) * kBM + row_in_tile, col0 = (next_tile % n_tiles) * bn + next_c * kStep;
+        next_c += 2;
+        if (next_c >= steps) next_c = group, next_tile += tile_stride;
+        if (row0 < P.m && col0 < P.n) {
+          if (lane == 0) {
+            const int tile = requested % kStagingTiles;
+            tma_store_wait_read<1>();  // the store that last left this staging tile is at least two stores back
+            mbar_expect_tx(&residual_full[tile], kStagingBytes);
+            tma_load_3d(staging[tile], &map_residual, &residual_full[tile], col0, row0, 0);
+          }
+          ++requested;
+          return;
+        }
+      }
+    };
+    if (P.residual) {
+      request();
+      request();
+    }
     int round = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x, ++round) {
+    for (int tile = first_tile; ok && tile < num_tiles; tile += tile_stride, ++round) {
       const int buf = round & 1;
-      const int m0 = (tile / n_tiles) * kBM, n0 = (tile % n_tiles) * kBN;
-      const int row = m0 + row_in_tile;
+      const int row0 = (tile / n_tiles) * kBM + row_in_tile, n0 = (tile % n_tiles) * bn;
+      const int row = row0 + lane;
       const bool live = row < P.m;
       const float in_scale = (!BF16 && live) ? P.input_scale[row] : 0.f;
-      ok = __all_sync(0xffffffffu, mbar_wait(&S.acc_full[buf], (round >> 1) & 1, abort_flag, status, kWaitTimeoutMma));
+      const size_t row_offset = static_cast<size_t>(live ? row : 0) * P.n;
+      ok = warp_rest(&S.acc_full[buf], (round >> 1) & 1, abort_flag, status, kWaitTimeoutMma);
       if (!ok) break;
       tc_fence_after();
-      const size_t row_offset = static_cast<size_t>(live ? row : 0) * P.n;
 #pragma unroll 1
-      for (int c = column_half * (kBN / 128); c < (column_half + 1) * (kBN / 128); ++c) {
-        // 64 columns per step.  Residual and multiply operands are requested before the accumulator is read, all at
-        // once: their latency, not their bandwidth, bounds the epilogue of a short-K product.
-        const int col0 = n0 + 64 * c;
-        uint4 res[8], mul[8];
-#pragma unroll
-        for (int g = 0; g < 8; ++g) {
-          const bool in = live && col0 + 8 * g < P.n;
-          res[g] = (in && P.residual) ? *reinterpret_cast<const uint4*>(P.residual + row_offset + col0 + 8 * g)
-                                      : make_uint4(0, 0, 0, 0);
-          mul[g] = (in && P.multiply) ? *reinterpret_cast<const uint4*>(P.multiply + row_offset + col0 + 8 * g)
-                                      : make_uint4(0, 0, 0, 0);
+      for (int c = group; c < steps; c += 2) {
+        const int col0 = n0 + kStep * c;
+        const bool inside = row0 < P.m && col0 < P.n;  // warp-uniform
+        uint8_t* mine = staging[used % kStagingTiles] + lane * 64;
+        auto piece = [&](int g) { return reinterpret_cast<uint4*>(mine + ((g ^ ((lane >> 1) & 3)) << 4)); };
+        if (inside) {
+          if (P.residual) {
+            request();
+            ok = warp_rest(&residual_full[used % kStagingTiles], (used / kStagingTiles) & 1, abort_flag, status,
+                           kWaitTimeoutLoad);
+          } else {
+            if (lane == 0) tma_store_wait_read<kStagingTiles - 1>();
+            __syncwarp();
+          }
         }
-        uint32_t acc[64];
-        __syncwarp();  // lanes that skipped the stores of the previous step rejoin before the aligned TMEM load
-        tmem_ld32(tmem + lane_base + buf * kBN + 64 * c, *reinterpret_cast<uint32_t(*)[32]>(&acc[0]));
-        tmem_ld32(tmem + lane_base + buf * kBN + 64 * c + 32, *reinterpret_cast<uint32_t(*)[32]>(&acc[32]));
+        uint32_t acc[kStep];
+        __syncwarp();
+        tmem_ld32(tmem + lane_base + buf * kMaxBN + kStep * c, acc);
         tc_wait_ld();
-        if (c == (column_half + 1) * (kBN / 128) - 1) {
+        if (c + 2 >= steps) {
           // the accumulator is in registers: the issuer may start the tile after next on it
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&S.acc_empty[buf]);
+          if (lane == 0) leader_arrive(leader_address(&S.acc_empty[buf]));
         }
-        if (!live || col0 >= P.n) continue;
+        if (!ok) break;
+        if (!inside) continue;
 #pragma unroll
-        for (int g = 0; g < 8; ++g) {  // 8 columns = 16 bytes of bf16 at a time
+        for (int g = 0; g < 4; ++g) {  // 8 columns = 16 bytes of bf16 at a time
           const int col = col0 + 8 * g;
-          if (col >= P.n) break;
-          float v[8];
-          if constexpr (BF16) {
+          if (col < P.n) {
+            float v[8];
+            if constexpr (BF16) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = __fmul_rn(__uint_as_float(acc[8 * g + i]), P.output_scale);
-          } else {
-            const float4 w0 = *reinterpret_cast<const float4*>(P.weight_scale + col);
-            const float4 w1 = *reinterpret_cast<const float4*>(P.weight_scale + col + 4);
-            const float ws[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+              for (int i = 0; i < 8; ++i) v[i] = __fmul_rn(__uint_as_float(acc[8 * g + i]), P.output_scale);
+            } else {
+              const float4 w0 = *reinterpret_cast<const float4*>(P.weight_scale + col);
+              const float4 w1 = *reinterpret_cast<const float4*>(P.weight_scale + col + 4);
+              const float ws[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-              v[i] = __fmul_rn(__fmul_rn(static_cast<float>(static_cast<int>(acc[8 * g + i])), ws[i]), in_scale);
-          }
-          if (P.bias) {
-            const uint4 raw = *reinterpret_cast<const uint4*>(P.bias + col);
-            const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+              for (int i = 0; i < 8; ++i)
+                v[i] = __fmul_rn(__fmul_rn(static_cast<float>(static_cast<int>(acc[8 * g + i])), ws[i]), in_scale);
+            }
+            if (P.bias) {
+              const uint4 raw = *reinterpret_cast<const uint4*>(P.bias + col);
+              const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                v[2 * i] = __fadd_rn(v[2 * i], bf16_lo(w[i]));
+                v[2 * i + 1] = __fadd_rn(v[2 * i + 1], bf16_hi(w[i]));
+              }
+            }
+            if (P.residual) {
+              const uint4 raw = *piece(g);
+              const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                v[2 * i] = __fadd_rn(v[2 * i], bf16_lo(w[i]));
+                v[2 * i + 1] = __fadd_rn(v[2 * i + 1], bf16_hi(w[i]));
+              }
+            }
+            if (P.use_silu) {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) v[i] = __fdividef(v[i], 1.0f + __expf(-v[i]));
+            }
+            if (P.multiply) {
+              const uint4 raw = live ? *reinterpret_cast<const uint4*>(P.multiply + row_offset + col) : make_uint4(0, 0, 0, 0);
+              const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                v[2 * i] = __fmul_rn(v[2 * i], bf16_lo(w[i]));
+                v[2 * i + 1] = __fmul_rn(v[2 * i + 1], bf16_hi(w[i]));
+              }
+            }
+            uint32_t o[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              v[2 * i] = __fadd_rn(v[2 * i], bf16_lo(w[i]));
-              v[2 * i + 1] = __fadd_rn(v[2 * i + 1], bf16_hi(w[i]));
+              const __nv_bfloat162 pair = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+              o[i] = *reinterpret_cast<const uint32_t*>(&pair);
             }
+            *piece(g) = make_uint4(o[0], o[1], o[2], o[3]);
           }
-          if (P.residual) {
-            const uint32_t w[4] = {res[g].x, res[g].y, res[g].z, res[g].w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              v[2 * i] = __fadd_rn(v[2 * i], bf16_lo(w[i]));
-              v[2 * i + 1] = __fadd_rn(v[2 * i + 1], bf16_hi(w[i]));
-            }
-          }
-          if (P.use_silu) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = __fdividef(v[i], 1.0f + __expf(-v[i]));
-          }
-          if (P.multiply) {
-            const uint32_t w[4] = {mul[g].x, mul[g].y, mul[g].z, mul[g].w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              v[2 * i] = __fmul_rn(v[2 * i], bf16_lo(w[i]));
-              v[2 * i + 1] = __fmul_rn(v[2 * i + 1], bf16_hi(w[i]));
-            }
-          }
-          uint32_t o[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const __nv_bfloat162 pair = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-            o[i] = *reinterpret_cast<const uint32_t*>(&pair);
-          }
-          *reinterpret_cast<uint4*>(P.output + row_offset + col) = make_uint4(o[0], o[1], o[2], o[3]);
         }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) tma_store_3d(&map_output, staging[used % kStagingTiles], col0, row0, 0);  // clips past the edges
+        ++used;
       }
     }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
 
+  if (*abort_flag) {  // gave up: let the copies in flight land before the pair exits (a microsecond; one millisecond)
+    for (const uint64_t start = global_timer_ns(); global_timer_ns() - start < 1000000ull;) {
+    }
+  }
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, kTmemCols);
+  __syncwarp();
+  pair_sync();  // nothing of the pair reads or reports to this CTA's shared memory any more
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
 }
 
 }  // namespace
@@ -267,17 +406,50 @@ matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
 namespace nob200 {
 namespace {
 
+// Columns of a tile: the width whose waves over the pairs cost least.  A chunk of K takes 2 BN cycles of tensor work or,
+// below 256 columns, the load of its 16 KiB + BN/2 x 128 bytes per SM at 64 bytes per cycle; a tile's start and end
+// count as some chunks' worth.  Wide tiles win on long calls; a call of one short wave is spread over more pairs.
+int tile_width(int m, int n, int k_chunks, int pairs) {
+  const long long m_tiles = (m + kBM - 1) / kBM;
+  int best = kMaxBN;
+  long long best_cost = 0;
+  for (int bn = kMaxBN; bn >= kMinBN; bn -= 32) {
+    const long long tiles = m_tiles * ((n + bn - 1) / bn);
+    const long long waves = (tiles + pairs - 1) / pairs;
+    const long long cost = waves * (static_cast<long long>(k_chunks) * (2 * bn > 256 + bn ? 2 * bn : 256 + bn) + 1000);
+    if (bn == kMaxBN || cost < best_cost) best = bn, best_cost = cost;
+  }
+  return best;
+}
+
+// Pairs of CTAs the device holds at once (a property of the device, asked once per device and kernel).
+template <typename Kernel>
+int resident_pairs(Kernel kernel, size_t smem, int device) {
+  static std::atomic<int> known[64];
+  if (device >= 0 && device < 64) {
+    const int pairs = known[device].load(std::memory_order_relaxed);
+    if (pairs > 0) return pairs;
+  }
+  int sms = 148, pairs = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  cudaLaunchAttribute attribute = {};
+  attribute.id = cudaLaunchAttributeClusterDimension;
+  attribute.val.clusterDim.x = 2, attribute.val.clusterDim.y = 1, attribute.val.clusterDim.z = 1;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(sms & ~1), config.blockDim = dim3(kThreads), config.dynamicSmemBytes = smem;
+  config.attrs = &attribute, config.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&pairs, kernel, &config) != cudaSuccess || pairs <= 0) {
+    (void)cudaGetLastError();
+    pairs = sms / 2;
+  }
+  if (device >= 0 && device < 64) known[device].store(pairs, std::memory_order_relaxed);
+  return pairs;
+}
+
 template <bool BF16>
 int launch_matmul(const char* name, int num_tokens, const void* input, const void* weight, int n, int k,
                   GemmParams params, void* stream) {
   const int element = BF16 ? 2 : 1;
-  CUtensorMap ma, mb;
-  const CUtensorMapDataType dtype = BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
-  const uint64_t pitch = static_cast<uint64_t>(k) * element;
-  int rc;
-  if ((rc = make_tensor_map_3d(&ma, dtype, input, k, num_tokens, 1, pitch, pitch * num_tokens, kBK / element, kBM, 1)))
-    return rc;
-  if ((rc = make_tensor_map_3d(&mb, dtype, weight, k, n, 1, pitch, pitch * n, kBK / element, kBN, 1))) return rc;
   params.m = num_tokens;
   params.n = n;
   params.k = k * element;
@@ -289,11 +461,29 @@ int launch_matmul(const char* name, int num_tokens, const void* input, const voi
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (err != cudaSuccess)
     return fail(kCudaError, "%s: cannot reserve %zu B of shared memory: %s", name, smem, cudaGetErrorString(err));
-  int device = 0, sms = 148;
-  if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  const long long tiles = static_cast<long long>((num_tokens + kBM - 1) / kBM) * ((n + kBN - 1) / kBN);
-  const int grid = static_cast<int>(tiles < sms ? tiles : sms);
-  kernel<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(ma, mb, params);
+  int device = 0;
+  cudaGetDevice(&device);
+  const int pairs = resident_pairs(kernel, smem, device);
+  params.bn = tile_width(num_tokens, n, (params.k + kBK - 1) / kBK, pairs);
+
+  CUtensorMap ma, mb, mr, mo;
+  const CUtensorMapDataType dtype = BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
+  const uint64_t pitch = static_cast<uint64_t>(k) * element, out_pitch = static_cast<uint64_t>(n) * 2;
+  int rc;
+  if ((rc = make_tensor_map_3d(&ma, dtype, input, k, num_tokens, 1, pitch, pitch * num_tokens, kBK / element, kBM / 2, 1)))
+    return rc;
+  if ((rc = make_tensor_map_3d(&mb, dtype, weight, k, n, 1, pitch, pitch * n, kBK / element, params.bn / 2, 1))) return rc;
+  auto wide = [&](CUtensorMap* map, const void* base) {
+    return make_tensor_map_3d(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, n, num_tokens, 1, out_pitch,
+                              out_pitch * num_tokens, kStep, 32, 1, CU_TENSOR_MAP_SWIZZLE_64B);
+  };
+  if ((rc = wide(&mo, params.output))) return rc;
+  mr = mo;
+  if (params.residual && (rc = wide(&mr, params.residual))) return rc;
+
+  const long long tiles = static_cast<long long>((num_tokens + kBM - 1) / kBM) * ((n + params.bn - 1) / params.bn);
+  const int grid = 2 * static_cast<int>(tiles < pairs ? tiles : pairs);
+  kernel<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(ma, mb, mr, mo, params);
   return check_launch(name);
 }
 

@@ -4,7 +4,7 @@ INT8 GEMM: bound to ``nob200_matmul_int8``.
 
 Interface of reference ``MatmulInt8Kernel`` (src/nano_omni/kernels/matmul/matmul_int8.py:13-240): same Workload
 and Arguments fields and order, validation and ``tops``.  The Config keeps the reference's tile fields so stored
-configs still validate; the sm_100a kernel has one tile shape (128 x 256 x 128).
+configs still validate; the sm_100a kernel chooses its tile (256 x 64..256 per pair of CTAs) from the shape.
 """
 
 from __future__ import annotations
