@@ -12,7 +12,7 @@
 //   out is rounded to bf16 (stored, or quantised to int8 with one scale per head and 32 tokens).
 // The reference leaves the order of the sum and the kind of reciprocal square root to its compiler (and its two
 // ref_programs differ: mean of squares vs squared vector norm).  Here every step is an IEEE fp32 operation in a
-// fixed order, which the CPU restatement repeats: a row lies on 16 lanes, 8 consecutive channels each; a lane adds
+// fixed order, which the CPU restatement repeats: a row is 16 chunks of 8 consecutive channels; a chunk adds
 // its squares in channel order starting from 0, the 16 partial sums are combined by an xor butterfly with strides
 // 8, 4, 2, 1; divide by 128, add 1e-5, square root, divide 1 by it; products and the sum or difference of the
 // rotation are rounded one by one (no fused multiply-add).
@@ -51,64 +51,89 @@ __device__ __forceinline__ Row8 row8_of(const uint4& raw) {
 
 __device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
-// x[k]: 8 channels [8 lane16, 8 lane16 + 8) of row k; w: the norm weight of those channels.  On return x holds the
-// normalised, rotated rows rounded to bf16 precision.  All 16 lanes of the rows' group must call it.  N rows go
-// through each stage together so that their loads, shuffles and the divide / square root sequences overlap.
+// A row lies on 8 lanes, each with two chunks of 8 channels: lanes 0-5 chunks t and t + 6, the two sides of the rotation's
+// pairs, lanes 6 and 7 the chunks 12, 13 and 14, 15 that pass through.  The rotation then needs no exchange between
+// lanes, and a row costs 5 shuffles per lane (the sum of squares) instead of 12 on twice as many lanes: shuffles and the
+// divide / square root sequence, which every lane repeats, bounded the kernels (16 lanes per row, before / after:
+// 9461 tokens x 14 heads 27 / 20 us, query quantiser 4096 x 24 24 / 20.6 us).
+struct RowPart {
+  Row8 a, b;
+};
+__device__ __forceinline__ int chunk_a(int lane8) { return lane8 < 6 ? lane8 : 2 * lane8; }
+__device__ __forceinline__ int chunk_b(int lane8) { return lane8 < 6 ? lane8 + 6 : 2 * lane8 + 1; }
+
+__device__ __forceinline__ RowPart load_part(const __nv_bfloat16* row, int lane8) {
+  return {load_row8(row + 8 * chunk_a(lane8)), load_row8(row + 8 * chunk_b(lane8))};
+}
+
+__device__ __forceinline__ float sum_of_squares(const Row8& x) {
+  float s = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) s = __fadd_rn(s, __fmul_rn(x.v[i], x.v[i]));
+  return s;
+}
+
+// x[k]: this lane's part of row k; w: the norm weight of those channels.  On return x holds the normalised, rotated rows
+// rounded to bf16 precision.  All lanes of the warp must call it.  N rows go through each stage together so that their
+// loads, shuffles and the divide / square root sequences overlap.
 template <int N, int NW = 1>  // NW = 1: one weight for all rows; NW = N: a weight per row
-__device__ __forceinline__ void norm_rope_rows(Row8 (&x)[N], const Row8 (&w)[NW], const float* __restrict__ cosines,
-                                               const float* __restrict__ sines, const int (&token)[N], int lane16,
+__device__ __forceinline__ void norm_rope_rows(RowPart (&x)[N], const RowPart (&w)[NW], const float* __restrict__ cosines,
+                                               const float* __restrict__ sines, const int (&token)[N], int lane8,
                                                bool use_rope) {
-  // lanes 0-5 hold channels 0-47 (first), lanes 6-11 channels 48-95 (second), lanes 12-15 pass through
-  const int partner = lane16 < 6 ? lane16 + 6 : lane16 - 6;
-  const bool first = lane16 < 6, rotates = use_rope && lane16 < 12;
+  const bool rotates = use_rope && lane8 < 6;
   float4 c[N][2], s[N][2];
   if (rotates) {
 #pragma unroll
     for (int k = 0; k < N; ++k) {
-      const int at = token[k] * 48 + 8 * (first ? lane16 : lane16 - 6);
+      const int at = token[k] * 48 + 8 * lane8;
       c[k][0] = *reinterpret_cast<const float4*>(cosines + at);
       c[k][1] = *reinterpret_cast<const float4*>(cosines + at + 4);
       s[k][0] = *reinterpret_cast<const float4*>(sines + at);
       s[k][1] = *reinterpret_cast<const float4*>(sines + at + 4);
     }
   }
+  // The sums p[0..15] of the chunks go through the butterfly with strides 8, 4, 2, 1: lane t first gets p[t] and p[t + 8].
+  // p[6], p[7] are the second chunks of lanes 0, 1; p[8..11] those of lanes 2-5; p[12..15] lanes 6 and 7.
+  const int from_b = lane8 < 4 ? lane8 + 2 : lane8 == 5 ? 6 : lane8 == 6 ? 0 : lane8 == 7 ? 1 : 4;
+  const int from_a = lane8 == 4 ? 6 : lane8 == 6 ? 7 : lane8;
   float ss[N];
 #pragma unroll
   for (int k = 0; k < N; ++k) {
-    ss[k] = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) ss[k] = __fadd_rn(ss[k], __fmul_rn(x[k].v[i], x[k].v[i]));
+    const float sa = sum_of_squares(x[k].a), sb = sum_of_squares(x[k].b);
+    const float other_b = __shfl_sync(0xffffffffu, sb, from_b, 8), other_a = __shfl_sync(0xffffffffu, sa, from_a, 8);
+    const float low = lane8 < 6 ? sa : other_b;
+    const float high = (lane8 == 4 || lane8 == 6) ? other_a : lane8 == 7 ? sb : other_b;
+    ss[k] = __fadd_rn(low, high);
   }
 #pragma unroll
-  for (int m = 8; m > 0; m >>= 1) {
+  for (int m = 4; m > 0; m >>= 1) {
 #pragma unroll
     for (int k = 0; k < N; ++k) ss[k] = __fadd_rn(ss[k], __shfl_xor_sync(0xffffffffu, ss[k], m));
   }
 #pragma unroll
   for (int k = 0; k < N; ++k) {
     const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fmul_rn(ss[k], 0.0078125f), 1e-5f)));
+    const RowPart& wk = w[NW == 1 ? 0 : k];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) x[k].v[i] = __fmul_rn(__fmul_rn(x[k].v[i], r), w[NW == 1 ? 0 : k].v[i]);
-  }
-  if (use_rope) {
-#pragma unroll
-    for (int k = 0; k < N; ++k) {
+    for (int i = 0; i < 8; ++i) {
+      x[k].a.v[i] = __fmul_rn(__fmul_rn(x[k].a.v[i], r), wk.a.v[i]);
+      x[k].b.v[i] = __fmul_rn(__fmul_rn(x[k].b.v[i], r), wk.b.v[i]);
+    }
+    if (rotates) {
       const float cc[8] = {c[k][0].x, c[k][0].y, c[k][0].z, c[k][0].w, c[k][1].x, c[k][1].y, c[k][1].z, c[k][1].w};
       const float sn[8] = {s[k][0].x, s[k][0].y, s[k][0].z, s[k][0].w, s[k][1].x, s[k][1].y, s[k][1].z, s[k][1].w};
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const float other = __shfl_sync(0xffffffffu, x[k].v[i], partner & 15, 16);
-        if (rotates) {
-          x[k].v[i] = first ? __fsub_rn(__fmul_rn(x[k].v[i], cc[i]), __fmul_rn(other, sn[i]))
-                            : __fadd_rn(__fmul_rn(other, sn[i]), __fmul_rn(x[k].v[i], cc[i]));
-        }
+        const float first = x[k].a.v[i], second = x[k].b.v[i];
+        x[k].a.v[i] = __fsub_rn(__fmul_rn(first, cc[i]), __fmul_rn(second, sn[i]));
+        x[k].b.v[i] = __fadd_rn(__fmul_rn(first, sn[i]), __fmul_rn(second, cc[i]));
       }
     }
-  }
 #pragma unroll
-  for (int k = 0; k < N; ++k) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) x[k].v[i] = round_bf16(x[k].v[i]);
+    for (int i = 0; i < 8; ++i) {
+      x[k].a.v[i] = round_bf16(x[k].a.v[i]);
+      x[k].b.v[i] = round_bf16(x[k].b.v[i]);
+    }
   }
 }
 
@@ -116,145 +141,101 @@ __device__ __forceinline__ uint32_t pack_bf16_pair(float lo, float hi) {
   return (__float_as_uint(lo) >> 16) | (__float_as_uint(hi) & 0xffff0000u);  // both already bf16-representable
 }
 
-// One group of 16 lanes per (token, head) row: 16 rows per CTA round (more rows per group cost occupancy and were
-// measured slower).  In place is allowed.
-__global__ void __launch_bounds__(256)
-head_norm_rope_kernel(const __nv_bfloat16* src, const __nv_bfloat16* __restrict__ weight,
-                      const float* __restrict__ cosines, const float* __restrict__ sines, __nv_bfloat16* dst,
-                      long long rows, int heads, int use_rope) {  // src and dst may be the same tensor
-  constexpr int kRows = 1;
-  const int lane16 = threadIdx.x & 15;
-  const Row8 w[1] = {load_row8(weight + 8 * lane16)};
-  const long long stride = static_cast<long long>(gridDim.x) * (16 * kRows);
-  // every lane of a warp runs the same number of rounds (the shuffles need all of them).  The piece of the next
-  // round is loaded before this round's shuffles, which the compiler would not move a load across: two rows of a
-  // thread are in flight instead of one.  (In place: the next round's rows are other rows than this round's.)
-  auto piece_at = [&](long long base) {
-    const long long row = base + (threadIdx.x >> 4);
-    return *reinterpret_cast<const uint4*>(src + (row < rows ? row : 0) * 128 + 8 * lane16);
-  };
-  const long long first_base = static_cast<long long>(blockIdx.x) * 16;
-  uint4 next_piece = first_base < rows ? piece_at(first_base) : make_uint4(0u, 0u, 0u, 0u);
-  for (long long base = first_base; base < rows; base += stride) {
-    Row8 x[kRows];
-    int token[kRows];
-    long long at[kRows];
-    bool live[kRows];
-    const uint4 piece = next_piece;
-    if (base + stride < rows) next_piece = piece_at(base + stride);
-#pragma unroll
-    for (int k = 0; k < kRows; ++k) {
-      const long long row = base + 16 * k + (threadIdx.x >> 4);
-      live[k] = row < rows;
-      at[k] = (live[k] ? row : 0) * 128 + 8 * lane16;
-      token[k] = static_cast<int>((live[k] ? row : 0) / heads);
-      x[k] = row8_of(piece);
-    }
-    norm_rope_rows<kRows>(x, w, cosines, sines, token, lane16, use_rope != 0);
-#pragma unroll
-    for (int k = 0; k < kRows; ++k) {
-      if (live[k]) {
-        uint4 out;
-        out.x = pack_bf16_pair(x[k].v[0], x[k].v[1]);
-        out.y = pack_bf16_pair(x[k].v[2], x[k].v[3]);
-        out.z = pack_bf16_pair(x[k].v[4], x[k].v[5]);
-        out.w = pack_bf16_pair(x[k].v[6], x[k].v[7]);
-        *reinterpret_cast<uint4*>(dst + at[k]) = out;
-      }
-    }
-  }
+__device__ __forceinline__ uint4 pack_row8(const Row8& x) {
+  return make_uint4(pack_bf16_pair(x.v[0], x.v[1]), pack_bf16_pair(x.v[2], x.v[3]), pack_bf16_pair(x.v[4], x.v[5]),
+                    pack_bf16_pair(x.v[6], x.v[7]));
 }
 
-// Q and K of the same (token, head) in one launch, in place: a 16-lane group takes the query row and the key row
-// together, so their loads are in flight at once and both use one read of the RoPE table entries.
+// 8 lanes per (token, head) row: 32 rows per CTA round.  TENSORS rows (of Q, or of Q and K, which share the rotary
+// planes' entries) go through together.  In place is allowed.
+struct NormRopeTensors {
+  const __nv_bfloat16* src[2];
+  const __nv_bfloat16* weight[2];
+  __nv_bfloat16* dst[2];  // may be src
+};
+
+template <int TENSORS>
 __global__ void __launch_bounds__(256)
-qk_norm_rope_kernel(__nv_bfloat16* query, __nv_bfloat16* key, const __nv_bfloat16* __restrict__ query_weight,
-                    const __nv_bfloat16* __restrict__ key_weight, const float* __restrict__ cosines,
-                    const float* __restrict__ sines, long long rows, int heads) {
-  const int lane16 = threadIdx.x & 15;
-  const Row8 w[2] = {load_row8(query_weight + 8 * lane16), load_row8(key_weight + 8 * lane16)};
-  const long long stride = static_cast<long long>(gridDim.x) * 16;
-  // every lane of a warp runs the same number of rounds (the shuffles need all of them)
-  // the pieces of the next round are loaded before this round's shuffles (see head_norm_rope_kernel)
-  auto offset_at = [&](long long base) {
-    const long long row = base + (threadIdx.x >> 4);
-    return (row < rows ? row : 0) * 128 + 8 * lane16;
-  };
-  const long long first_base = static_cast<long long>(blockIdx.x) * 16;
-  uint4 next_q = make_uint4(0u, 0u, 0u, 0u), next_k = next_q;
-  if (first_base < rows) {
-    next_q = *reinterpret_cast<const uint4*>(query + offset_at(first_base));
-    next_k = *reinterpret_cast<const uint4*>(key + offset_at(first_base));
-  }
-  for (long long base = first_base; base < rows; base += stride) {
-    const long long row = base + (threadIdx.x >> 4);
-    const bool live = row < rows;
-    const long long at = (live ? row : 0) * 128 + 8 * lane16;
-    Row8 x[2] = {row8_of(next_q), row8_of(next_k)};
-    if (base + stride < rows) {
-      next_q = *reinterpret_cast<const uint4*>(query + offset_at(base + stride));
-      next_k = *reinterpret_cast<const uint4*>(key + offset_at(base + stride));
+norm_rope_kernel(const NormRopeTensors tensors, const float* __restrict__ cosines, const float* __restrict__ sines,
+                 long long rows, int heads, int use_rope) {
+  const int lane8 = threadIdx.x & 7;
+  const int at_a = 8 * chunk_a(lane8), at_b = 8 * chunk_b(lane8);
+  RowPart w[TENSORS];
+#pragma unroll
+  for (int k = 0; k < TENSORS; ++k) w[k] = load_part(tensors.weight[k], lane8);
+  const long long stride = static_cast<long long>(gridDim.x) * 32;
+  // every lane of a warp runs the same number of rounds (the shuffles need all of them).  The pieces of the next
+  // round are loaded before this round's shuffles, which the compiler would not move a load across: two rows of a
+  // thread are in flight instead of one.  (In place: the next round's rows are other rows than this round's.)
+  uint4 next[TENSORS][2];
+  auto fetch = [&](long long base) {
+    const long long row = base + (threadIdx.x >> 3);
+#pragma unroll
+    for (int k = 0; k < TENSORS; ++k) {
+      const __nv_bfloat16* p = tensors.src[k] + (row < rows ? row : 0) * 128;
+      next[k][0] = *reinterpret_cast<const uint4*>(p + at_a);
+      next[k][1] = *reinterpret_cast<const uint4*>(p + at_b);
     }
+  };
+  const long long first_base = static_cast<long long>(blockIdx.x) * 32;
+  if (first_base < rows) fetch(first_base);
+  for (long long base = first_base; base < rows; base += stride) {
+    const long long row = base + (threadIdx.x >> 3);
+    const bool live = row < rows;
     const int tok = static_cast<int>((live ? row : 0) / heads);
-    const int token[2] = {tok, tok};
-    norm_rope_rows<2, 2>(x, w, cosines, sines, token, lane16, true);
+    RowPart x[TENSORS];
+    int token[TENSORS];
+#pragma unroll
+    for (int k = 0; k < TENSORS; ++k) {
+      x[k] = {row8_of(next[k][0]), row8_of(next[k][1])};
+      token[k] = tok;
+    }
+    if (base + stride < rows) fetch(base + stride);
+    norm_rope_rows<TENSORS, TENSORS>(x, w, cosines, sines, token, lane8, use_rope != 0);
     if (live) {
 #pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        uint4 out;
-        out.x = pack_bf16_pair(x[k].v[0], x[k].v[1]);
-        out.y = pack_bf16_pair(x[k].v[2], x[k].v[3]);
-        out.z = pack_bf16_pair(x[k].v[4], x[k].v[5]);
-        out.w = pack_bf16_pair(x[k].v[6], x[k].v[7]);
-        *reinterpret_cast<uint4*>((k ? key : query) + at) = out;
+      for (int k = 0; k < TENSORS; ++k) {
+        __nv_bfloat16* p = tensors.dst[k] + row * 128;
+        *reinterpret_cast<uint4*>(p + at_a) = pack_row8(x[k].a);
+        *reinterpret_cast<uint4*>(p + at_b) = pack_row8(x[k].b);
       }
     }
   }
 }
 
-// One CTA per (32-token group, head): 128 threads, 8 rows per pass, 4 passes.
+// One CTA per (32-token group, head): 128 threads, 16 rows per pass, 2 passes.
 __global__ void __launch_bounds__(128)
 query_prepare_kernel(const __nv_bfloat16* __restrict__ src, const __nv_bfloat16* __restrict__ weight,
                      const float* __restrict__ cosines, const float* __restrict__ sines,
                      int8_t* __restrict__ quantized, float* __restrict__ scales, int tokens, int heads, int groups,
                      int use_rope) {
   const int head = blockIdx.x, group = blockIdx.y;  // heads fastest: CTAs in flight read whole rows of the source
-  const int lane16 = threadIdx.x & 15, row_in_pass = threadIdx.x >> 4;
-  const Row8 w[1] = {load_row8(weight + 8 * lane16)};
+  const int lane8 = threadIdx.x & 7, row_in_pass = threadIdx.x >> 3;
+  const int at_a = 8 * chunk_a(lane8), at_b = 8 * chunk_b(lane8);
+  const RowPart w[1] = {load_part(weight, lane8)};
   const size_t columns = static_cast<size_t>(heads) * 128;
-  Row8 x[4];
-  float amax = 0.f;
-  uint4 loaded[4];  // the four rows' loads are in flight together; the shuffles below would keep them apart
+  uint4 loaded[2][2];  // both rows' loads are in flight together; the shuffles below would keep them apart
 #pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    const int t = group * 32 + p * 8 + row_in_pass;
-    loaded[p] = __ldg(reinterpret_cast<const uint4*>(src + static_cast<size_t>(t < tokens ? t : 0) * columns + head * 128 +
-                                                     8 * lane16));
+  for (int p = 0; p < 2; ++p) {
+    const int t = group * 32 + p * 16 + row_in_pass;
+    const __nv_bfloat16* row = src + static_cast<size_t>(t < tokens ? t : 0) * columns + head * 128;
+    loaded[p][0] = __ldg(reinterpret_cast<const uint4*>(row + at_a));
+    loaded[p][1] = __ldg(reinterpret_cast<const uint4*>(row + at_b));
   }
-  // kTogether rows go through the norm and the rotation together.  One at a time is fastest (175 us at 32768 tokens x
-  // 24 heads; two 211, four 246: the registers of the extra rows cost more occupancy than the overlap gains).
-  constexpr int kTogether = 1;
+  RowPart x[2];
+  float amax = 0.f;
 #pragma unroll
-  for (int p0 = 0; p0 < 4; p0 += kTogether) {
-    int token[kTogether];
-    bool live[kTogether];
-    Row8 rows_now[kTogether];
+  for (int p = 0; p < 2; ++p) {
+    const int t = group * 32 + p * 16 + row_in_pass;
+    const bool live = t < tokens;
+    const int token[1] = {live ? t : 0};
+    RowPart now[1] = {{row8_of(loaded[p][0]), row8_of(loaded[p][1])}};
+    norm_rope_rows<1>(now, w, cosines, sines, token, lane8, use_rope != 0);
+    x[p] = now[0];
 #pragma unroll
-    for (int k = 0; k < kTogether; ++k) {
-      const int t = group * 32 + (p0 + k) * 8 + row_in_pass;
-      live[k] = t < tokens;
-      token[k] = live[k] ? t : 0;
-      rows_now[k] = row8_of(loaded[p0 + k]);
-    }
-    norm_rope_rows<kTogether>(rows_now, w, cosines, sines, token, lane16, use_rope != 0);
-#pragma unroll
-    for (int k = 0; k < kTogether; ++k) {
-      x[p0 + k] = rows_now[k];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        if (!live[k]) x[p0 + k].v[i] = 0.f;  // rows past the end quantise to zero and do not count in the maximum
-        amax = fmaxf(amax, fabsf(x[p0 + k].v[i]));
-      }
+    for (int i = 0; i < 8; ++i) {
+      if (!live) x[p].a.v[i] = x[p].b.v[i] = 0.f;  // rows past the end quantise to zero and do not count in the maximum
+      amax = fmaxf(amax, fmaxf(fabsf(x[p].a.v[i]), fabsf(x[p].b.v[i])));
     }
   }
   __shared__ float warp_max[4];
@@ -268,20 +249,24 @@ query_prepare_kernel(const __nv_bfloat16* __restrict__ src, const __nv_bfloat16*
   if (threadIdx.x == 0) scales[static_cast<size_t>(head) * groups + group] = scale;
   int8_t* dst_base = quantized + (static_cast<size_t>(head) * groups + group) * 32 * 128;
 #pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    const int r = p * 8 + row_in_pass;
-    uint32_t word[2] = {0, 0};
+  for (int p = 0; p < 2; ++p) {
+    int8_t* dst = dst_base + (p * 16 + row_in_pass) * 128;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      // rint(RN(x / scale)): the product with RN(1/scale) rounds to the same integer unless it lies within 4e-5
-      // of a half-integer; only then the IEEE division is done (as in the int8 Q/K quantiser).
-      float a = x[p].v[i] * inv_scale;
-      float q = rintf(a);
-      if (0.5f - fabsf(a - q) < 4e-5f) q = rintf(__fdiv_rn(x[p].v[i], scale));
-      q = fminf(fmaxf(q, -128.f), 127.f);
-      word[i >> 2] |= (static_cast<uint32_t>(static_cast<int>(q)) & 0xffu) << (8 * (i & 3));
+    for (int side = 0; side < 2; ++side) {
+      uint32_t word[2] = {0, 0};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        // rint(RN(x / scale)): the product with RN(1/scale) rounds to the same integer unless it lies within 4e-5
+        // of a half-integer; only then the IEEE division is done (as in the int8 Q/K quantiser).
+        const float value = side ? x[p].b.v[i] : x[p].a.v[i];
+        float a = value * inv_scale;
+        float q = rintf(a);
+        if (0.5f - fabsf(a - q) < 4e-5f) q = rintf(__fdiv_rn(value, scale));
+        q = fminf(fmaxf(q, -128.f), 127.f);
+        word[i >> 2] |= (static_cast<uint32_t>(static_cast<int>(q)) & 0xffu) << (8 * (i & 3));
+      }
+      *reinterpret_cast<uint2*>(dst + (side ? at_b : at_a)) = make_uint2(word[0], word[1]);
     }
-    *reinterpret_cast<uint2*>(dst_base + r * 128 + lane16 * 8) = make_uint2(word[0], word[1]);
   }
 }
 
@@ -295,12 +280,13 @@ extern "C" int nob200_h3_head_norm_rope(int tokens, const void* input, const voi
   NOB_REQUIRE(input && weight && output, "h3_head_norm_rope: NULL tensor");
   NOB_REQUIRE((cosines == nullptr) == (sines == nullptr), "h3_head_norm_rope: cosines and sines come together");
   const long long rows = static_cast<long long>(tokens) * heads;
-  const long long ctas = (rows + 15) / 16;
-  const unsigned grid = static_cast<unsigned>(ctas < 148 * 16 ? ctas : 148 * 16);
-  head_norm_rope_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(input), static_cast<const __nv_bfloat16*>(weight),
-      static_cast<const float*>(cosines), static_cast<const float*>(sines), static_cast<__nv_bfloat16*>(output), rows,
-      heads, cosines != nullptr);
+  const long long ctas = (rows + 31) / 32;
+  const unsigned grid = static_cast<unsigned>(ctas < 148 * 8 ? ctas : 148 * 8);
+  const NormRopeTensors tensors = {{static_cast<const __nv_bfloat16*>(input)},
+                                   {static_cast<const __nv_bfloat16*>(weight)},
+                                   {static_cast<__nv_bfloat16*>(output)}};
+  norm_rope_kernel<1><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      tensors, static_cast<const float*>(cosines), static_cast<const float*>(sines), rows, heads, cosines != nullptr);
   return check_launch("h3_head_norm_rope");
 }
 
@@ -311,12 +297,13 @@ extern "C" int nob200_h3_qk_norm_rope(int tokens, void* query, void* key, const 
   NOB_REQUIRE(tokens > 0 && heads > 0, "h3_qk_norm_rope: sizes must be positive");
   NOB_REQUIRE(query && key && query_weight && key_weight && cosines && sines, "h3_qk_norm_rope: NULL tensor");
   const long long rows = static_cast<long long>(tokens) * heads;
-  const long long ctas = (rows + 15) / 16;
-  const unsigned grid = static_cast<unsigned>(ctas < 148 * 16 ? ctas : 148 * 16);
-  qk_norm_rope_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<__nv_bfloat16*>(query), static_cast<__nv_bfloat16*>(key),
-      static_cast<const __nv_bfloat16*>(query_weight), static_cast<const __nv_bfloat16*>(key_weight),
-      static_cast<const float*>(cosines), static_cast<const float*>(sines), rows, heads);
+  const long long ctas = (rows + 31) / 32;
+  const unsigned grid = static_cast<unsigned>(ctas < 148 * 8 ? ctas : 148 * 8);
+  auto *q = static_cast<__nv_bfloat16*>(query), *k = static_cast<__nv_bfloat16*>(key);
+  const NormRopeTensors tensors = {
+      {q, k}, {static_cast<const __nv_bfloat16*>(query_weight), static_cast<const __nv_bfloat16*>(key_weight)}, {q, k}};
+  norm_rope_kernel<2><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      tensors, static_cast<const float*>(cosines), static_cast<const float*>(sines), rows, heads, 1);
   return check_launch("h3_qk_norm_rope");
 }
 
@@ -347,84 +334,116 @@ extern "C" int nob200_h3_query_prepare(int tokens, const void* source, const voi
 namespace nob200 {
 namespace {
 
-__device__ __forceinline__ void radix4(float& a, float& b, float& c, float& d) {
-  const float p = __fadd_rn(a, b), q = __fsub_rn(a, b), r = __fadd_rn(c, d), u = __fsub_rn(c, d);
-  a = __fadd_rn(p, u);
-  b = __fsub_rn(p, u);
-  c = __fadd_rn(q, r);
-  d = __fsub_rn(r, q);
+// Two columns at a time, one of each of two groups: the packed operations round their halves one by one.
+struct Pair {
+  uint64_t v;
+};
+__device__ __forceinline__ Pair pair_of(float lo, float hi) {
+  Pair r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void halves(Pair p, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p.v));
+}
+__device__ __forceinline__ Pair operator+(Pair a, Pair b) {
+  Pair r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ Pair operator*(Pair a, Pair b) {
+  Pair r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ Pair operator-(Pair a, Pair b) {  // b * -1 is exact: one rounding, that of the difference
+  Pair r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(b.v), "l"(0xbf800000bf800000ull), "l"(a.v));
+  return r;
 }
 
-// One CTA per row; a group of 256 columns lies on 16 lanes with 16 consecutive columns each.
+__device__ __forceinline__ void radix4(Pair& a, Pair& b, Pair& c, Pair& d) {
+  const Pair p = a + b, q = a - b, r = c + d, u = c - d;
+  a = p + u;
+  b = p - u;
+  c = q + r;
+  d = r - q;
+}
+
+// One CTA per row; a group of 256 columns lies on 16 lanes with 16 consecutive columns each, and a half-warp rotates two
+// groups at once.  The kernel is bound by its instructions, about 30 per column one by one; with the packed rotation,
+// packed rounding and the boundary test below about half (15104 x 7168: 135 us, now 105 us; 50 us of traffic).
 __global__ void __launch_bounds__(128)
 rowwise_int8_kernel(const __nv_bfloat16* __restrict__ src, int8_t* __restrict__ dst, float* __restrict__ scales,
                     int columns, int rotate) {
-  extern __shared__ __nv_bfloat16 rotated[];  // the row after rotation and bf16 rounding
+  extern __shared__ __align__(16) __nv_bfloat16 rotated[];  // the row after rotation and bf16 rounding
   __shared__ float warp_max[4];
-  __shared__ float transpose[8][16 * 17];  // one 256-column group per half-warp
+  __shared__ uint64_t transpose[8][16 * 17];  // two 256-column groups per half-warp
   const size_t row = blockIdx.x;
   const int lane16 = threadIdx.x & 15, half_warp = threadIdx.x >> 4;
   const __nv_bfloat16* in = src + row * columns;
   float amax = 0.f;
-  // both half-warps of a warp run every round (the warp synchronises around the transpose); a half-warp past the
-  // last group works on group 0 again and discards the result
   const int groups = columns / 256;
-  for (int first = 0; first < groups; first += 8) {
-    const bool live = first + half_warp < groups;
-    const int g = live ? first + half_warp : 0;
-    float x[16];
-    const Row8 lo = load_row8(in + g * 256 + 16 * lane16), hi = load_row8(in + g * 256 + 16 * lane16 + 8);
+  if (rotate) {
+    // both half-warps of a warp run every round (the warp synchronises around the transpose); a group past the last
+    // one is group 0 again, its result discarded.  The next round's loads are in flight during this round.
+    uint4 next[2][2];
+    auto fetch = [&](int first) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) x[i] = lo.v[i], x[8 + i] = hi.v[i];
-    if (rotate) {
+      for (int s = 0; s < 2; ++s) {
+        const int g = first + 8 * s + half_warp;
+        const uint4* at = reinterpret_cast<const uint4*>(in + (g < groups ? g : 0) * 256 + 16 * lane16);
+        next[s][0] = at[0];
+        next[s][1] = at[1];
+      }
+    };
+    fetch(0);
+    __nv_bfloat162 top = __floats2bfloat162_rn(0.f, 0.f);
+    for (int first = 0; first < groups; first += 16) {
+      const int ga = first + half_warp, gb = ga + 8;
+      Pair x[16];
+      const Row8 a0 = row8_of(next[0][0]), a1 = row8_of(next[0][1]), b0 = row8_of(next[1][0]), b1 = row8_of(next[1][1]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = pair_of(a0.v[i], b0.v[i]), x[8 + i] = pair_of(a1.v[i], b1.v[i]);
+      if (first + 16 < groups) fetch(first + 16);
 #pragma unroll
       for (int i = 0; i < 16; i += 4) radix4(x[i], x[i + 1], x[i + 2], x[i + 3]);  // digit 0: column stride 1
 #pragma unroll
       for (int i = 0; i < 4; ++i) radix4(x[i], x[i + 4], x[i + 8], x[i + 12]);  // digit 1: column stride 4
       // digits 2 and 3 (column strides 16 and 64) lie across the lanes: transpose through shared memory so that a
-      // lane holds columns lane16 + 16 r, r = 0..15, and they become register digits too (rows padded to 17 words)
-      float* scratch = transpose[half_warp];
+      // lane holds columns lane16 + 16 r, r = 0..15, and they become register digits too (rows padded to 17 pairs)
+      uint64_t* scratch = transpose[half_warp];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) scratch[17 * lane16 + i] = x[i];
+      for (int i = 0; i < 16; ++i) scratch[17 * lane16 + i] = x[i].v;
       __syncwarp();
 #pragma unroll
-      for (int r = 0; r < 16; ++r) x[r] = scratch[17 * r + lane16];
+      for (int r = 0; r < 16; ++r) x[r].v = scratch[17 * r + lane16];
       __syncwarp();
 #pragma unroll
       for (int i = 0; i < 16; i += 4) radix4(x[i], x[i + 1], x[i + 2], x[i + 3]);  // digit 2
 #pragma unroll
       for (int i = 0; i < 4; ++i) radix4(x[i], x[i + 4], x[i + 8], x[i + 12]);  // digit 3
+      const bool live_a = ga < groups, live_b = gb < groups;
 #pragma unroll
-      for (int i = 0; i < 16; ++i) x[i] = round_bf16(__fmul_rn(x[i], 0.0625f));
-      if (live) {
-#pragma unroll
-        for (int r = 0; r < 16; ++r) {
-          amax = fmaxf(amax, fabsf(x[r]));
-          rotated[g * 256 + lane16 + 16 * r] = __float2bfloat16_rn(x[r]);  // exact: already bf16-representable
-        }
+      for (int r = 0; r < 16; ++r) {
+        float a, b;
+        halves(x[r] * pair_of(0.0625f, 0.0625f), a, b);
+        // a discarded group repeats group 0, whose maximum counts anyway
+        const __nv_bfloat162 rounded = __floats2bfloat162_rn(a, b);
+        top = __hmax2(top, __habs2(rounded));
+        if (live_a) rotated[ga * 256 + lane16 + 16 * r] = rounded.x;
+        if (live_b) rotated[gb * 256 + lane16 + 16 * r] = rounded.y;
       }
-    } else if (live) {
-      uint32_t w[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        amax = fmaxf(amax, fmaxf(fabsf(x[2 * i]), fabsf(x[2 * i + 1])));
-        w[i] = pack_bf16_pair(x[2 * i], x[2 * i + 1]);
-      }
-      uint4* out = reinterpret_cast<uint4*>(rotated + g * 256 + 16 * lane16);
-      out[0] = make_uint4(w[0], w[1], w[2], w[3]);
-      out[1] = make_uint4(w[4], w[5], w[6], w[7]);
     }
-  }
-  // columns beyond the last whole group (row-wise form only; a multiple of 8)
-  for (int c = groups * 256 + 8 * threadIdx.x; c < columns; c += 8 * 128) {
-    const Row8 v = load_row8(in + c);
-    uint32_t w[4];
+    amax = fmaxf(__bfloat162float(top.x), __bfloat162float(top.y));
+  } else {
+    for (int c = 8 * threadIdx.x; c < columns; c += 8 * 128) {  // columns is a multiple of 8
+      const uint4 raw = *reinterpret_cast<const uint4*>(in + c);
+      const Row8 v = row8_of(raw);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      amax = fmaxf(amax, fmaxf(fabsf(v.v[2 * i]), fabsf(v.v[2 * i + 1])));
-      w[i] = pack_bf16_pair(v.v[2 * i], v.v[2 * i + 1]);
+      for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v.v[i]));
+      *reinterpret_cast<uint4*>(rotated + c) = raw;
     }
-    *reinterpret_cast<uint4*>(rotated + c) = make_uint4(w[0], w[1], w[2], w[3]);
   }
 #pragma unroll
   for (int m = 16; m > 0; m >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, m));
@@ -435,18 +454,39 @@ rowwise_int8_kernel(const __nv_bfloat16* __restrict__ src, int8_t* __restrict__ 
   const float inv_scale = __frcp_rn(scale);
   if (threadIdx.x == 0) scales[row] = scale;
   int8_t* out = dst + row * columns;
+  const Pair inverse = pair_of(inv_scale, inv_scale), magic = pair_of(12582912.f, 12582912.f);  // 2^23 * 1.5
   for (int c = 8 * threadIdx.x; c < columns; c += 8 * 128) {
     const Row8 v = load_row8(rotated + c);
-    uint32_t word[2] = {0, 0};
+    // rint(RN(x / scale)) as in the other int8 quantisers: the product with RN(1 / scale) rounds to the same integer
+    // unless it lies within 4e-5 of a half-integer (or is not finite); only then the IEEE division is done.  The adder
+    // rounds to nearest even, and the low byte of product + 2^23 * 1.5 is the code (|product| <= 127 and an ulp).
+    uint32_t code[8];
+    bool near = false;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      // rint(RN(x / scale)) as in the other int8 quantisers: exact division only near a rounding boundary
-      float a = v.v[i] * inv_scale;
-      float q = rintf(a);
-      if (!(0.5f - fabsf(a - q) >= 4e-5f)) q = rintf(__fdiv_rn(v.v[i], scale));
-      q = fminf(fmaxf(q, -127.f), 127.f);
-      word[i >> 2] |= (static_cast<uint32_t>(static_cast<int>(q)) & 0xffu) << (8 * (i & 3));
+    for (int i = 0; i < 8; i += 2) {
+      const Pair product = pair_of(v.v[i], v.v[i + 1]) * inverse;
+      const Pair moved = product + magic;
+      float d0, d1, t0, t1;
+      halves(product - (moved - magic), d0, d1);
+      halves(moved, t0, t1);
+      near = near || !(fabsf(d0) <= 0.5f - 4e-5f) || !(fabsf(d1) <= 0.5f - 4e-5f);
+      code[i] = __float_as_uint(t0);
+      code[i + 1] = __float_as_uint(t1);
     }
+    if (near) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        float a = v.v[i] * inv_scale;
+        float q = rintf(a);
+        if (!(0.5f - fabsf(a - q) >= 4e-5f)) q = rintf(__fdiv_rn(v.v[i], scale));
+        code[i] = static_cast<uint32_t>(static_cast<int>(fminf(fmaxf(q, -127.f), 127.f)));
+      }
+    }
+    uint32_t word[2];
+#pragma unroll
+    for (int w = 0; w < 2; ++w)
+      word[w] = __byte_perm(__byte_perm(code[4 * w], code[4 * w + 1], 0x0040),
+                            __byte_perm(code[4 * w + 2], code[4 * w + 3], 0x0040), 0x5410);
     *reinterpret_cast<uint2*>(out + c) = make_uint2(word[0], word[1]);
   }
 }
@@ -465,7 +505,7 @@ extern "C" int nob200_int8_rowwise(int num_tokens, const void* input, void* outp
               "int8_rowwise: columns (%d) must be a multiple of 8, and of the rotation group", columns);
   NOB_REQUIRE(columns <= 65536, "int8_rowwise: at most 65536 columns (the row is staged in shared memory)");
   const size_t smem = static_cast<size_t>(columns) * 2;
-  if (smem + 9 * 1024 > 48 * 1024) {  // the kernel also holds 8.5 KiB of static shared memory (the transpose)
+  if (smem + 18 * 1024 > 48 * 1024) {  // the kernel also holds 17 KiB of static shared memory (the transpose)
     cudaError_t err = cudaFuncSetAttribute(rowwise_int8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess)
       return fail(kCudaError, "int8_rowwise: cannot reserve %zu B of shared memory: %s", smem, cudaGetErrorString(err));
