@@ -107,8 +107,9 @@ hadamard_rows_kernel(const __nv_bfloat16* src, __nv_bfloat16* dst, long long row
 // order starting from the first token; chunk sums are then added sequentially
 // in chunk order; the total is divided (IEEE) by the group's divisor.
 constexpr int kMeanChunk = 128;
+constexpr int kMeanBatch = 32;
 
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 6)  // a register budget that lets a batch of loads be in flight
 mean_chunk_kernel(const __nv_bfloat16* __restrict__ in, float* __restrict__ dst, int num_tokens, int columns,
                   int tokens_per_block, int chunks_per_group, int include_padding, int direct) {
   const int col = (blockIdx.x * 128 + threadIdx.x) * 4;
@@ -121,14 +122,25 @@ mean_chunk_kernel(const __nv_bfloat16* __restrict__ in, float* __restrict__ dst,
   end = min(end, num_tokens);
   float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
   const __nv_bfloat16* p = in + static_cast<size_t>(begin) * columns + col;
-#pragma unroll 8
-  for (int t = begin; t < end; ++t, p += columns) {
-    const uint2 raw = *reinterpret_cast<const uint2*>(p);
+  auto add = [&](const uint2& raw) {
     a0 += __uint_as_float(raw.x << 16);
     a1 += __uint_as_float(raw.x & 0xffff0000u);
     a2 += __uint_as_float(raw.y << 16);
     a3 += __uint_as_float(raw.y & 0xffff0000u);
+  };
+  // The additions of a chunk are one chain, the loads are not: kMeanBatch of them are in flight together.  Eight were
+  // enough for long calls (45 us for 60778 x 1792), but a short call is a few CTAs that wait for memory once per batch
+  // (1021 x 1792: 11.9 us, now 4.9).
+  int t = begin;
+  for (; t + kMeanBatch <= end; t += kMeanBatch, p += static_cast<size_t>(kMeanBatch) * columns) {
+    uint2 raw[kMeanBatch];
+#pragma unroll
+    for (int i = 0; i < kMeanBatch; ++i) raw[i] = *reinterpret_cast<const uint2*>(p + static_cast<size_t>(i) * columns);
+#pragma unroll
+    for (int i = 0; i < kMeanBatch; ++i) add(raw[i]);
   }
+#pragma unroll 8
+  for (; t < end; ++t, p += columns) add(*reinterpret_cast<const uint2*>(p));
   if (direct) {
     const int valid = min(tokens_per_block, num_tokens - group_begin);
     const float div = static_cast<float>(include_padding ? tokens_per_block : valid);
@@ -271,10 +283,23 @@ quantize_qk_kernel(const __nv_bfloat16* __restrict__ src, const float* __restric
 }
 
 // ------------------------------------------------------------- V statistics
-// amax[c] over all tokens, accumulated with atomicMax on the (non-negative) bit
-// pattern, then turned into max(amax / 2.25, 1e-10) in place.
+// amax[c] over all tokens, then max(amax / 2.25, 1e-10).  |bf16| as fp32 bit patterns: integer max == float max for
+// non-negative values.
 constexpr int kVScaleTokens = 256;
 
+__device__ __forceinline__ void amax_of(uint32_t (&m)[8], const uint4& raw) {
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m[2 * i] = max(m[2 * i], (w[i] << 16) & 0x7fffffffu);
+    m[2 * i + 1] = max(m[2 * i + 1], w[i] & 0x7fff0000u);
+  }
+}
+__device__ __forceinline__ float value_scale_of(uint32_t amax_bits) {
+  return fmaxf(__uint_as_float(amax_bits) / 2.25f, 1e-10f);
+}
+
+// Long calls: CTAs of 256 columns x 256 tokens combine through atomicMax; a second kernel turns maxima into scales.
 __global__ void __launch_bounds__(256)
 value_amax_kernel(const __nv_bfloat16* __restrict__ src, uint32_t* __restrict__ amax_bits, int num_tokens,
                   int columns) {
@@ -286,16 +311,8 @@ value_amax_kernel(const __nv_bfloat16* __restrict__ src, uint32_t* __restrict__ 
   uint32_t m[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (col < columns) {
 #pragma unroll 4
-    for (int t = begin + warp; t < end; t += 8) {
-      const uint4 raw = *reinterpret_cast<const uint4*>(src + static_cast<size_t>(t) * columns + col);
-      const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        // |bf16| as fp32 bit patterns; integer max == float max for non-negative values
-        m[2 * i] = max(m[2 * i], (w[i] << 16) & 0x7fffffffu);
-        m[2 * i + 1] = max(m[2 * i + 1], w[i] & 0x7fff0000u);
-      }
-    }
+    for (int t = begin + warp; t < end; t += 8)
+      amax_of(m, *reinterpret_cast<const uint4*>(src + static_cast<size_t>(t) * columns + col));
   }
 #pragma unroll
   for (int i = 0; i < 8; ++i) part[warp][lane][i] = m[i];
@@ -313,7 +330,37 @@ value_amax_kernel(const __nv_bfloat16* __restrict__ src, uint32_t* __restrict__ 
 
 __global__ void value_scale_finish_kernel(float* __restrict__ scales, int columns) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < columns) scales[c] = fmaxf(scales[c] / 2.25f, 1e-10f);
+  if (c < columns) scales[c] = value_scale_of(__float_as_uint(scales[c]));
+}
+
+// Short calls: one CTA owns 64 columns over all tokens and writes their scales, one launch instead of a memset and two
+// kernels.  8 lanes read 128 bytes of a token, 64 tokens at a time, eight loads per thread in flight.  At 1021 tokens x
+// 1792 columns 8.0 us for the three, 3.8 us for this one; a CTA's share grows with the tokens, so calls above
+// kVScaleShort keep the split over tokens.
+constexpr int kVScaleShort = 2048;
+
+__global__ void __launch_bounds__(512, 1)
+value_scale_short_kernel(const __nv_bfloat16* __restrict__ src, float* __restrict__ scales, int num_tokens, int columns) {
+  __shared__ uint32_t part[16][64];
+  const int group = threadIdx.x & 7, row = threadIdx.x >> 3, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const __nv_bfloat16* p = src + blockIdx.x * 64 + group * 8;  // columns is a multiple of 128
+  uint32_t m[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 8
+  for (int t = row; t < num_tokens; t += 64)
+    amax_of(m, *reinterpret_cast<const uint4*>(p + static_cast<size_t>(t) * columns));
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    m[i] = max(m[i], __shfl_xor_sync(0xffffffffu, m[i], 8));
+    m[i] = max(m[i], __shfl_xor_sync(0xffffffffu, m[i], 16));
+    if (lane < 8) part[warp][8 * lane + i] = m[i];
+  }
+  __syncthreads();
+  if (threadIdx.x < 64) {
+    uint32_t v = part[0][threadIdx.x];
+#pragma unroll
+    for (int w = 1; w < 16; ++w) v = max(v, part[w][threadIdx.x]);
+    scales[blockIdx.x * 64 + threadIdx.x] = value_scale_of(v);
+  }
 }
 
 // ------------------------------------------------------------ V -> fp8 e4m3
@@ -669,6 +716,11 @@ extern "C" int nob200_int8_fp8_value_scale(int num_tokens, const void* source, v
   NOB_REQUIRE(source && scales, "int8_fp8_value_scale: NULL tensor");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int columns = heads * 128;
+  if (num_tokens <= kVScaleShort) {
+    value_scale_short_kernel<<<columns / 64, 512, 0, s>>>(static_cast<const __nv_bfloat16*>(source),
+                                                          static_cast<float*>(scales), num_tokens, columns);
+    return check_launch("int8_fp8_value_scale(short)");
+  }
   cudaError_t err = cudaMemsetAsync(scales, 0, static_cast<size_t>(columns) * sizeof(float), s);
   if (err != cudaSuccess) return fail(kCudaError, "int8_fp8_value_scale: %s", cudaGetErrorString(err));
   const int token_blocks = (num_tokens + kVScaleTokens - 1) / kVScaleTokens;
