@@ -18,9 +18,12 @@
 //                blocks (src/nano_omni/kernels/attention/nvfp4/sol_finalize.py:212-270); the output may alias
 //                the numerator, every thread reads its own row before it writes it.
 //
-// CTA organisation.  One CTA owns 128 query rows of one head.  The TMA producer first builds the list of
-// 128-key tiles that one of the CTA's query blocks selects, with one flag per (query block, 64-key half), followed
-// by the tiles of pooled pseudo-keys.  The entries of that list are dealt alternately to two STREAMS: stream 0
+// CTA organisation.  One CTA owns 128 query rows of one head.  The TMA producer first builds the list of 64-key blocks
+// that one of the CTA's query blocks selects, with one flag per query block (128-token blocks are two such blocks).
+// Two listed blocks, wherever they lie, make one ENTRY: a tile of 128 keys for the MMAs, fetched as 64-row boxes.  (A
+// tile of 128 consecutive keys for every one with a selected half had 50 % of all tiles on the list where a query block
+// selects 16 % of the 64-key blocks; the list of pairs has 30 %: 7310 tokens x 14 heads 223 us, now 171.)  Tiles
+// of pooled pseudo-keys follow.  The entries are dealt alternately to two STREAMS: stream 0
 // takes entries 0, 2, 4, ..., stream 1 entries 1, 3, 5, ...  Each stream is a complete online softmax over its
 // share of the keys with its own score buffer, accumulator (TMEM) and (maximum, sum), run by one softmax
 // warpgroup; the tcgen05 issuer ping-pongs between them as the dense kernel does between its two query tiles, so
@@ -52,12 +55,12 @@ constexpr int kMmaWarp = 9;
 constexpr uint32_t kTmemCols = 512;
 constexpr float kRescaleThreshold = 8.0f;
 constexpr int kMaxTiles = 2048;  // key tiles of 128 tokens: up to 262144 tokens
+constexpr int kItem = 64;        // keys of a list item
 
 struct __align__(1024) Shared {
   uint8_t q[kTileBytes];
   uint8_t kv[kStages][kTileBytes];
-  uint16_t tile_list[kMaxTiles];
-  uint8_t tile_flags[kMaxTiles];  // bit 2*(query block inside the tile) + half: selected
+  uint16_t items[2 * kMaxTiles];  // 4 x (64-key block) + one bit per query block of the tile that selected it
   float4 merge[2][kTile];         // per stream and row: (maximum used, sum, raw maximum, stream has a result)
   uint64_t q_full;
   uint64_t kv_full[kStages];
@@ -67,7 +70,7 @@ struct __align__(1024) Shared {
   uint64_t o_final[2];
   uint64_t list_ready;
   uint64_t merge_ready;
-  int num_exact;
+  int num_items;
   uint32_t tmem_base;
   uint32_t abort;
 };
@@ -105,7 +108,7 @@ fa_fwd_sol_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   const int head = blockIdx.y;
   const int q0 = blockIdx.x * kTile;
   const int num_tokens = P.num_tokens;
-  const int n_kv = (num_tokens + kTile - 1) / kTile;             // key tiles of the exact phase
+  const int n_blocks = (num_tokens + kItem - 1) / kItem;  // 64-key blocks of the exact phase
   const int n_pool = MODE == kExactState ? 0 : (P.num_blocks + kTile - 1) / kTile;  // tiles of pooled pseudo-keys
   volatile uint32_t* abort_flag = &S.abort;
   uint32_t* status = P.status;
@@ -143,15 +146,16 @@ fa_fwd_sol_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   if (warp >= 8) {
     reg_dealloc<56>();
     if (warp == kProducerWarp) {
-      // ---------------------------------------------- tile list, then TMA producer
+      // ---------------------------------------------- item list, then TMA producer
       const int qb_first = q0 / P.block;
       const int qb_per_tile = kTile / P.block;  // 2 or 1
-      // Every lane looks at 8 consecutive key tiles per round, all their mask bytes in flight at once; a warp scan
-      // keeps the list in ascending tile order.
+      const int kb_shift = P.block == 64 ? 0 : 1;
+      // Every lane looks at 8 consecutive 64-key blocks per round, all their mask bytes in flight at once; a warp scan
+      // keeps the list in ascending order.
       int count = 0;
       constexpr int kPerLane = 8;
-      for (int base = 0; MODE != kFinalize && base < n_kv; base += 32 * kPerLane) {
-        const int kt0 = base + kPerLane * lane;
+      for (int base = 0; MODE != kFinalize && base < n_blocks; base += 32 * kPerLane) {
+        const int first = base + kPerLane * lane;
         uint32_t flags[kPerLane];
 #pragma unroll
         for (int i = 0; i < kPerLane; ++i) flags[i] = 0;
@@ -161,12 +165,8 @@ fa_fwd_sol_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           const uint8_t* row = P.mask + qb * mask_row_stride + static_cast<size_t>(head) * P.num_blocks;
 #pragma unroll
           for (int i = 0; i < kPerLane; ++i) {
-#pragma unroll
-            for (int h2 = 0; h2 < 2; ++h2) {
-              const int kb = (P.block == 64) ? 2 * (kt0 + i) + h2 : kt0 + i;
-              if (kt0 + i < n_kv && kb < P.num_blocks && (row[kb] || (P.force_first_block && kb == 0)))
-                flags[i] |= 1u << (2 * u + h2);
-            }
+            const int kb = (first + i) >> kb_shift;
+            if (first + i < n_blocks && (row[kb] || (P.force_first_block && kb == 0))) flags[i] |= 1u << u;
           }
         }
         int mine = 0;
@@ -183,10 +183,8 @@ fa_fwd_sol_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 #pragma unroll
         for (int i = 0; i < kPerLane; ++i) {
           if (flags[i]) {
-            if (NOB_CHECK(at >= 0 && at < kMaxTiles, status)) {
-              S.tile_list[at] = static_cast<uint16_t>(kt0 + i);
-              S.tile_flags[at] = static_cast<uint8_t>(flags[i]);
-            }
+            if (NOB_CHECK(at >= 0 && at < 2 * kMaxTiles, status))
+              S.items[at] = static_cast<uint16_t>(4 * (first + i) + flags[i]);
             ++at;
           }
         }
@@ -194,7 +192,7 @@ fa_fwd_sol_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       }
       __syncwarp();
       if (lane == 0) {
-        S.num_exact = count;
+        S.num_items = count;
         mbar_arrive(&S.list_ready);  // release: the list and its length are visible to the waiters
 
         tma_prefetch_desc(&map_q);
@@ -204,23 +202,28 @@ fa_fwd_sol_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         mbar_expect_tx(&S.q_full, kTileBytes);
         tma_load_3d(S.q, &map_q, &S.q_full, 0, head, q0);
         tma_load_3d(S.q + kHalfBytes, &map_q, &S.q_full, 64, head, q0);
-        const int n_it = count + n_pool;
+        const int num_exact = (count + 1) / 2;
+        const int n_it = num_exact + n_pool;
         int issued = 0;
-        // load number `issued` of the consumption order: K-like (is_v = 0) or V-like tile of entry j
+        // load number `issued` of the order: K-like (is_v = 0) or V-like tile of entry j
         auto load = [&](int j, int is_v) -> bool {
           const int st = issued % kStages;
           if (issued >= kStages) {
             if (!mbar_wait(&S.kv_empty[st], ((issued / kStages) - 1) & 1, abort_flag, status, kWaitTimeoutRing)) return false;
           }
           mbar_expect_tx(&S.kv_full[st], kTileBytes);
-          if (j < count) {
+          if (j < num_exact) {
             const CUtensorMap* map = is_v ? &map_v : &map_k;
-            const int tok = S.tile_list[j] * kTile;
-            tma_load_3d(S.kv[st], map, &S.kv_full[st], 0, head, tok);
-            tma_load_3d(S.kv[st] + kHalfBytes, map, &S.kv_full[st], 64, head, tok);
+            // an odd list ends with a block twice; nobody selects the second
+            const int tok0 = (S.items[2 * j] >> 2) * kItem;
+            const int tok1 = 2 * j + 1 < count ? (S.items[2 * j + 1] >> 2) * kItem : tok0;
+            tma_load_3d(S.kv[st], map, &S.kv_full[st], 0, head, tok0);
+            tma_load_3d(S.kv[st] + kHalfBytes, map, &S.kv_full[st], 64, head, tok0);
+            tma_load_3d(S.kv[st] + kHalfBytes / 2, map, &S.kv_full[st], 0, head, tok1);
+            tma_load_3d(S.kv[st] + kHalfBytes + kHalfBytes / 2, map, &S.kv_full[st], 64, head, tok1);
           } else {
             const int plane = is_v ? P.pooled_v_plane : P.pooled_k_plane;
-            const int row = (j - count) * kTile;
+            const int row = (j - num_exact) * kTile;
             tma_load_3d(S.kv[st], &map_pooled, &S.kv_full[st], 0, row, plane * P.heads + head);
             tma_load_3d(S.kv[st] + kHalfBytes, &map_pooled, &S.kv_full[st], 64, row, plane * P.heads + head);
           }
@@ -301,7 +304,7 @@ fa_fwd_sol_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         };
 
         bool ok = warp_rest(&S.list_ready, 0, abort_flag, status, kWaitTimeoutLoad);
-        const int n_it = ok ? S.num_exact + n_pool : 0;
+        const int n_it = ok ? (S.num_items + 1) / 2 + n_pool : 0;
         ok = ok && warp_rest(&S.q_full, 0, abort_flag, status, kWaitTimeoutLoad);
         int taken = 0;  // loads consumed so far, in the order the producer issues them
         // waits for the next load of the order and returns its stage (-1: gave up)
@@ -369,7 +372,8 @@ fa_fwd_sol_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       uint64_t la = 0ull, lb = 0ull;
       int done = 0;  // entries this stream has processed: phase of its S/P barriers
       bool ok = __all_sync(0xffffffffu, mbar_wait(&S.list_ready, 0, abort_flag, status, kWaitTimeoutLoad));
-      const int num_exact = ok ? S.num_exact : 0;
+      const int num_items = ok ? S.num_items : 0;
+      const int num_exact = (num_items + 1) / 2;
       const int n_it = ok ? num_exact + n_pool : 0;
       if (MODE == kFinalize && t == 0) {
         // stream 0 starts from the exact stage's numerator (accumulator) and its (maximum, sum)
@@ -524,11 +528,11 @@ fa_fwd_sol_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       for (int j = t; ok && j < n_it; j += 2) {
         uint32_t valid[4];
         if (j < num_exact) {
-          const uint32_t mine = (S.tile_flags[j] >> (2 * u)) & 3u;
-          const int limit = num_tokens - S.tile_list[j] * kTile;  // keys of the tile that exist
 #pragma unroll
           for (int h2 = 0; h2 < 2; ++h2) {
-            const int n_valid = ((mine >> h2) & 1u) ? max(0, min(64, limit - 64 * h2)) : 0;
+            const uint32_t item = 2 * j + h2 < num_items ? S.items[2 * j + h2] : 0u;
+            const int limit = num_tokens - static_cast<int>(item >> 2) * kItem;  // keys of the block that exist
+            const int n_valid = ((item >> u) & 1u) ? min(kItem, limit) : 0;
             valid[2 * h2] = n_valid >= 32 ? 0xffffffffu : ((1u << n_valid) - 1u);
             valid[2 * h2 + 1] = n_valid >= 64 ? 0xffffffffu : (n_valid > 32 ? ((1u << (n_valid - 32)) - 1u) : 0u);
           }
@@ -667,10 +671,10 @@ int launch_sol(int num_tokens, int head_offset, const void* query, const void* k
                                token_stride, 64, 1, kTile)))
     return rc;
   if ((rc = make_tensor_map_3d(&mk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, key, 128, heads, num_tokens, head_stride,
-                               token_stride, 64, 1, kTile)))
+                               token_stride, 64, 1, kItem)))
     return rc;
   if ((rc = make_tensor_map_3d(&mv, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, value, 128, heads, num_tokens, head_stride,
-                               token_stride, 64, 1, kTile)))
+                               token_stride, 64, 1, kItem)))
     return rc;
   // pooled [planes, heads, blocks, 128]: rows = blocks, outer = plane * heads + head
   if (mode == kExactState) {
