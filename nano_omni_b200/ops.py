@@ -230,8 +230,10 @@ class Op(abc.ABC):
 
     def bind(self, scratch_base: int) -> tuple[Kernel, ...]:
         """``prepare()`` with every scratch descriptor resolved to ``scratch_base + offset``."""
-        calls, _ = self.prepare()
+        return self._resolved(self.prepare()[0], scratch_base)
 
+    @staticmethod
+    def _resolved(calls: tuple[Kernel, ...], scratch_base: int) -> tuple[Kernel, ...]:
         def resolve(tensor: TensorDesc) -> TensorDesc:
             if tensor.kind != TensorKind.SCRATCH:
                 return tensor
@@ -258,9 +260,9 @@ class Op(abc.ABC):
                 raise RuntimeError(f"{function.__name__}: {_lib.last_error()} (status {code})")
 
     def _plan_for(self, base: int) -> _Plan:
-        _, need = self.prepare()
+        calls, need = self.prepare()
         assert base % 256 == 0, "scratch must be 256-byte aligned"
-        plan = _Plan(need, tuple(call for kernel in self.bind(base) for call in kernel.recorded()))
+        plan = _Plan(need, tuple(call for kernel in self._resolved(calls, base) for call in kernel.recorded()))
         plans = dict(self._plans)
         while len(plans) >= _KEPT_PLANS:
             del plans[next(iter(plans))]
