@@ -371,7 +371,7 @@ class DenseBf16Attention(_SliceAttention):
     def kernels(self, scratch: ScratchLayout) -> list[Kernel]:
         sequence = KernelSequence(scratch)
         query, key, value = (t.view(self.head_shape) for t in self.prepared_inputs(sequence))
-        if self.units.tail_units:
+        if self.units.tail_units or self.units.query_rows != 256:  # fp32 shares, as the launch by units takes them
             need = key_share_workspace_bytes(self.rows, self.heads, self.units)
         else:
             need = splitkv_workspace_bytes(self.rows, self.heads, self.kv_splits)
