@@ -39,8 +39,11 @@ uint32_t* status_word_device_ptr();  // address of the file-scope status word
 
 #ifdef __CUDACC__
 namespace nob200 {
-// Launches a kernel whose first statement is pdl_wait(): its CTAs may be brought onto the SMs while the kernel before it
-// in the stream drains (programmatic dependent launch), which takes the launch latency (2-3 us) off the path.
+// Launches a kernel that calls pdl_wait() in every thread before it touches global memory: its CTAs may be brought onto
+// the SMs while the kernel before it in the stream drains (programmatic dependent launch), which takes the launch
+// latency (2-3 us) and the kernel's on-chip set-up off the path.
+// An operator is a chain of such launches: 1021 tokens x 14 heads int8-fp8, eight kernels, 64.4 -> 49.8 us; a bf16
+// product of 512 x 7168 x 5376 43.5 -> 42.1 us; calls of milliseconds unchanged.
 template <typename... Params, typename... Args>
 int launch_pdl(const char* what, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, void* stream, Args&&... args) {
   cudaLaunchAttribute attribute = {};
@@ -88,9 +91,11 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
   return t;
 }
 
-// ---- programmatic dependent launch.  A kernel launched by launch_pdl() starts with pdl_wait(), in every thread: it
-// returns when the kernels before it in the stream have completed and their writes are visible.  pdl_release() lets the
-// next kernel of the stream be scheduled from the moment every CTA has called it (or exited); it orders no memory.
+// ---- programmatic dependent launch.  A kernel launched by launch_pdl() calls pdl_wait(), in every thread, before its
+// first access to global memory (on-chip set-up may come first): it returns when the kernels before it in the stream
+// have completed and their writes are visible.  pdl_release() lets the next kernel of the stream be scheduled from the
+// moment every CTA has called it (or exited); it orders no memory.  The pointers such a kernel reads through carry no
+// __restrict__: a load that the compiler may take for constant could be moved above the wait.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -140,6 +140,7 @@ fa_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = S.tmem_base;
+  pdl_wait();     // launched as a programmatic dependent: the set-up above overlaps the kernel before
   pdl_release();  // the merge of the shares may be scheduled behind the last CTAs
 
   if (warp >= 8) {
@@ -555,9 +556,9 @@ int launch_dense_bf16(int num_tokens, int head_offset, const void* query, const 
   if (err != cudaSuccess)
     return fail(kCudaError, "%s: cannot reserve %zu B of shared memory: %s", name, smem, cudaGetErrorString(err));
   const float scale_log2 = 0.08838834764831845f * 1.4426950408889634f;
-  kernel<<<key_split_blocks(split, heads), kThreads, smem, static_cast<cudaStream_t>(stream)>>>(
-      mq, mk, mv, route, num_tokens, total_heads, head_offset, scale_log2, status, split);
-  if ((rc = check_launch(name))) return rc;
+  if ((rc = launch_pdl(name, kernel, key_split_blocks(split, heads), kThreads, smem, stream, mq, mk, mv, route, num_tokens,
+                       total_heads, head_offset, scale_log2, status, split)))
+    return rc;
   return split.tail_rows ? launch_merge_splits(split, route, num_tokens, total_heads, head_offset, stream) : kOk;
 }
 

@@ -78,8 +78,8 @@ __device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float
 }
 __global__ void __launch_bounds__(kThreads, 1)
 fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                   const __grid_constant__ CUtensorMap map_v, const float* __restrict__ query_scale,
-                   const float* __restrict__ key_scale, const float* __restrict__ value_scale,
+                   const __grid_constant__ CUtensorMap map_v, const float* query_scale,
+                   const float* key_scale, const float* value_scale,
                    __nv_bfloat16* __restrict__ out, int num_query_tokens, int num_kv_tokens, int heads,
                    float scale_log2, uint32_t* status, int query_block, int key_block, const KeySplit split) {
   extern __shared__ uint8_t smem_raw[];
@@ -129,6 +129,7 @@ fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = S.tmem_base;
+  pdl_wait();     // launched as a programmatic dependent: the set-up above overlaps the kernel before
   pdl_release();  // the merge of the shares may be scheduled behind the last CTAs
 
   if (warp >= 8) {
@@ -446,11 +447,11 @@ int launch_dense_int8_fp8(int num_kv_tokens, int num_query_tokens, const void* q
     return fail(kCudaError, "dense_int8_fp8_d128: cannot reserve %zu B of shared memory: %s", smem,
                 cudaGetErrorString(err));
   const float scale_log2 = 0.08838834764831845f * 1.4426950408889634f;
-  fa_fwd_i8f8_kernel<<<key_split_blocks(split, heads), kThreads, smem, static_cast<cudaStream_t>(stream)>>>(
-      mq, mk, mv, static_cast<const float*>(query_scale), static_cast<const float*>(key_scale),
-      static_cast<const float*>(value_scale), static_cast<__nv_bfloat16*>(output), num_query_tokens, num_kv_tokens,
-      heads, scale_log2, status, query_block, key_block, split);
-  if ((rc = check_launch("dense_int8_fp8_d128"))) return rc;
+  if ((rc = launch_pdl("dense_int8_fp8_d128", fa_fwd_i8f8_kernel, key_split_blocks(split, heads), kThreads, smem, stream, mq,
+                       mk, mv, static_cast<const float*>(query_scale), static_cast<const float*>(key_scale),
+                       static_cast<const float*>(value_scale), static_cast<__nv_bfloat16*>(output), num_query_tokens,
+                       num_kv_tokens, heads, scale_log2, status, query_block, key_block, split)))
+    return rc;
   if (!split.tail_rows) return kOk;
   OutRoute route = {};
   route.peer[0] = static_cast<__nv_bfloat16*>(output);

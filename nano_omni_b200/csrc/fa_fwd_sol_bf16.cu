@@ -139,6 +139,8 @@ fa_fwd_sol_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = S.tmem_base;
+  pdl_wait();  // launched as a programmatic dependent: the set-up above overlaps the kernel before
+  pdl_release();
 
   // Order in which the issuer consumes K and V tiles of the entry sequence: K(0), K(1), then for every entry j
   // V(j) followed by K(j+2).  Producer and issuer both walk it with a running counter that names ring stage and
@@ -716,8 +718,7 @@ int launch_sol(int num_tokens, int head_offset, const void* query, const void* k
     return fail(kCudaError, "sol_attention_d128: cannot reserve %zu B of shared memory: %s", smem,
                 cudaGetErrorString(err));
   dim3 grid((num_tokens + kTile - 1) / kTile, heads);
-  kernel<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(mq, mk, mv, mp, params);
-  return check_launch("sol_attention_d128");
+  return launch_pdl("sol_attention_d128", kernel, grid, kThreads, smem, stream, mq, mk, mv, mp, params);
 }
 }  // namespace
 }  // namespace nob200

@@ -190,6 +190,10 @@ matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
   pair_sync();  // the peer's barriers exist before anything reports to them
   tc_fence_after();
   const uint32_t tmem = S.tmem_base;
+  // Launched as a programmatic dependent: everything above happens while the kernel before it drains.  All CTAs are
+  // resident at once, so the next kernel may be brought up from here on.
+  pdl_wait();
+  pdl_release();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -483,8 +487,7 @@ int launch_matmul(const char* name, int num_tokens, const void* input, const voi
 
   const long long tiles = static_cast<long long>((num_tokens + kBM - 1) / kBM) * ((n + params.bn - 1) / params.bn);
   const int grid = 2 * static_cast<int>(tiles < pairs ? tiles : pairs);
-  kernel<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(ma, mb, mr, mo, params);
-  return check_launch(name);
+  return launch_pdl(name, kernel, grid, kThreads, smem, stream, ma, mb, mr, mo, params);
 }
 
 }  // namespace

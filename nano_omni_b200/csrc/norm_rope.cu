@@ -77,8 +77,8 @@ __device__ __forceinline__ float sum_of_squares(const Row8& x) {
 // rounded to bf16 precision.  All lanes of the warp must call it.  N rows go through each stage together so that their
 // loads, shuffles and the divide / square root sequences overlap.
 template <int N, int NW = 1>  // NW = 1: one weight for all rows; NW = N: a weight per row
-__device__ __forceinline__ void norm_rope_rows(RowPart (&x)[N], const RowPart (&w)[NW], const float* __restrict__ cosines,
-                                               const float* __restrict__ sines, const int (&token)[N], int lane8,
+__device__ __forceinline__ void norm_rope_rows(RowPart (&x)[N], const RowPart (&w)[NW], const float* cosines,
+                                               const float* sines, const int (&token)[N], int lane8,
                                                bool use_rope) {
   const bool rotates = use_rope && lane8 < 6;
   float4 c[N][2], s[N][2];
@@ -156,8 +156,10 @@ struct NormRopeTensors {
 
 template <int TENSORS>
 __global__ void __launch_bounds__(256)
-norm_rope_kernel(const NormRopeTensors tensors, const float* __restrict__ cosines, const float* __restrict__ sines,
+norm_rope_kernel(const NormRopeTensors tensors, const float* cosines, const float* sines,
                  long long rows, int heads, int use_rope) {
+  pdl_wait();
+  pdl_release();
   const int lane8 = threadIdx.x & 7;
   const int at_a = 8 * chunk_a(lane8), at_b = 8 * chunk_b(lane8);
   RowPart w[TENSORS];
@@ -205,10 +207,12 @@ norm_rope_kernel(const NormRopeTensors tensors, const float* __restrict__ cosine
 
 // One CTA per (32-token group, head): 128 threads, 16 rows per pass, 2 passes.
 __global__ void __launch_bounds__(128)
-query_prepare_kernel(const __nv_bfloat16* __restrict__ src, const __nv_bfloat16* __restrict__ weight,
-                     const float* __restrict__ cosines, const float* __restrict__ sines,
-                     int8_t* __restrict__ quantized, float* __restrict__ scales, int tokens, int heads, int groups,
+query_prepare_kernel(const __nv_bfloat16* src, const __nv_bfloat16* weight,
+                     const float* cosines, const float* sines,
+                     int8_t* quantized, float* scales, int tokens, int heads, int groups,
                      int use_rope) {
+  pdl_wait();
+  pdl_release();
   const int head = blockIdx.x, group = blockIdx.y;  // heads fastest: CTAs in flight read whole rows of the source
   const int lane8 = threadIdx.x & 7, row_in_pass = threadIdx.x >> 3;
   const int at_a = 8 * chunk_a(lane8), at_b = 8 * chunk_b(lane8);
@@ -219,8 +223,8 @@ query_prepare_kernel(const __nv_bfloat16* __restrict__ src, const __nv_bfloat16*
   for (int p = 0; p < 2; ++p) {
     const int t = group * 32 + p * 16 + row_in_pass;
     const __nv_bfloat16* row = src + static_cast<size_t>(t < tokens ? t : 0) * columns + head * 128;
-    loaded[p][0] = __ldg(reinterpret_cast<const uint4*>(row + at_a));
-    loaded[p][1] = __ldg(reinterpret_cast<const uint4*>(row + at_b));
+    loaded[p][0] = *reinterpret_cast<const uint4*>(row + at_a);
+    loaded[p][1] = *reinterpret_cast<const uint4*>(row + at_b);
   }
   RowPart x[2];
   float amax = 0.f;
@@ -285,9 +289,8 @@ extern "C" int nob200_h3_head_norm_rope(int tokens, const void* input, const voi
   const NormRopeTensors tensors = {{static_cast<const __nv_bfloat16*>(input)},
                                    {static_cast<const __nv_bfloat16*>(weight)},
                                    {static_cast<__nv_bfloat16*>(output)}};
-  norm_rope_kernel<1><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      tensors, static_cast<const float*>(cosines), static_cast<const float*>(sines), rows, heads, cosines != nullptr);
-  return check_launch("h3_head_norm_rope");
+  return launch_pdl("h3_head_norm_rope", norm_rope_kernel<1>, grid, 256, 0, stream, tensors,
+                    static_cast<const float*>(cosines), static_cast<const float*>(sines), rows, heads, cosines != nullptr);
 }
 
 extern "C" int nob200_h3_qk_norm_rope(int tokens, void* query, void* key, const void* query_weight,
@@ -302,9 +305,8 @@ extern "C" int nob200_h3_qk_norm_rope(int tokens, void* query, void* key, const 
   auto *q = static_cast<__nv_bfloat16*>(query), *k = static_cast<__nv_bfloat16*>(key);
   const NormRopeTensors tensors = {
       {q, k}, {static_cast<const __nv_bfloat16*>(query_weight), static_cast<const __nv_bfloat16*>(key_weight)}, {q, k}};
-  norm_rope_kernel<2><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      tensors, static_cast<const float*>(cosines), static_cast<const float*>(sines), rows, heads, 1);
-  return check_launch("h3_qk_norm_rope");
+  return launch_pdl("h3_qk_norm_rope", norm_rope_kernel<2>, grid, 256, 0, stream, tensors,
+                    static_cast<const float*>(cosines), static_cast<const float*>(sines), rows, heads, 1);
 }
 
 extern "C" int nob200_h3_query_prepare(int tokens, const void* source, const void* weight, const void* cosines,
@@ -315,11 +317,10 @@ extern "C" int nob200_h3_query_prepare(int tokens, const void* source, const voi
   NOB_REQUIRE((cosines == nullptr) == (sines == nullptr), "h3_query_prepare: cosines and sines come together");
   const int groups = (tokens + 31) / 32;
   NOB_REQUIRE(groups <= 65535, "h3_query_prepare: %d token groups exceed the grid limit", groups);
-  query_prepare_kernel<<<dim3(heads, groups), 128, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(source), static_cast<const __nv_bfloat16*>(weight),
-      static_cast<const float*>(cosines), static_cast<const float*>(sines), static_cast<int8_t*>(quantized),
-      static_cast<float*>(scales), tokens, heads, groups, cosines != nullptr);
-  return check_launch("h3_query_prepare");
+  return launch_pdl("h3_query_prepare", query_prepare_kernel, dim3(heads, groups), 128, 0, stream,
+                    static_cast<const __nv_bfloat16*>(source), static_cast<const __nv_bfloat16*>(weight),
+                    static_cast<const float*>(cosines), static_cast<const float*>(sines), static_cast<int8_t*>(quantized),
+                    static_cast<float*>(scales), tokens, heads, groups, cosines != nullptr);
 }
 
 // ------------------------------------------------- row-wise int8 of the projection inputs, with group rotation
@@ -374,8 +375,10 @@ __device__ __forceinline__ void radix4(Pair& a, Pair& b, Pair& c, Pair& d) {
 // groups at once.  The kernel is bound by its instructions, about 30 per column one by one; with the packed rotation,
 // packed rounding and the boundary test below about half (15104 x 7168: 135 us, now 105 us; 50 us of traffic).
 __global__ void __launch_bounds__(128)
-rowwise_int8_kernel(const __nv_bfloat16* __restrict__ src, int8_t* __restrict__ dst, float* __restrict__ scales,
+rowwise_int8_kernel(const __nv_bfloat16* src, int8_t* dst, float* scales,
                     int columns, int rotate) {
+  pdl_wait();
+  pdl_release();
   extern __shared__ __align__(16) __nv_bfloat16 rotated[];  // the row after rotation and bf16 rounding
   __shared__ float warp_max[4];
   __shared__ uint64_t transpose[8][16 * 17];  // two 256-column groups per half-warp
@@ -510,8 +513,7 @@ extern "C" int nob200_int8_rowwise(int num_tokens, const void* input, void* outp
     if (err != cudaSuccess)
       return fail(kCudaError, "int8_rowwise: cannot reserve %zu B of shared memory: %s", smem, cudaGetErrorString(err));
   }
-  rowwise_int8_kernel<<<num_tokens, 128, smem, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(input), static_cast<int8_t*>(output), static_cast<float*>(scales), columns,
-      rotation_group == 256);
-  return check_launch("int8_rowwise");
+  return launch_pdl("int8_rowwise", rowwise_int8_kernel, num_tokens, 128, smem, stream,
+                    static_cast<const __nv_bfloat16*>(input), static_cast<int8_t*>(output), static_cast<float*>(scales),
+                    columns, rotation_group == 256);
 }

@@ -110,8 +110,10 @@ constexpr int kMeanChunk = 128;
 constexpr int kMeanBatch = 32;
 
 __global__ void __launch_bounds__(128, 6)  // a register budget that lets a batch of loads be in flight
-mean_chunk_kernel(const __nv_bfloat16* __restrict__ in, float* __restrict__ dst, int num_tokens, int columns,
+mean_chunk_kernel(const __nv_bfloat16* in, float* dst, int num_tokens, int columns,
                   int tokens_per_block, int chunks_per_group, int include_padding, int direct) {
+  pdl_wait();
+  pdl_release();
   const int col = (blockIdx.x * 128 + threadIdx.x) * 4;
   if (col >= columns) return;
   const int chunk_id = blockIdx.y;  // group * chunks_per_group + chunk
@@ -155,8 +157,10 @@ mean_chunk_kernel(const __nv_bfloat16* __restrict__ in, float* __restrict__ dst,
 constexpr int kFinishChunks = 256;
 
 __global__ void __launch_bounds__(256)
-mean_finish_kernel(const float* __restrict__ partial, float* __restrict__ out, int num_tokens, int columns,
+mean_finish_kernel(const float* partial, float* out, int num_tokens, int columns,
                    int tokens_per_block, int chunks_per_group, int include_padding) {
+  pdl_wait();
+  pdl_release();
   __shared__ float tile[kFinishChunks][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + lane;
@@ -196,9 +200,11 @@ mean_finish_kernel(const float* __restrict__ partial, float* __restrict__ out, i
 // registers of holding them as fp32, so five CTAs fit an SM and enough loads are in flight to keep HBM busy.
 template <int TPB, bool HADAMARD>
 __global__ void __launch_bounds__(TPB >= 64 ? 256 : 128, (TPB == 128 || HADAMARD) ? 1 : (TPB == 64 ? 5 : 10))
-quantize_qk_kernel(const __nv_bfloat16* __restrict__ src, const float* __restrict__ mean,
-                   int8_t* __restrict__ quantized, float* __restrict__ scales, int num_tokens, int heads,
+quantize_qk_kernel(const __nv_bfloat16* src, const float* mean,
+                   int8_t* quantized, float* scales, int num_tokens, int heads,
                    int num_blocks, int center) {
+  pdl_wait();
+  pdl_release();
   constexpr int kThreads = TPB >= 64 ? 256 : 128;
   constexpr int kRowsPerPass = kThreads / 16;
   constexpr int kPasses = TPB / kRowsPerPass;
@@ -211,7 +217,7 @@ quantize_qk_kernel(const __nv_bfloat16* __restrict__ src, const float* __restric
 #pragma unroll
   for (int p = 0; p < kPasses; ++p) {
     const int token = block * TPB + p * kRowsPerPass + row_in_pass;
-    raw[p] = token < num_tokens ? __ldg(reinterpret_cast<const uint4*>(src + static_cast<size_t>(token) * columns + ch))
+    raw[p] = token < num_tokens ? *reinterpret_cast<const uint4*>(src + static_cast<size_t>(token) * columns + ch)
                                 : make_uint4(0u, 0u, 0u, 0u);
   }
   Vec8 mu;
@@ -340,7 +346,9 @@ __global__ void value_scale_finish_kernel(float* __restrict__ scales, int column
 constexpr int kVScaleShort = 2048;
 
 __global__ void __launch_bounds__(512, 1)
-value_scale_short_kernel(const __nv_bfloat16* __restrict__ src, float* __restrict__ scales, int num_tokens, int columns) {
+value_scale_short_kernel(const __nv_bfloat16* src, float* scales, int num_tokens, int columns) {
+  pdl_wait();
+  pdl_release();
   __shared__ uint32_t part[16][64];
   const int group = threadIdx.x & 7, row = threadIdx.x >> 3, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const __nv_bfloat16* p = src + blockIdx.x * 64 + group * 8;  // columns is a multiple of 128
@@ -380,8 +388,10 @@ __device__ __forceinline__ uint32_t e4m3_of_quotient(float x, float scale, float
 }
 
 __global__ void __launch_bounds__(256)
-quantize_value_kernel(const __nv_bfloat16* __restrict__ src, const float* __restrict__ scale,
-                      uint8_t* __restrict__ out, int num_tokens, int heads, int padded_tokens) {
+quantize_value_kernel(const __nv_bfloat16* src, const float* scale,
+                      uint8_t* out, int num_tokens, int heads, int padded_tokens) {
+  pdl_wait();
+  pdl_release();
   // [channel][word of four stored positions]; the word index is XORed with the channel's group of 8 so
   // that the 16 channel groups of a warp hit 16 different banks
   __shared__ __align__(16) uint32_t tile[128][16];
@@ -406,7 +416,7 @@ quantize_value_kernel(const __nv_bfloat16* __restrict__ src, const float* __rest
   for (int b = 0; b < 4; ++b) {
     const int token = base_token + (b & 1) + 8 * (b >> 1);
     loaded[b] = token < num_tokens
-                 ? __ldg(reinterpret_cast<const uint4*>(src + static_cast<size_t>(token) * columns + head * 128 + ch))
+                 ? *reinterpret_cast<const uint4*>(src + static_cast<size_t>(token) * columns + head * 128 + ch)
                  : make_uint4(0u, 0u, 0u, 0u);
   }
 #pragma unroll
@@ -651,27 +661,23 @@ extern "C" int nob200_token_group_mean(int num_tokens, const void* input, void* 
   const size_t need = nob200_token_group_mean_workspace_bytes(num_tokens, columns, tokens_per_block);
   NOB_REQUIRE(need == 0 || (workspace && workspace_bytes >= need),
               "token_group_mean: workspace of %zu B required, %zu B given", need, workspace_bytes);
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int col_blocks = (columns / 4 + 127) / 128;
   // Only chunks that hold at least one token are launched per group; the grid's y
   // covers groups*chunks_per_group and empty chunks write zeros that are never read.
   const long long total_chunks = static_cast<long long>(groups) * chunks_per_group;
   NOB_REQUIRE(total_chunks <= 65535, "token_group_mean: %lld chunks exceed the grid limit", total_chunks);
   if (chunks_per_group == 1) {
-    mean_chunk_kernel<<<dim3(col_blocks, (unsigned)total_chunks), 128, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(input), static_cast<float*>(output), num_tokens, columns, eff_tpb, 1,
-        include_padding, 1);
-    return check_launch("token_group_mean");
+    return launch_pdl("token_group_mean", mean_chunk_kernel, dim3(col_blocks, (unsigned)total_chunks), 128, 0, stream,
+                      static_cast<const __nv_bfloat16*>(input), static_cast<float*>(output), num_tokens, columns, eff_tpb,
+                      1, include_padding, 1);
   }
-  mean_chunk_kernel<<<dim3(col_blocks, (unsigned)total_chunks), 128, 0, s>>>(
-      static_cast<const __nv_bfloat16*>(input), static_cast<float*>(workspace), num_tokens, columns, eff_tpb,
-      chunks_per_group, include_padding, 0);
-  int rc = check_launch("token_group_mean(partial)");
+  int rc = launch_pdl("token_group_mean(partial)", mean_chunk_kernel, dim3(col_blocks, (unsigned)total_chunks), 128, 0,
+                      stream, static_cast<const __nv_bfloat16*>(input), static_cast<float*>(workspace), num_tokens,
+                      columns, eff_tpb, chunks_per_group, include_padding, 0);
   if (rc) return rc;
-  mean_finish_kernel<<<dim3((columns + 31) / 32, groups), 256, 0, s>>>(
-      static_cast<const float*>(workspace), static_cast<float*>(output), num_tokens, columns, eff_tpb,
-      chunks_per_group, include_padding);
-  return check_launch("token_group_mean(finish)");
+  return launch_pdl("token_group_mean(finish)", mean_finish_kernel, dim3((columns + 31) / 32, groups), 256, 0, stream,
+                    static_cast<const float*>(workspace), static_cast<float*>(output), num_tokens, columns, eff_tpb,
+                    chunks_per_group, include_padding);
 }
 
 extern "C" int nob200_int8_fp8_quantize_qk(int num_tokens, const void* source, const void* statistics,
@@ -684,7 +690,6 @@ extern "C" int nob200_int8_fp8_quantize_qk(int num_tokens, const void* source, c
   NOB_REQUIRE(!center || statistics, "int8_fp8_quantize_qk: centring needs the statistics tensor");
   const int num_blocks = (num_tokens + tokens_per_block - 1) / tokens_per_block;
   NOB_REQUIRE(num_blocks <= 65535, "int8_fp8_quantize_qk: %d token blocks exceed the grid limit", num_blocks);
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
   const dim3 grid(heads, num_blocks);
   const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(source);
   const float* mean = static_cast<const float*>(statistics);
@@ -692,22 +697,15 @@ extern "C" int nob200_int8_fp8_quantize_qk(int num_tokens, const void* source, c
   float* sc = static_cast<float*>(scales);
   auto launch = [&](auto tokens_tag, auto hadamard_tag) {
     constexpr int kTokens = decltype(tokens_tag)::value;
-    quantize_qk_kernel<kTokens, decltype(hadamard_tag)::value>
-        <<<grid, kTokens >= 64 ? 256 : 128, 0, s>>>(src, mean, q, sc, num_tokens, heads, num_blocks, center);
+    return launch_pdl("int8_fp8_quantize_qk", quantize_qk_kernel<kTokens, decltype(hadamard_tag)::value>, grid,
+                      kTokens >= 64 ? 256 : 128, 0, stream, src, mean, q, sc, num_tokens, heads, num_blocks, center);
   };
   auto by_rotation = [&](auto tokens_tag) {
-    if (hadamard)
-      launch(tokens_tag, std::true_type{});
-    else
-      launch(tokens_tag, std::false_type{});
+    return hadamard ? launch(tokens_tag, std::true_type{}) : launch(tokens_tag, std::false_type{});
   };
-  if (tokens_per_block == 32)
-    by_rotation(std::integral_constant<int, 32>{});
-  else if (tokens_per_block == 64)
-    by_rotation(std::integral_constant<int, 64>{});
-  else
-    by_rotation(std::integral_constant<int, 128>{});
-  return check_launch("int8_fp8_quantize_qk");
+  if (tokens_per_block == 32) return by_rotation(std::integral_constant<int, 32>{});
+  if (tokens_per_block == 64) return by_rotation(std::integral_constant<int, 64>{});
+  return by_rotation(std::integral_constant<int, 128>{});
 }
 
 extern "C" int nob200_int8_fp8_value_scale(int num_tokens, const void* source, void* scales, int heads,
@@ -717,9 +715,8 @@ extern "C" int nob200_int8_fp8_value_scale(int num_tokens, const void* source, v
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int columns = heads * 128;
   if (num_tokens <= kVScaleShort) {
-    value_scale_short_kernel<<<columns / 64, 512, 0, s>>>(static_cast<const __nv_bfloat16*>(source),
-                                                          static_cast<float*>(scales), num_tokens, columns);
-    return check_launch("int8_fp8_value_scale(short)");
+    return launch_pdl("int8_fp8_value_scale(short)", value_scale_short_kernel, columns / 64, 512, 0, stream,
+                      static_cast<const __nv_bfloat16*>(source), static_cast<float*>(scales), num_tokens, columns);
   }
   cudaError_t err = cudaMemsetAsync(scales, 0, static_cast<size_t>(columns) * sizeof(float), s);
   if (err != cudaSuccess) return fail(kCudaError, "int8_fp8_value_scale: %s", cudaGetErrorString(err));
@@ -739,10 +736,9 @@ extern "C" int nob200_int8_fp8_quantize_value(int num_tokens, const void* source
   NOB_REQUIRE(source && scale && output, "int8_fp8_quantize_value: NULL tensor");
   const int blocks = (num_tokens + 63) / 64;
   NOB_REQUIRE(blocks <= 65535, "int8_fp8_quantize_value: %d token blocks exceed the grid limit", blocks);
-  quantize_value_kernel<<<dim3(heads, blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(source), static_cast<const float*>(scale), static_cast<uint8_t*>(output),
-      num_tokens, heads, blocks * 64);
-  return check_launch("int8_fp8_quantize_value");
+  return launch_pdl("int8_fp8_quantize_value", quantize_value_kernel, dim3(heads, blocks), 256, 0, stream,
+                    static_cast<const __nv_bfloat16*>(source), static_cast<const float*>(scale),
+                    static_cast<uint8_t*>(output), num_tokens, heads, blocks * 64);
 }
 
 extern "C" int nob200_nvfp4_prepare(int num_tokens, const void* source, const void* mean, void* quantized,

@@ -24,9 +24,11 @@ constexpr float kSqrt128 = 11.313708498984761f;
 // One CTA of 64 threads per (block, head); thread c2 owns channels 2*c2, 2*c2+1 and walks
 // the block's tokens in order (4-byte loads, 256 B per token row across the CTA).
 __global__ void __launch_bounds__(64)
-sol_pool_kernel(const __nv_bfloat16* __restrict__ key, const __nv_bfloat16* __restrict__ value,
-                const float* __restrict__ key_mean, __nv_bfloat16* __restrict__ out, int num_tokens, int heads,
+sol_pool_kernel(const __nv_bfloat16* key, const __nv_bfloat16* value,
+                const float* key_mean, __nv_bfloat16* out, int num_tokens, int heads,
                 int block, int num_blocks) {
+  pdl_wait();
+  pdl_release();
   const int b = blockIdx.x, head = blockIdx.y, c = threadIdx.x * 2;
   const int begin = b * block, end = min(begin + block, num_tokens);
   const size_t row_stride = static_cast<size_t>(heads) * 128;
@@ -77,7 +79,9 @@ constexpr int kStatsBlocks = 512, kStatsChannels = 32;
 
 template <bool ALIGNED>
 __global__ void __launch_bounds__(256)
-sol_stats_kernel(const __nv_bfloat16* __restrict__ pooled, float* __restrict__ out, int num_blocks) {
+sol_stats_kernel(const __nv_bfloat16* pooled, float* out, int num_blocks) {
+  pdl_wait();
+  pdl_release();
   __shared__ uint4 staged[kStatsBlocks][kStatsChannels / 8];
   const int head = blockIdx.x, c0 = blockIdx.y * kStatsChannels, lane = threadIdx.x;
   const __nv_bfloat16* p = pooled + static_cast<size_t>(head) * num_blocks * 128 + c0;
@@ -145,9 +149,11 @@ __device__ __forceinline__ uint64_t add_pair(uint64_t x, uint64_t y) {
 
 template <int ROWS, bool ALIGNED>
 __global__ void __launch_bounds__(kSelectThreads, 3)  // shared memory holds three; registers for 16 loads in flight
-sol_select_kernel(const __nv_bfloat16* __restrict__ query, const __nv_bfloat16* __restrict__ pooled_key,
-                  const float* __restrict__ stats, uint8_t* __restrict__ mask, float* __restrict__ scores,
+sol_select_kernel(const __nv_bfloat16* query, const __nv_bfloat16* pooled_key,
+                  const float* stats, uint8_t* mask, float* scores,
                   int num_tokens, int heads, int block, int num_blocks, int num_protected, float tau) {
+  pdl_wait();
+  pdl_release();
   constexpr int kQb = 4 * ROWS;
   extern __shared__ __align__(16) uint8_t select_smem[];
   SelectShared<ROWS>& S = *reinterpret_cast<SelectShared<ROWS>*>(select_smem);
@@ -306,8 +312,10 @@ constexpr int kTopkWarps = 4;
 
 template <int PER_LANE>
 __global__ void __launch_bounds__(32 * kTopkWarps)
-sol_topk_kernel(const float* __restrict__ scores, uint8_t* __restrict__ mask, int rows, int num_blocks,
+sol_topk_kernel(const float* scores, uint8_t* mask, int rows, int num_blocks,
                 int num_protected, int keep) {
+  pdl_wait();
+  pdl_release();
   const int row = blockIdx.x * kTopkWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= rows) return;
   const size_t base = static_cast<size_t>(row) * num_blocks;
@@ -374,9 +382,8 @@ struct SelectLaunch {
     const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess)
       return fail(kCudaError, "%s: cannot reserve %zu B of shared memory: %s", name, smem, cudaGetErrorString(err));
-    kernel<<<dim3((num_blocks + 4 * ROWS - 1) / (4 * ROWS), heads), kSelectThreads, smem, stream>>>(
-        query, pooled_key, stats, mask, scores, num_tokens, heads, block, num_blocks, num_protected, tau);
-    return check_launch(name);
+    return launch_pdl(name, kernel, dim3((num_blocks + 4 * ROWS - 1) / (4 * ROWS), heads), kSelectThreads, smem, stream,
+                      query, pooled_key, stats, mask, scores, num_tokens, heads, block, num_blocks, num_protected, tau);
   }
 
   // 8 query blocks per lane read the least shared memory per product, 4 make twice the CTAs: where 32-block CTAs
@@ -401,19 +408,17 @@ extern "C" int nob200_sol_pool(int num_tokens, const void* key, const void* valu
   NOB_REQUIRE(key && value && output, "sol_pool: NULL tensor");
   NOB_REQUIRE(heads <= 65535, "sol_pool: heads exceed the grid limit");
   const int nb = (num_tokens + block - 1) / block;
-  sol_pool_kernel<<<dim3(nb, heads), 64, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(key), static_cast<const __nv_bfloat16*>(value),
-      static_cast<const float*>(key_mean), static_cast<__nv_bfloat16*>(output), num_tokens, heads, block, nb);
-  return check_launch("sol_pool");
+  return launch_pdl("sol_pool", sol_pool_kernel, dim3(nb, heads), 64, 0, stream,
+                    static_cast<const __nv_bfloat16*>(key), static_cast<const __nv_bfloat16*>(value),
+                    static_cast<const float*>(key_mean), static_cast<__nv_bfloat16*>(output), num_tokens, heads, block, nb);
 }
 
 extern "C" int nob200_sol_stats(const void* pooled, void* output, int heads, int num_blocks, void* stream) {
   NOB_REQUIRE(heads > 0 && num_blocks > 0, "sol_stats: sizes must be positive");
   NOB_REQUIRE(pooled && output, "sol_stats: NULL tensor");
   auto* kernel = aligned16(pooled) ? sol_stats_kernel<true> : sol_stats_kernel<false>;
-  kernel<<<dim3(heads, 128 / kStatsChannels), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(pooled), static_cast<float*>(output), num_blocks);
-  return check_launch("sol_stats");
+  return launch_pdl("sol_stats", kernel, dim3(heads, 128 / kStatsChannels), 256, 0, stream,
+                    static_cast<const __nv_bfloat16*>(pooled), static_cast<float*>(output), num_blocks);
 }
 
 extern "C" size_t nob200_sol_select_workspace_bytes(int num_tokens, int heads, int block, int topk_blocks) {
@@ -454,7 +459,6 @@ extern "C" int nob200_sol_select(int num_tokens, int num_protected_blocks, const
                  : nb <= 512  ? sol_topk_kernel<16>
                  : nb <= 1024 ? sol_topk_kernel<32>
                               : sol_topk_kernel<64>;
-  kernel<<<(rows + kTopkWarps - 1) / kTopkWarps, 32 * kTopkWarps, 0, s>>>(
-      launch.scores, static_cast<uint8_t*>(output), rows, nb, num_protected_blocks, keep);
-  return check_launch("sol_select(topk)");
+  return launch_pdl("sol_select(topk)", kernel, (rows + kTopkWarps - 1) / kTopkWarps, 32 * kTopkWarps, 0, stream,
+                    launch.scores, static_cast<uint8_t*>(output), rows, nb, num_protected_blocks, keep);
 }
