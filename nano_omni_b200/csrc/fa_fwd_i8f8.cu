@@ -54,6 +54,7 @@ struct __align__(1024) Shared {
   uint64_t s_taken[2];     // the softmax warps of tile t hold them in registers: the buffer is free
   uint64_t p_full[2][2];   // P_t(j) is written, by parity of j (the softmax may run a tile ahead of the value issuer)
   uint64_t pv_done[2][2];  // O_t += P_t(j) V_j is complete, by parity of j: that P buffer is free, O_t may be rescaled
+  KeySplit::Share share;
   uint32_t tmem_base;
   uint32_t abort;
   float key_scale[kKeptScales];
@@ -96,14 +97,6 @@ fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   const int n_kv = share.kv_end - kv_begin;
   volatile uint32_t* abort_flag = &S.abort;
 
-  // Key scales of this CTA's keys, one per 64 keys (scales per `key_block`, 64 or 128 tokens), to shared memory: read
-  // from global memory inside the loop they cost 4 % of the kernel.
-  const int k_blocks = (num_kv_tokens + key_block - 1) / key_block;
-  const int halves_log2 = key_block == 128 ? 1 : 0;  // 64-key halves per key scale
-  const float* ks_head = key_scale + static_cast<size_t>(head) * k_blocks;
-  auto key_scale_of = [&](int half64) { return ks_head[min(half64 >> halves_log2, k_blocks - 1)]; };
-  for (int i = threadIdx.x; i < min(2 * n_kv, kKeptScales); i += kThreads) S.key_scale[i] = key_scale_of(2 * kv_begin + i);
-
   if (threadIdx.x == 0) {
     mbar_init(&S.q_full, 1);
     for (int s = 0; s < kStages; ++s) {
@@ -118,6 +111,7 @@ fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       mbar_init(&S.pv_done[t][0], 1);
       mbar_init(&S.pv_done[t][1], 1);
     }
+    S.share = share;
     S.abort = 0;
     mbar_fence_init();
   }
@@ -125,11 +119,22 @@ fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     tmem_alloc(&S.tmem_base, kTmemCols);
     tmem_relinquish();
   }
+  pdl_wait();  // launched as a programmatic dependent: the set-up above overlaps the kernel before
+
+  // Key scales of this CTA's keys, one per 64 keys (scales per `key_block`, 64 or 128 tokens), to shared memory: read
+  // from global memory inside the loop they cost 4 % of the kernel.  Behind the wait, because the kernel before may be
+  // the one that writes them.  Head and block count are worked out again for the few calls that read past the kept
+  // scales: kept in registers over the key loop, they spill there.
+  auto key_scale_of = [&](int in_head, int half64) {
+    const int k_blocks = (num_kv_tokens + key_block - 1) / key_block;
+    return key_scale[static_cast<size_t>(in_head) * k_blocks + min(key_block == 128 ? half64 >> 1 : half64, k_blocks - 1)];
+  };
+  for (int i = threadIdx.x; i < min(2 * n_kv, kKeptScales); i += kThreads) S.key_scale[i] = key_scale_of(head, 2 * kv_begin + i);
+
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = S.tmem_base;
-  pdl_wait();     // launched as a programmatic dependent: the set-up above overlaps the kernel before
   pdl_release();  // the merge of the shares may be scheduled behind the last CTAs
 
   if (warp >= 8) {
@@ -263,7 +268,8 @@ fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         if (2 * j + 1 < kKeptScales) {
           ks0 = S.key_scale[2 * j], ks1 = S.key_scale[2 * j + 1];
         } else {
-          ks0 = key_scale_of(2 * jt), ks1 = key_scale_of(2 * jt + 1);
+          const int in_head = KeySplit::reload(S.share).head;
+          ks0 = key_scale_of(in_head, 2 * jt), ks1 = key_scale_of(in_head, 2 * jt + 1);
         }
         ok = poll(&S.s_full[t], j & 1, kWaitTimeoutMma);
         if (!ok) break;
@@ -366,14 +372,17 @@ fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         unpack2(lb, l2, l3);
         const float l = (l0 + l1) + (l2 + l3);
         const float inv = 1.0f / l;
+        const KeySplit::Share at_end = KeySplit::reload(S.share);
+        const int head = at_end.head, q0 = at_end.q_tile * split.unit_rows;
+        const int token = q0 + t * kTile + (warp & 3) * 32 + lane;
         const float* vs = value_scale + head * 128;
-        const bool divided = share.piece >= 0;
+        const bool divided = at_end.piece >= 0;
         bool store = token < num_query_tokens && NOB_CHECK(head < heads, status);
         __nv_bfloat16* dst = out + (static_cast<size_t>(store ? token : 0) * heads + head) * 128;
         size_t row_at = 0;
         if (divided) {
           // the probability scale 448/8 is common to all shares and cancels in the merge
-          row_at = split.partial_row(share.piece, head, store ? token : q0, num_query_tokens);
+          row_at = split.partial_row(at_end.piece, head, store ? token : q0, num_query_tokens);
           store = store && NOB_CHECK(row_at < static_cast<size_t>(split.splits) * split.tail_rows, status);
           if (store) split.lse[row_at] = m_used + log2f(l);
         }
