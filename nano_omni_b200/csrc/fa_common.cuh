@@ -55,6 +55,12 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
+// NaN if either is (fmaxf returns the other one)
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float d;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+  return d;
+}
 // 2^x for a pair on the FMA pipe: x = n + r with n = round(x), r in [-0.5, 0.5];
 // 2^r by a degree-3 polynomial (relative error 7.5e-5, below bf16 resolution),
 // n added into the exponent field.  x is clamped at -126 (result ~1e-38).

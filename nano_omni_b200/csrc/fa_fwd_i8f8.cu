@@ -301,8 +301,9 @@ fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         }
         a0 = max3(a0, a2, fmaxf(__uint_as_float(s[62]), __uint_as_float(s[63])));
         a1 = max3(a1, a3, fmaxf(__uint_as_float(s[126]), __uint_as_float(s[127])));
-        // factors of the two 64-key halves, kept positive so that the -inf of a key past the end stays -inf under them
-        const float f0 = fmaxf(qf * ks0, 1e-30f), f1 = fmaxf(qf * ks1, 1e-30f);
+        // factors of the two 64-key halves, kept positive so that the -inf of a key past the end stays -inf under them; a
+        // scale that is not a number stays one and shows in the output
+        const float f0 = max_nan(qf * ks0, 1e-30f), f1 = max_nan(qf * ks1, 1e-30f);
         const float mx = fmaxf(a0 * f0, a1 * f1);
         if (j == 0) {
           m_used = mx;

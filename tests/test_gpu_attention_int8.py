@@ -270,3 +270,21 @@ def test_query_slice_operator_divides_the_keys():
     torch.cuda.synchronize()
     want = attend(prepared, Tq, Tk, h).cpu().float()
     assert (out.cpu().float() - want).abs().max() <= 2.0**-6 * v.float().abs().max().item()
+
+
+@pytest.mark.parametrize("what", ["key", "query"])
+def test_scales_that_are_not_numbers_show_in_the_output(what):
+    """A NaN key scale reaches every row of its head, a NaN query scale the 32 rows of its block, and nothing else."""
+    h, T, bad = 2, 300, 1
+    q, k, v = (randn_bf16(2900 + i, T, h * 128) for i in range(3))
+    clean = quantise(q, k, v, h)
+    want = attend(clean, T, T, h)
+    for block in range(0, 5 if what == "key" else 10, 4):  # a whole key tile, the ragged last one; first and last rows
+        scales = clean[4].clone() if what == "key" else clean[3].clone()
+        scales[bad, block] = float("nan")
+        operands = (*clean[:4], scales, clean[5]) if what == "key" else (*clean[:3], scales, *clean[4:])
+        got = attend(operands, T, T, h)
+        hit = torch.zeros(T, h, 128, dtype=torch.bool, device="cuda")
+        hit[slice(None) if what == "key" else slice(32 * block, 32 * block + 32), bad] = True
+        hit = hit.view(T, h * 128)
+        assert got[hit].isnan().all() and torch.equal(got[~hit], want[~hit])
