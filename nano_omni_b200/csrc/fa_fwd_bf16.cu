@@ -48,6 +48,9 @@ constexpr int kMmaWarp = 9;   // issues the score MMAs (S = Q K^T)
 constexpr int kPvWarp = 10;   // issues the value MMAs (O += P V)
 constexpr uint32_t kTmemCols = 512;
 constexpr float kRescaleThreshold = 8.0f;      // log2 units
+// Below every finite maximum (-FLT_MAX * log2e / sqrt(128) = -4.3e37).  Keys of score -inf then weigh 0 where a CTA's
+// first tile holds nothing else (relative to -inf they would be NaN); a share without weight has the log-sum-exp -inf.
+constexpr float kLowestMaximum = -1e38f;
 
 struct __align__(1024) Shared {
   uint8_t q[2][kTileBytes];
@@ -346,7 +349,7 @@ fa_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         if (lane == 0) TRACE(4 + warp, j, 2);
         bool pv_waited = j == 0;  // P_t and O_t are untouched by the tensor core before the first PV
         if (j == 0) {
-          m_used = mx;
+          m_used = fmaxf(mx, kLowestMaximum);
         } else if (__any_sync(0xffffffffu, mx > m_used + kRescaleThreshold)) {
           const float m_new = fmaxf(m_used, mx);
           const float alpha = ex2(m_used - m_new);
@@ -494,7 +497,9 @@ fa_merge_splits_kernel(const KeySplit split, const OutRoute out, int num_tokens,
   float wsum = 0.f;
   for (int z = 0; z < split.splits; ++z) {
     const size_t at = static_cast<size_t>(z * split.tail_rows + row);
-    const float w = exp2f(split.lse[at] - mx);
+    const float lse = split.lse[at];
+    if (lse == -INFINITY) continue;  // no weight in this share: its row is 0 / 0
+    const float w = exp2f(lse - mx);
     wsum += w;
     if (kF32) {
       const float4* src = reinterpret_cast<const float4*>(static_cast<const float*>(split.partial) + at * 128 + piece * 8);

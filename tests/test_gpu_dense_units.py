@@ -81,3 +81,23 @@ def test_int8_key_scales_past_the_kept_ones():
     want = torch.softmax(logits.double(), dim=1)[:, kept:].sum(1)
     # probabilities rounded to e4m3 in the numerator only: 2^-4 relative
     assert ((got.reshape(32, 128) - want[:, None]).abs() <= (2.0**-4 + 2.0**-8) * want[:, None] + 1e-4).all()
+
+
+@pytest.mark.parametrize("plan", [UnitPlan(256, 1, 0), UnitPlan(256, 2, 0), UnitPlan(256, 2, 1), UnitPlan(128, 4, 0)])
+@pytest.mark.parametrize("first", [False, True])
+def test_keys_of_no_weight_fill_a_share(monkeypatch, plan, first):
+    """Keys whose scores are minus infinity (here: overflow) weigh nothing, also where they are all that a share has."""
+    T, h = 512, 2
+    q, k, v = (randn_bf16(4900 + i, T, h * 128).float() for i in range(3))
+    none = slice(0, 256) if first else slice(256, 512)
+    live = slice(256, 512) if first else slice(0, 256)
+    big = 2.0**64
+    k = k / big
+    k[none] = -big / 4
+    q, k = (q.abs() * big).bfloat16(), k.bfloat16()
+    got = attend(monkeypatch, "bf16", plan, q, k, v.bfloat16(), T, h)
+    qs, ks, vs = (x.double().view(T, h, 128) for x in (q, k, v.bfloat16()))
+    weights = torch.softmax(torch.einsum("qhd,khd->hqk", qs, ks[live]) / 128**0.5, -1)
+    want = torch.einsum("hqk,khd->qhd", weights, vs[live])
+    # probabilities and output rounded to bf16
+    assert ((got - want).abs() <= 2 * 2.0**-9 * vs.abs().max() + 2.0**-8 * want.abs()).all()
