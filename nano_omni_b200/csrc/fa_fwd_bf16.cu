@@ -573,6 +573,7 @@ int make_key_split(KeySplit* split, const char* name, int num_query_tokens, int 
                    int kv_splits, int tail_units, bool partial_f32, void* workspace, size_t workspace_bytes) {
   const int n_kv = (num_kv_tokens + kTile - 1) / kTile;
   NOB_REQUIRE(unit_rows == kTile || unit_rows == 2 * kTile, "%s: unit_rows must be 128 or 256 (got %d)", name, unit_rows);
+  NOB_REQUIRE(heads <= 65535, "%s: heads %d exceeds the limit of 65535", name, heads);
   NOB_REQUIRE(kv_splits >= 1 && kv_splits <= 64 && kv_splits <= n_kv, "%s: kv_splits %d outside [1, min(64, %d)]",
               name, kv_splits, n_kv);
   const int q_tiles = (num_query_tokens + unit_rows - 1) / unit_rows;

@@ -170,3 +170,23 @@ def test_argument_rejection_of_the_later_entry_points(lib):
     fn.restype = ctypes.c_int
     assert fn(7, 1024, 1, p, null) == -1 and b"kind" in lib.nob200_last_error()
     assert fn(0, 1023, 1, p, null) == -1 and b"multiple of 4" in lib.nob200_last_error()
+
+
+def test_head_limit_of_the_dense_entry_points(lib):
+    """At most 65535 heads, by every launch of the dense kernels (no GPU needed)."""
+    lib.nob200_last_error.restype = ctypes.c_char_p
+    null, p, z, h = ctypes.c_void_p(0), ctypes.c_void_p(256), ctypes.c_size_t(0), 65536
+    name = "nob200_dense_bf16_attention_d128"
+    calls = {
+        name: (300, 0, p, p, p, p, h, h, null),
+        name + "_splitkv": (300, 0, p, p, p, p, h, h, 1, null, z, null),
+        name + "_units": (300, 0, p, p, p, p, h, h, 128, 1, 0, null, z, null),
+        "nob200_dense_int8_fp8_d128": (300, 300, p, p, p, p, p, p, p, h, null),
+        "nob200_dense_int8_fp8_d128_splitkv": (300, 300, p, p, p, p, p, p, p, h, 32, 64, 1, null, z, null),
+        "nob200_dense_int8_fp8_d128_units": (300, 300, p, p, p, p, p, p, p, h, 32, 64, 128, 1, 0, null, z, null),
+        "nob200_dense_int8_fp8_d128_blocks": (300, 300, p, p, p, p, p, p, p, h, 32, 64, null),
+    }
+    for symbol, arguments in calls.items():
+        fn = getattr(lib, symbol)
+        fn.restype = ctypes.c_int
+        assert fn(*arguments) == -1 and b"heads 65536" in lib.nob200_last_error(), symbol
