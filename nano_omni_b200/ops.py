@@ -204,7 +204,10 @@ class Op(abc.ABC):
         self.inputs = inputs
         self.output_specs = outputs
         self.outputs: tuple[TensorDesc, ...] | None = None
-        self._plans: dict[int, _Plan] = {}
+
+    def __setattr__(self, name: str, value) -> None:
+        super().__setattr__(name, value)
+        super().__setattr__("_plans", {})  # scratch address -> _Plan; made from the attributes as they were
 
     def to(self, *outputs: TensorDesc):
         """Bind the outputs once; returns this operator."""
@@ -244,9 +247,9 @@ class Op(abc.ABC):
     def run(self, scratch, stream: int | None = None) -> None:
         """Submit every call on ``stream``; ``scratch`` is a CUDA uint8 tensor of at least ``prepare()[1]`` bytes.
 
-        The plan is made once per scratch address and kept with the operator: its inputs, outputs and options are fixed
-        from ``to()`` on, so every later run replays the same C calls.  (Planning afresh on every run cost 60-390 us of
-        host time, more than the kernels of a small call take.)
+        The plan is made once per scratch address and kept with the operator until one of its attributes is set, so every
+        later run replays the same C calls.  (Planning afresh on every run cost 60-390 us of host time, more than the
+        kernels of a small call take.)
         """
         base = scratch.data_ptr()
         plan = self._plans.get(base)
@@ -260,19 +263,30 @@ class Op(abc.ABC):
                 raise RuntimeError(f"{function.__name__}: {_lib.last_error()} (status {code})")
 
     def _plan_for(self, base: int) -> _Plan:
+        known = self._plans
         calls, need = self.prepare()
         assert base % 256 == 0, "scratch must be 256-byte aligned"
         plan = _Plan(need, tuple(call for kernel in self._resolved(calls, base) for call in kernel.recorded()))
-        plans = dict(self._plans)
+        plans = dict(known)
         while len(plans) >= _KEPT_PLANS:
             del plans[next(iter(plans))]
         plans[base] = plan
-        self._plans = plans  # replaced whole: another thread that runs this operator sees the old or the new table
+        # replaced whole: another thread that runs this operator sees the old or the new table
+        if self._plans is known:  # else an attribute was set meanwhile
+            super().__setattr__("_plans", plans)
         return plan
 
     @abc.abstractmethod
     def kernels(self, scratch: ScratchLayout) -> Iterable[Kernel]:
         raise NotImplementedError
+
+
+def _holds_list(value) -> bool:
+    return isinstance(value, list) or (isinstance(value, tuple) and any(map(_holds_list, value)))
+
+
+def _as_tuples(value):
+    return tuple(map(_as_tuples, value)) if isinstance(value, (list, tuple)) else value
 
 
 class Linear(Op):
@@ -282,6 +296,15 @@ class Linear(Op):
     def __init__(self, input: TensorDesc, weight: TensorDesc, **options) -> None:
         super().__init__(input, weight, outputs=((DType.BF16, (input.shape[0], weight.shape[0])),))
         self.options = options
+        self._planned_options: tuple[dict | None, tuple | None] = (None, None)
+
+    def run(self, scratch, stream: int | None = None) -> None:
+        planned, lists = self._planned_options
+        if self.options != planned or (lists is not None and _as_tuples(list(self.options.values())) != lists):
+            # the dictionary, or a list in it, was changed in place
+            values = tuple(self.options.values())
+            self._planned_options = dict(self.options), _as_tuples(values) if _holds_list(values) else None
+        super().run(scratch, stream)
 
     def kernels(self, scratch: ScratchLayout) -> list[Kernel]:
         sequence = KernelSequence(scratch)
@@ -364,9 +387,16 @@ class DenseBf16Attention(_SliceAttention):
     def __init__(self, query, key, value, *, total_heads: int, head_offset: int = 0, kv_splits: int | None = None,
                  rotation: Rotation | None = None):  # fmt: skip
         super().__init__(query, key, value, total_heads=total_heads, head_offset=head_offset, rotation=rotation)
-        # an explicit count divides the keys of every unit
-        self.units = UnitPlan(256, kv_splits, 0) if kv_splits is not None else plan_units(self.rows, self.heads)
-        self.kv_splits = self.units.kv_splits
+        self.units = plan_units(self.rows, self.heads) if kv_splits is None else UnitPlan(256, kv_splits, 0)
+
+    @property
+    def kv_splits(self) -> int:
+        return self.units.kv_splits
+
+    @kv_splits.setter
+    def kv_splits(self, count: int) -> None:
+        """An explicit count divides the keys of every unit."""
+        self.units = UnitPlan(256, count, 0)
 
     def kernels(self, scratch: ScratchLayout) -> list[Kernel]:
         sequence = KernelSequence(scratch)
