@@ -188,6 +188,7 @@ class KernelSequence:
             raise ValueError(f"unsupported linear weight dtype: {weight.dtype}")
 
 
+_SUBMIT = Kernel.submit
 _KEPT_PLANS = 4  # scratch addresses an operator remembers: an arena per stream, seldom more than two
 
 
@@ -197,6 +198,19 @@ class _Plan:
 
     need: int
     calls: tuple[tuple[object, tuple], ...]
+    submit: object  # ``Kernel.submit`` as it was
+
+
+def _launches(kernel: Kernel) -> list[tuple[object, tuple]]:
+    """The calls of one launch: the recorded C calls, or the ``submit`` that a class (or a tool) has put in its place."""
+    if type(kernel).submit is _SUBMIT:
+        return kernel.recorded()
+
+    def submit(stream: ctypes.c_void_p) -> int:
+        kernel.submit(stream.value or 0)
+        return 0
+
+    return [(submit, ())]
 
 
 class Op(abc.ABC):
@@ -249,11 +263,11 @@ class Op(abc.ABC):
 
         The plan is made once per scratch address and kept with the operator until one of its attributes is set, so every
         later run replays the same C calls.  (Planning afresh on every run cost 60-390 us of host time, more than the
-        kernels of a small call take.)
+        kernels of a small call take.)  A kernel class with a ``submit`` of its own has it called instead.
         """
         base = scratch.data_ptr()
         plan = self._plans.get(base)
-        if plan is None:
+        if plan is None or plan.submit is not Kernel.submit:
             plan = self._plan_for(base)
         assert scratch.numel() * scratch.element_size() >= plan.need, f"operator needs {plan.need} B of scratch"
         stream = ctypes.c_void_p(_lib.current_stream() if stream is None else stream)
@@ -266,7 +280,9 @@ class Op(abc.ABC):
         known = self._plans
         calls, need = self.prepare()
         assert base % 256 == 0, "scratch must be 256-byte aligned"
-        plan = _Plan(need, tuple(call for kernel in self._resolved(calls, base) for call in kernel.recorded()))
+        kernels = self._resolved(calls, base) if type(self).bind is Op.bind else self.bind(base)
+        launches = tuple(call for kernel in kernels for call in _launches(kernel))
+        plan = _Plan(need, launches, Kernel.submit)
         plans = dict(known)
         while len(plans) >= _KEPT_PLANS:
             del plans[next(iter(plans))]

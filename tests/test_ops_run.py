@@ -9,7 +9,7 @@ import pytest
 import torch
 
 from nano_omni_b200 import _lib, ops
-from nano_omni_b200.core import DType, TensorDesc
+from nano_omni_b200.core import DType, Kernel, TensorDesc
 from nano_omni_b200.kernels.dense_bf16 import UnitPlan
 from tests.test_ops_plan import EXPECTED, make
 
@@ -112,6 +112,48 @@ def test_key_split_count_divides_every_unit(calls):
     op = make("dense", "bf16")
     op.kv_splits = 3
     assert op.kv_splits == 3 and op.prepare()[0][-1].config.kv_splits == 3 and op.units == UnitPlan(256, 3, 0)
+
+
+def test_submit_of_a_kernel_class_is_called(calls, monkeypatch):
+    """Classes (or tools) that put their own ``submit`` around a launch see the launches of operators too."""
+    op = make("sol", "bf16")
+    scratch = arena(op.prepare()[1])
+    expected = submitted(op, scratch, 0, calls)
+    op.run(scratch, 0)
+    assert calls == expected
+    seen = []
+    plain = Kernel.submit
+    monkeypatch.setattr(Kernel, "submit", lambda self, stream=None: (seen.append((self.name, stream)), plain(self, stream))[1])
+    del calls[:]
+    op.run(scratch, 0)
+    assert calls == expected and seen == [(name, 0) for name in EXPECTED[("sol", "bf16")]]
+
+    class Counted(ops.SolPoolKernel):
+        def submit(self, stream=None):
+            seen.append("counted")
+            super().submit(stream)
+
+    monkeypatch.undo()
+    monkeypatch.setattr(ops, "SolPoolKernel", Counted)
+    monkeypatch.setattr(_lib, "symbol", lambda name: lambda *arguments: 0)
+    op = make("sol", "bf16")
+    del seen[:]
+    for _ in range(2):
+        op.run(scratch, 7)
+    assert seen == ["counted"] * 2
+
+
+def test_bind_of_an_operator_class_is_used(calls):
+    class Twice(ops.DenseBf16Attention):
+        def bind(self, scratch_base):
+            return 2 * super().bind(scratch_base)
+
+    plain = make("dense", "bf16")
+    op = Twice(*plain.inputs, total_heads=plain.total_heads, head_offset=plain.head_offset).to(*plain.outputs)
+    scratch = arena(op.prepare()[1])
+    expected = submitted(plain, scratch, 3, calls)
+    op.run(scratch, 3)
+    assert calls == 2 * expected
 
 
 def test_a_failing_call_is_an_error(calls, monkeypatch):
