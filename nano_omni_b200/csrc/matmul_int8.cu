@@ -426,9 +426,11 @@ int tile_width(int m, int n, int k_chunks, int pairs) {
   return best;
 }
 
-// Pairs of CTAs the device holds at once (a property of the device, asked once per device and kernel).
-template <typename Kernel>
-int resident_pairs(Kernel kernel, size_t smem, int device) {
+// Pairs of CTAs of this kernel that the device holds at once, asked once per device and form of the kernel (both forms
+// have the same function type, so the form itself is the parameter).
+template <bool BF16>
+int resident_pairs(size_t smem, int device) {
+  auto kernel = matmul_kernel<BF16>;
   static std::atomic<int> known[64];
   if (device >= 0 && device < 64) {
     const int pairs = known[device].load(std::memory_order_relaxed);
@@ -467,7 +469,7 @@ int launch_matmul(const char* name, int num_tokens, const void* input, const voi
     return fail(kCudaError, "%s: cannot reserve %zu B of shared memory: %s", name, smem, cudaGetErrorString(err));
   int device = 0;
   cudaGetDevice(&device);
-  const int pairs = resident_pairs(kernel, smem, device);
+  const int pairs = resident_pairs<BF16>(smem, device);
   params.bn = tile_width(num_tokens, n, (params.k + kBK - 1) / kBK, pairs);
 
   CUtensorMap ma, mb, mr, mo;
