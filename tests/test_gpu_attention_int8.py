@@ -247,15 +247,16 @@ def test_key_splits_agree_with_one_share(Tq, Tk, splits):
 
 
 def test_query_slice_operator_divides_the_keys():
-    """QuerySlice picks key splits for a slice that would leave the last wave of SMs short, and the result stays that
-    of the unsplit kernel (attention_slices.py:113-161 is the reference operator)."""
+    """QuerySlice divides the keys of a slice that would leave the last wave of SMs short, and the result stays that of
+    the undivided kernel (attention_slices.py:113-161 is the reference operator)."""
     from nano_omni_b200 import ops as nob_ops
-    from nano_omni_b200.kernels.dense_bf16 import choose_kv_splits
+    from nano_omni_b200.kernels.dense_bf16 import choose_kv_splits, plan_units
 
     h, Tq, Tk = 37, 512, 4096
-    assert choose_kv_splits(4096, 56, num_kv_tokens=60778) == 2  # 896 CTAs: 6.05 waves of 148
-    splits = choose_kv_splits(Tq, h, num_kv_tokens=Tk)
-    assert splits == 2  # 74 CTAs on 148 SMs
+    assert choose_kv_splits(4096, 56, num_kv_tokens=60778) == 2  # the rule of the sequence-parallel path: 6.05 waves
+    assert plan_units(4096, 56, 60778).tail_units > 0  # the operator's: the units past the sixth wave
+    plan = plan_units(Tq, h, Tk)
+    assert plan.kv_splits > 1  # 74 units of 256 rows on 148 SMs
     q = randn_bf16(21, Tq, h * 128)
     k, v = randn_bf16(22, Tk, h * 128), randn_bf16(23, Tk, h * 128)
     prepared = quantise(q, k, v, h)
@@ -263,7 +264,8 @@ def test_query_slice_operator_divides_the_keys():
     out = torch.full((Tq, h * 128), float("nan"), dtype=torch.bfloat16, device="cuda")
     op = nob_ops.QuerySlice(desc(q), desc(k8), desc(ks), desc(v8), desc(vs), total_tokens=Tk).to(desc(out))
     calls, need = op.prepare()
-    assert calls[-1].config.kv_splits == splits
+    config = calls[-1].config
+    assert (config.query_rows, config.kv_splits, config.tail_units) == plan
     scratch = torch.empty(need + 256, dtype=torch.uint8, device="cuda")
     aligned = scratch[(-scratch.data_ptr()) % 256 :]
     op.run(aligned)

@@ -2,8 +2,10 @@
 
 Every plan computes the same attention; what differs is the grid the probabilities are rounded on, because a share
 tracks the running maximum of its own keys.  A normalised weight is off by at most half a step of that rounding in each
-of the two results (bf16 2^-9, e4m3 2^-4, the ue4m3 block scale of nvfp4 2^-4, relative; the row sums are unrounded), and
-the output is rounded to bf16, so outputs differ by at most 2 * step * max|v| + 2^-8 max|v|.
+of the two results (bf16 2^-9, e4m3 2^-4, the ue4m3 block scale of nvfp4 2^-4, relative; the row sums are unrounded).
+The values are independent N(0, 1), so the errors of a row's weights add by their squares, as the row itself does: over
+the rows of a query tile the results differ by at most sqrt(2) * step of their norm, and 2^-8 for the output in bf16.
+(A lost share of five changes a tile by 0.5 of its norm, heads or rows in the wrong place by 1.4.)
 """
 
 import pytest
@@ -50,7 +52,35 @@ def test_unit_plans_agree_with_whole_units(monkeypatch, precision, T, plan):
     whole = attend(monkeypatch, precision, UnitPlan(256, 1, 0), q, k, v, T, h)
     got = attend(monkeypatch, precision, plan, q, k, v, T, h)
     assert torch.isfinite(got).all()
-    assert (got - whole).abs().max().item() <= (2 * STEP[precision] + 2.0**-8) * v.float().abs().max().item()
+    for tile_got, tile_whole in zip(got.split(128), whole.split(128)):
+        off = (tile_got - tile_whole).norm(dim=(0, 2)) / tile_whole.norm(dim=(0, 2))  # per head
+        assert off.max().item() <= 2**0.5 * STEP[precision] + 2.0**-8
+
+
+@pytest.mark.parametrize("precision", ["bf16", "int8_fp8", "nvfp4"])
+@pytest.mark.parametrize(
+    "T,plan",
+    [
+        (257, UnitPlan(256, 2, 1)),
+        (640, UnitPlan(256, 5, 4)),
+        (1000, UnitPlan(128, 3, 0)),
+        (2100, UnitPlan(128, 4, 7)),
+        (2100, UnitPlan(256, 16, 5)),
+    ],
+)
+def test_every_share_counts_by_its_keys(monkeypatch, precision, T, plan):
+    """Equal weights, and values that name their key tile (the channel) and head (the height): a channel of the output is
+    its tile's part of the keys.  Values survive the quantisers exactly but for nvfp4's block scale (2^-4)."""
+    h = 3
+    q = torch.zeros(T, h * 128, dtype=torch.bfloat16, device="cuda")
+    k = randn_bf16(4700, T, h * 128)
+    tile = torch.arange(T, device="cuda") // 128
+    named = torch.nn.functional.one_hot(tile, 128).float()
+    height = torch.arange(1, h + 1, device="cuda", dtype=torch.float32)[:, None]
+    v = (named[:, None] * height).bfloat16().view(T, h * 128)
+    got = attend(monkeypatch, precision, plan, q, k, v, T, h)
+    want = (named.mean(0) * height).expand(T, h, 128)
+    assert ((got - want).abs() <= (2.0**-8 + (2.0**-4 if precision == "nvfp4" else 0.0)) * want + 1e-6).all()
 
 
 def test_plans_fill_the_last_wave():
