@@ -190,3 +190,17 @@ def test_head_limit_of_the_dense_entry_points(lib):
         fn = getattr(lib, symbol)
         fn.restype = ctypes.c_int
         assert fn(*arguments) == -1 and b"heads 65536" in lib.nob200_last_error(), symbol
+
+
+def test_workspace_of_key_shares_is_the_planned_one(lib):
+    """The library's size of the fp32 shares against the one that operators reserve (no GPU needed)."""
+    from nano_omni_b200.kernels.dense_bf16 import UnitPlan, key_share_workspace_bytes, plan_units
+
+    fn = lib.nob200_key_split_workspace_bytes
+    fn.restype = ctypes.c_size_t
+    for tokens, heads in ((1, 1), (127, 2), (129, 3), (640, 3), (1021, 14), (4096, 24), (9461, 14), (32768, 24)):
+        plans = [UnitPlan(rows, splits, tail) for rows in (128, 256) for splits in (1, 2, 7, 64) for tail in (0, 1, 2, heads)]
+        for plan in [*plans, plan_units(tokens, heads), plan_units(tokens, heads, 60778)]:
+            if plan.tail_units <= -(-tokens // plan.query_rows) * heads:
+                assert fn(tokens, heads, *plan) == key_share_workspace_bytes(tokens, heads, plan), (tokens, heads, plan)
+    assert fn(640, 3, 192, 2, 1) == fn(640, 3, 128, 65, 1) == fn(640, 3, 256, 2, 10) == 0  # refused by the launch

@@ -205,3 +205,40 @@ def test_benchmark_stated_quantisation_variants():
     # test holds the result to cosine 0.999 against the oracle on the same quantised operands
     assert torch.isfinite(got4).all() and rm.cosine(got4, want) >= 0.85
     assert (out4[:, :off] == 5).all() and (out4[:, off + h :] == 5).all()
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_runs_after_the_first_follow_inputs_scratch_and_stream(captured):
+    """An operator run again: other contents in the same input tensors, two scratch arenas in turn, each on a stream of
+    its own, and replayed from a graph.  Bit for bit what an operator made for that run gives."""
+    T, h = 1021, 3
+    shared = [torch.empty(T, h * 128, dtype=torch.bfloat16, device="cuda") for _ in range(3)]
+    out = torch.empty(T, h * 128, dtype=torch.bfloat16, device="cuda")
+    make = lambda tensors: ops.DenseInt8Fp8Attention(*(desc(t) for t in tensors))  # noqa: E731
+    op = make(shared).to(desc(out))
+    need = op.prepare()[1]
+    arenas = [torch.empty(need + 256, dtype=torch.uint8, device="cuda") for _ in range(2)]
+    arenas = [a[(-a.data_ptr()) % 256 :] for a in arenas]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    graphs = []
+    for i in range(6):
+        fresh = [randn_bf16(5200 + 3 * i + j, T, h * 128) for j in range(3)]
+        want = torch.empty_like(out)
+        execute(make(fresh), want)
+        for tensor, contents in zip(shared, fresh):
+            tensor.copy_(contents)
+        out.fill_(float("nan"))
+        scratch, stream = arenas[i % 2], streams[i % 2]
+        scratch.fill_(0xA5)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            if captured and i < 2:
+                op.run(scratch)
+                stream.synchronize()
+                out.fill_(float("nan"))
+                graphs.append(torch.cuda.CUDAGraph())
+                with torch.cuda.graph(graphs[i], stream=stream):
+                    op.run(scratch)
+            graphs[i % 2].replay() if captured else op.run(scratch)
+        torch.cuda.synchronize()
+        assert torch.equal(out.view(torch.int16), want.view(torch.int16)), i
