@@ -42,7 +42,7 @@ namespace nob200 {
 // Launches a kernel that calls pdl_wait() in every thread before it touches global memory: its CTAs may be brought onto
 // the SMs while the kernel before it in the stream drains (programmatic dependent launch), which takes the launch
 // latency (2-3 us) and the kernel's on-chip set-up off the path.
-// An operator is a chain of such launches: 1021 tokens x 14 heads int8-fp8, eight kernels, 64.4 -> 49.8 us; a bf16
+// Most kernels of an operator are launched so: 1021 tokens x 14 heads int8-fp8, eight kernels, 64.4 -> 49.8 us; a bf16
 // product of 512 x 7168 x 5376 43.5 -> 42.1 us; calls of milliseconds unchanged.
 template <typename... Params, typename... Args>
 int launch_pdl(const char* what, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, void* stream, Args&&... args) {

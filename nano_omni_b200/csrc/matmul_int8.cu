@@ -413,6 +413,9 @@ namespace {
 // Columns of a tile: the width whose waves over the pairs cost least.  A chunk of K takes 2 BN cycles of tensor work or,
 // below 256 columns, the load of its 16 KiB + BN/2 x 128 bytes per SM at 64 bytes per cycle; a tile's start and end
 // count as some chunks' worth.  Wide tiles win on long calls; a call of one short wave is spread over more pairs.
+// All seven widths timed on twelve shapes (int8 and bf16, 256 to 15104 rows, rank-64 products among them): the rule takes
+// the fastest in each (512 x 7168 x 5376 bf16: 44.2 us at 224, 97.3 at 64, 46.1 at 256; 1000 x 5376 x 7168 int8: 52.2 at
+// 160, 58.4 at 256), with any constant from 0 to 4000 in place of the 1000 cycles.
 int tile_width(int m, int n, int k_chunks, int pairs) {
   const long long m_tiles = (m + kBM - 1) / kBM;
   int best = kMaxBN;

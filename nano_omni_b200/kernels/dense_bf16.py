@@ -4,8 +4,8 @@ Interface of reference ``DenseBf16AttentionKernel``
 (src/nano_omni/kernels/attention/dense_bf16.py:13-36, 198-255): same Workload
 fields, Arguments fields and order, validation asserts and ``tops`` formula.
 The Config keeps the reference's field names so stored configs still validate,
-but the sm_100a kernel has one tile shape (two 128-row query tiles x 128 keys,
-384 threads) and ignores other choices.
+but the sm_100a kernel has one tile shape (128 query rows x 128 keys, one or two
+query tiles per CTA, 384 threads) and ignores other choices.
 """
 
 from __future__ import annotations
@@ -80,10 +80,11 @@ def plan_units(num_tokens: int, heads: int, num_kv_tokens: int | None = None, sm
     """Units and key shares of a dense launch, so that its last wave of CTAs fills the SMs.
 
     A unit is 256 (or 128) query rows of one head on one SM.  The units past the last full wave, or those and one wave
-    more, may have their keys divided.  Times are counted in key tiles of a 256-row unit (1.6 us): a 128-row unit
-    takes 0.72 of one per key tile; a CTA costs 4 beside its tiles (launch, first loads, pipeline fill, epilogue: 6-7
-    us), the merge 2.5 and 0.025 per 256-row share (fp32 rows written and read through L2).  The plain launch (256 rows,
-    no shares) stays unless the estimate falls by 2 %.
+    more, may have their keys divided.  Times are counted in key tiles of a 256-row unit; the counts were measured on the
+    bf16 kernel, whose tile takes 1.6 us (int8-fp8 1.5, nvfp4 1.7): a 128-row unit takes 0.72 of one per key tile; a CTA
+    costs 4 beside its tiles (launch, first loads, pipeline fill, epilogue: 6-7 us), the merge 2.5 and 0.025 per 256-row
+    share (fp32 rows written and read through L2).  The plain launch (256 rows, no shares) stays unless the estimate
+    falls by 2 %.  ``sm_count`` is that of a B200.
     """
     tiles = -(-(num_tokens if num_kv_tokens is None else num_kv_tokens) // 128)
     best, plan = None, UnitPlan(256, 1, 0)

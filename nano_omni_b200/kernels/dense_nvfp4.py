@@ -4,8 +4,7 @@ Interface of reference ``DenseNvfp4Kernel`` (src/nano_omni/kernels/attention/den
 562-676): same Arguments fields and order, the same shapes accepted and rejected, the same ``tops``.  Both
 products run as block-scaled fp4 tensor-core MMAs; probabilities are re-quantised to e2m1 with one ue4m3 scale per
 16 keys as in the reference kernel (dense_nvfp4.py:255-289).  The trailing ``workspace`` (no counterpart in the
-reference) is accepted for callers written against the earlier bf16-expansion path and ignored: the kernel needs
-no scratch.
+reference) holds the fp32 key shares when the Config divides keys (``kv_splits`` > 1) and is ignored otherwise.
 """
 
 from __future__ import annotations
