@@ -56,6 +56,9 @@ def test_nothing_is_read_before_the_wait(file, name, parameters, body):
             assert not re.search(rf"\b{word}\b", before), f"{name} touches {word} before the wait"
         else:  # a record of sizes and pointers: its members may be copied, not reached through
             assert not re.search(rf"\b{word}\.\w+\s*(\[|->)|[=(,;{{]\s*\*\s*{word}\.\w+", before), f"{name} reads through {word}"
+        # loads that the compiler may take for constant could be moved above the wait
+        assert not ("const" in parameter and "__restrict__" in parameter), f"{name}: {word}"
+    assert "__ldg" not in body
     assert not re.search(r"\breturn\b", before), "a thread may leave before the wait"
 
 
