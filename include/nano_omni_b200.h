@@ -371,6 +371,19 @@ int nob200_matmul_int8(int num_tokens, const void* input, const void* weight, co
                        int k, int use_silu, void* stream);
 
 /*
+ * nob200_matmul_int8 with up to two low-rank adapters inside: the products sum_r compressed_i[m, r] * expansion_i[n, r]
+ * (bf16 operands, fp32 accumulation) join the scaled sum before bias and residual.  compressed_i bf16 [num_tokens, rank_i]
+ * (the strength belongs into it), expansion_i bf16 [n, rank_i], rank_i a multiple of 64; rank1 0 (pointers NULL): one
+ * adapter.  Replaces the chain of MatmulBf16Kernel updates through the residual
+ * (src/nano_omni/ops/matmul/sequence.py:160-200), without rounding in between.
+ */
+int nob200_matmul_int8_adapters(int num_tokens, const void* input, const void* weight, const void* bias,
+                                const void* residual, const void* multiply, void* output, const void* weight_scale,
+                                const void* input_scale, int n, int k, int use_silu, const void* compressed0,
+                                const void* expansion0, int rank0, const void* compressed1, const void* expansion1, int rank1,
+                                void* stream);
+
+/*
  * BF16 GEMM with the same fused epilogue: the bf16 projections and the LoRA side products of a projection
  * (compress: input x down^T; update: compressed x up^T * strength + residual).
  * Replaces MatmulBf16Kernel / program matmul_bf16 (src/nano_omni/kernels/matmul/matmul_bf16.py:29-207; Arguments:
@@ -382,6 +395,12 @@ int nob200_matmul_int8(int num_tokens, const void* input, const void* weight, co
 int nob200_matmul_bf16(int num_tokens, const void* input, const void* weight, const void* bias, const void* residual,
                        const void* multiply, void* output, float output_scale, int n, int k, int use_silu,
                        void* stream);
+
+/* The same with adapters inside (see nob200_matmul_int8_adapters); output_scale is 1. */
+int nob200_matmul_bf16_adapters(int num_tokens, const void* input, const void* weight, const void* bias,
+                                const void* residual, const void* multiply, void* output, int n, int k, int use_silu,
+                                const void* compressed0, const void* expansion0, int rank0, const void* compressed1,
+                                const void* expansion1, int rank1, void* stream);
 
 /*
  * Row-wise int8 of the projection inputs.  rotation_group 0 replaces Int8RowwiseKernel / program int8_rowwise

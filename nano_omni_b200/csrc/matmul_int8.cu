@@ -26,10 +26,16 @@
 //             different lines per instruction, and that bounded the products with a short K (LoRA updates).
 // int8 15104 x 5376 x 7168 395 -> 347 us (2 N M K at the measured rate: 346), the rank-64 pair beside it 175 -> 144 us,
 // bf16 512 x 7168 x 5376 42 -> 36 us.
+// Low-rank adapters (the ADAPTED form) are multiplied inside: sum_r compressed[m, r] * expansion[n, r], one more chunk of
+// K per 64 of the rank.  bf16: behind the main operands' chunks, into the same accumulator.  int8: the epilogue warps first
+// turn the int32 accumulator into scaled fp32 in place, and kind::f16 MMAs add to that, behind the first chunks of the next
+// tile so that the tensor pipe does not wait for them.  As GEMMs of their own the updates are bound by the output they read
+// and write: a rank-64 pair with 15104 x 5376 x 7168 int8 took 664 us, inside it takes 604.
 // BN is 64 .. 256, chosen per shape by tile_width().  Every wait is bounded.
 #include <cuda.h>
 
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
 #include "fa_common.cuh"
@@ -49,6 +55,10 @@ constexpr int kStep = 32;         // columns per epilogue step
 constexpr int kStagingTiles = 4;  // per epilogue warp: [32 rows][64 bytes], 64-byte swizzle
 constexpr int kStagingBytes = 32 * kStep * 2;
 constexpr uint32_t kTmemCols = 512;
+constexpr int kMaxAdapters = 2;
+// int8 form: the adapters of a tile are multiplied behind this many chunks of the next one, when the epilogue warps have
+// long turned the tile's accumulator into fp32 (about three chunks) and long before they must have drained it
+constexpr int kAdapterDelay = 8;
 
 struct __align__(1024) GemmShared {
   uint8_t a[kStages][kABytes];
@@ -58,6 +68,8 @@ struct __align__(1024) GemmShared {
   uint64_t empty[kStages];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];  // the leader's; sixteen warps arrive
+  uint64_t acc_scaled[2];    // int8 with adapters, the leader's: the accumulator holds scaled fp32; sixteen warps arrive
+  uint64_t adapter_full[2];  // and the adapters' products
   uint64_t residual_full[kEpilogueWarps][kStagingTiles];
   uint32_t tmem_base;
   uint32_t abort;
@@ -73,7 +85,13 @@ struct GemmParams {
   int m, n, k, use_silu;  // k in bytes of a row
   int bn;                 // columns of a tile, a multiple of 32
   float output_scale;     // bf16 form only
+  int adapter_chunks[kMaxAdapters];  // ADAPTED form: chunks of 64 columns of each adapter's rank
   uint32_t* status;
+};
+
+// Operands of the adapters' products, bf16: the compressed activations [M, rank] and the expansion [N, rank].
+struct AdapterMaps {
+  CUtensorMap compressed[kMaxAdapters], expansion[kMaxAdapters];
 };
 
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
@@ -146,11 +164,11 @@ __device__ __forceinline__ void mma_pair_chunk(uint32_t d, uint64_t a, uint64_t 
 #undef NOB_MMA4
 }
 
-template <bool BF16>
+template <bool BF16, bool ADAPTED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
               const __grid_constant__ CUtensorMap map_residual, const __grid_constant__ CUtensorMap map_output,
-              const GemmParams P) {
+              const __grid_constant__ AdapterMaps maps, const GemmParams P) {
   extern __shared__ uint8_t smem_raw[];
   GemmShared& S = *reinterpret_cast<GemmShared*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -162,6 +180,7 @@ matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
   const int num_tiles = m_tiles * n_tiles;
   const int first_tile = blockIdx.x >> 1, tile_stride = gridDim.x >> 1;
   const int k_chunks = (P.k + kBK - 1) / kBK;
+  const int adapter_at = min(kAdapterDelay, k_chunks - 1);  // chunk of a tile ahead of which the tile before is completed
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -171,6 +190,8 @@ matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
     for (int b = 0; b < 2; ++b) {
       mbar_init(&S.acc_full[b], 1);
       mbar_init(&S.acc_empty[b], 2 * kEpilogueWarps);
+      mbar_init(&S.acc_scaled[b], 2 * kEpilogueWarps);
+      mbar_init(&S.adapter_full[b], 1);
     }
     for (int w = 0; w < kEpilogueWarps; ++w)
       for (int i = 0; i < kStagingTiles; ++i) mbar_init(&S.residual_full[w][i], 1);
@@ -203,21 +224,33 @@ matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
       const uint32_t stage_bytes = static_cast<uint32_t>(kABytes + bn / 2 * kBK);
       int issued = 0;
       bool ok = true;
+      auto load = [&](const CUtensorMap* a, const CUtensorMap* b, int column, int m0, int n0) {
+        const int st = issued % kStages;
+        if (issued >= kStages) {
+          ok = mbar_wait(&S.empty[st], ((issued / kStages) - 1) & 1, abort_flag, status, kWaitTimeoutRing);
+          if (!ok) return;
+        }
+        // the phase cannot complete before the leader's arrival, so the follower's bytes may come first
+        if (rank == 0) mbar_expect_tx(&S.full[st], 2 * stage_bytes);
+        const uint32_t bar = leader_address(&S.full[st]);
+        tma_load_pair(S.a[st], a, bar, column, m0, 0);
+        tma_load_pair(S.b[st], b, bar, column, n0, 0);
+        ++issued;
+      };
+      auto load_adapters = [&](int tile) {
+        const int m0 = (tile / n_tiles) * kBM + rank * (kBM / 2), n0 = (tile % n_tiles) * bn + rank * (bn / 2);
+        for (int i = 0; i < kMaxAdapters; ++i)
+          for (int c = 0; ok && c < P.adapter_chunks[i]; ++c)
+            load(&maps.compressed[i], &maps.expansion[i], c * (kBK / 2), m0, n0);
+      };
       for (int tile = first_tile; ok && tile < num_tiles; tile += tile_stride) {
         const int m0 = (tile / n_tiles) * kBM + rank * (kBM / 2), n0 = (tile % n_tiles) * bn + rank * (bn / 2);
-        for (int kc = 0; kc < k_chunks; ++kc, ++issued) {
-          const int st = issued % kStages;
-          if (issued >= kStages) {
-            ok = mbar_wait(&S.empty[st], ((issued / kStages) - 1) & 1, abort_flag, status, kWaitTimeoutRing);
-            if (!ok) break;
-          }
-          // the phase cannot complete before the leader's arrival, so the follower's bytes may come first
-          if (rank == 0) mbar_expect_tx(&S.full[st], 2 * stage_bytes);
-          const uint32_t bar = leader_address(&S.full[st]);
+        for (int kc = 0; ok && kc < k_chunks; ++kc) {
+          if (ADAPTED && !BF16 && kc == adapter_at && tile != first_tile) load_adapters(tile - tile_stride);
           constexpr int kElementsPerChunk = BF16 ? kBK / 2 : kBK;
-          tma_load_pair(S.a[st], &map_a, bar, kc * kElementsPerChunk, m0, 0);
-          tma_load_pair(S.b[st], &map_b, bar, kc * kElementsPerChunk, n0, 0);
+          if (ok) load(&map_a, &map_b, kc * kElementsPerChunk, m0, n0);
         }
+        if (ADAPTED && (BF16 || tile + tile_stride >= num_tiles)) load_adapters(tile);
       }
       // the last commits have reported here before this CTA's barriers go away
       for (int i = issued > kStages ? issued - kStages : 0; ok && i < issued; ++i)
@@ -232,6 +265,32 @@ matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
       const uint64_t a0 = desc + (smem_u32(S.a[0]) >> 4), b0 = desc + (smem_u32(S.b[0]) >> 4);
       int taken = 0, round = 0;
       bool ok = true;
+      // the next stage of the ring, into accumulator `d`
+      auto multiply = [&](auto bf16_tag, uint32_t d, uint32_t instruction, bool accumulate, uint64_t* then) {
+        const int st = taken % kStages;
+        ok = warp_rest(&S.full[st], (taken / kStages) & 1, abort_flag, status, kWaitTimeoutLoad);
+        if (!ok) return;
+        tc_fence_after();
+        if (elect_one()) {
+          mma_pair_chunk<decltype(bf16_tag)::value>(d, a0 + st * (kABytes >> 4), b0 + st * (kBBytes >> 4), instruction,
+                                                    accumulate ? 1u : 0u);
+          commit_pair(&S.empty[st]);
+          if (then) commit_pair(then);
+        }
+        __syncwarp();
+        ++taken;
+      };
+      const int adapter_chunks = ADAPTED ? P.adapter_chunks[0] + P.adapter_chunks[1] : 0;
+      // int8: the adapters of the tile of round `r`, on top of its scaled fp32 accumulator
+      auto adapters = [&](int r) {
+        const int buf = r & 1;
+        ok = warp_rest(&S.acc_scaled[buf], (r >> 1) & 1, abort_flag, status, kWaitTimeoutSoftmax);
+        if (!ok) return;
+        tc_fence_after();
+        for (int c = 0; ok && c < adapter_chunks; ++c)
+          multiply(std::true_type{}, tmem + buf * kMaxBN, umma_idesc(kDF32, kFmtBF16, kFmtBF16, 0, 0, kBM, bn), true,
+                   c + 1 == adapter_chunks ? &S.adapter_full[buf] : nullptr);
+      };
       for (int tile = first_tile; ok && tile < num_tiles; tile += tile_stride, ++round) {
         const int buf = round & 1;
         if (round >= 2) {  // both CTAs' epilogues must have drained this accumulator (its (round / 2)-th use)
@@ -240,18 +299,12 @@ matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
           tc_fence_after();
         }
         const uint32_t d = tmem + buf * kMaxBN;
-        for (int kc = 0; kc < k_chunks; ++kc, ++taken) {
-          const int st = taken % kStages;
-          ok = warp_rest(&S.full[st], (taken / kStages) & 1, abort_flag, status, kWaitTimeoutLoad);
-          if (!ok) break;
-          tc_fence_after();
-          if (elect_one()) {
-            mma_pair_chunk<BF16>(d, a0 + st * (kABytes >> 4), b0 + st * (kBBytes >> 4), idesc, kc > 0 ? 1u : 0u);
-            commit_pair(&S.empty[st]);
-            if (kc + 1 == k_chunks) commit_pair(&S.acc_full[buf]);
-          }
-          __syncwarp();
+        const int chunks = k_chunks + (BF16 ? adapter_chunks : 0);
+        for (int kc = 0; ok && kc < chunks; ++kc) {
+          if (ADAPTED && !BF16 && kc == adapter_at && round > 0) adapters(round - 1);
+          if (ok) multiply(std::bool_constant<BF16>{}, d, idesc, kc > 0, kc + 1 == chunks ? &S.acc_full[buf] : nullptr);
         }
+        if (ADAPTED && !BF16 && ok && tile + tile_stride >= num_tiles) adapters(round);
       }
     }
   } else {
@@ -299,6 +352,34 @@ matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
       ok = warp_rest(&S.acc_full[buf], (round >> 1) & 1, abort_flag, status, kWaitTimeoutMma);
       if (!ok) break;
       tc_fence_after();
+      if constexpr (ADAPTED && !BF16) {
+        // the products of the main operands to scaled fp32, in place, and the adapters' on top of them
+#pragma unroll 1
+        for (int c = group; c < steps; c += 2) {
+          const int col0 = n0 + kStep * c;
+          const uint32_t addr = tmem + lane_base + buf * kMaxBN + kStep * c;
+          uint32_t acc[kStep];
+          tmem_ld32(addr, acc);
+          tc_wait_ld();
+#pragma unroll
+          for (int i = 0; i < kStep; i += 4) {
+            const float4 ws = col0 + i < P.n ? *reinterpret_cast<const float4*>(P.weight_scale + col0 + i)
+                                             : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float w[4] = {ws.x, ws.y, ws.z, ws.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              acc[i + k] = __float_as_uint(__fmul_rn(__fmul_rn(static_cast<float>(static_cast<int>(acc[i + k])), w[k]), in_scale));
+          }
+          tmem_st32(addr, acc);
+        }
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) leader_arrive(leader_address(&S.acc_scaled[buf]));
+        ok = warp_rest(&S.adapter_full[buf], (round >> 1) & 1, abort_flag, status, kWaitTimeoutMma);
+        if (!ok) break;
+        tc_fence_after();
+      }
 #pragma unroll 1
       for (int c = group; c < steps; c += 2) {
         const int col0 = n0 + kStep * c;
@@ -332,7 +413,10 @@ matmul_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
           const int col = col0 + 8 * g;
           if (col < P.n) {
             float v[8];
-            if constexpr (BF16) {
+            if constexpr (ADAPTED) {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(acc[8 * g + i]);
+            } else if constexpr (BF16) {
 #pragma unroll
               for (int i = 0; i < 8; ++i) v[i] = __fmul_rn(__uint_as_float(acc[8 * g + i]), P.output_scale);
             } else {
@@ -431,9 +515,9 @@ int tile_width(int m, int n, int k_chunks, int pairs) {
 
 // Pairs of CTAs of this kernel that the device holds at once, asked once per device and form of the kernel (both forms
 // have the same function type, so the form itself is the parameter).
-template <bool BF16>
+template <bool BF16, bool ADAPTED>
 int resident_pairs(size_t smem, int device) {
-  auto kernel = matmul_kernel<BF16>;
+  auto kernel = matmul_kernel<BF16, ADAPTED>;
   static std::atomic<int> known[64];
   if (device >= 0 && device < 64) {
     const int pairs = known[device].load(std::memory_order_relaxed);
@@ -455,9 +539,26 @@ int resident_pairs(size_t smem, int device) {
   return pairs;
 }
 
-template <bool BF16>
+struct Adapters {  // rank 0: there is none
+  const void* compressed[kMaxAdapters] = {};
+  const void* expansion[kMaxAdapters] = {};
+  int ranks[kMaxAdapters] = {};
+};
+
+int check_adapters(const char* name, const Adapters& adapters) {
+  NOB_REQUIRE(adapters.ranks[0] > 0, "%s: rank %d of the first adapter", name, adapters.ranks[0]);
+  for (int i = 0; i < kMaxAdapters; ++i) {
+    NOB_REQUIRE(adapters.ranks[i] >= 0 && adapters.ranks[i] % 64 == 0, "%s: rank %d of adapter %d is no multiple of 64", name,
+                adapters.ranks[i], i);
+    NOB_REQUIRE(adapters.ranks[i] == 0 || (adapters.compressed[i] && adapters.expansion[i]), "%s: NULL tensor of adapter %d",
+                name, i);
+  }
+  return kOk;
+}
+
+template <bool BF16, bool ADAPTED>
 int launch_matmul(const char* name, int num_tokens, const void* input, const void* weight, int n, int k,
-                  GemmParams params, void* stream) {
+                  GemmParams params, void* stream, const Adapters& adapters = Adapters()) {
   const int element = BF16 ? 2 : 1;
   params.m = num_tokens;
   params.n = n;
@@ -465,14 +566,14 @@ int launch_matmul(const char* name, int num_tokens, const void* input, const voi
   params.status = status_word_device_ptr();
   if (!params.status) return fail(kCudaError, "%s: no current CUDA device", name);
 
-  auto kernel = matmul_kernel<BF16>;
+  auto kernel = matmul_kernel<BF16, ADAPTED>;
   const size_t smem = sizeof(GemmShared) + 1024;
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (err != cudaSuccess)
     return fail(kCudaError, "%s: cannot reserve %zu B of shared memory: %s", name, smem, cudaGetErrorString(err));
   int device = 0;
   cudaGetDevice(&device);
-  const int pairs = resident_pairs<BF16>(smem, device);
+  const int pairs = resident_pairs<BF16, ADAPTED>(smem, device);
   params.bn = tile_width(num_tokens, n, (params.k + kBK - 1) / kBK, pairs);
 
   CUtensorMap ma, mb, mr, mo;
@@ -490,22 +591,35 @@ int launch_matmul(const char* name, int num_tokens, const void* input, const voi
   mr = mo;
   if (params.residual && (rc = wide(&mr, params.residual))) return rc;
 
+  AdapterMaps maps = {};
+  for (int i = 0; i < kMaxAdapters && adapters.ranks[i]; ++i) {
+    const uint64_t rank = adapters.ranks[i];
+    params.adapter_chunks[i] = adapters.ranks[i] / 64;
+    if ((rc = make_tensor_map_3d(&maps.compressed[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, adapters.compressed[i], rank,
+                                 num_tokens, 1, rank * 2, rank * 2 * num_tokens, 64, kBM / 2, 1)))
+      return rc;
+    if ((rc = make_tensor_map_3d(&maps.expansion[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, adapters.expansion[i], rank, n, 1,
+                                 rank * 2, rank * 2 * n, 64, params.bn / 2, 1)))
+      return rc;
+  }
+
   const long long tiles = static_cast<long long>((num_tokens + kBM - 1) / kBM) * ((n + params.bn - 1) / params.bn);
   const int grid = 2 * static_cast<int>(tiles < pairs ? tiles : pairs);
-  return launch_pdl(name, kernel, grid, kThreads, smem, stream, ma, mb, mr, mo, params);
+  return launch_pdl(name, kernel, grid, kThreads, smem, stream, ma, mb, mr, mo, maps, params);
 }
 
 }  // namespace
 }  // namespace nob200
 
-extern "C" int nob200_matmul_int8(int num_tokens, const void* input, const void* weight, const void* bias,
-                                  const void* residual, const void* multiply, void* output, const void* weight_scale,
-                                  const void* input_scale, int n, int k, int use_silu, void* stream) {
-  using namespace nob200;
-  NOB_REQUIRE(num_tokens > 0 && n > 0 && k > 0, "matmul_int8: sizes must be positive");
-  NOB_REQUIRE(input && weight && output && weight_scale && input_scale, "matmul_int8: NULL tensor");
-  NOB_REQUIRE(k % 16 == 0, "matmul_int8: k (%d) must be a multiple of 16 (row pitch of the TMA tiles)", k);
-  NOB_REQUIRE(n % 8 == 0, "matmul_int8: n (%d) must be a multiple of 8 (16-byte rows of the bf16 epilogue)", n);
+namespace nob200 {
+namespace {
+int matmul_int8(const char* name, int num_tokens, const void* input, const void* weight, const void* bias,
+                const void* residual, const void* multiply, void* output, const void* weight_scale, const void* input_scale,
+                int n, int k, int use_silu, const Adapters* adapters, void* stream) {
+  NOB_REQUIRE(num_tokens > 0 && n > 0 && k > 0, "%s: sizes must be positive", name);
+  NOB_REQUIRE(input && weight && output && weight_scale && input_scale, "%s: NULL tensor", name);
+  NOB_REQUIRE(k % 16 == 0, "%s: k (%d) must be a multiple of 16 (row pitch of the TMA tiles)", name, k);
+  NOB_REQUIRE(n % 8 == 0, "%s: n (%d) must be a multiple of 8 (16-byte rows of the bf16 epilogue)", name, n);
   GemmParams params = {};
   params.weight_scale = static_cast<const float*>(weight_scale);
   params.input_scale = static_cast<const float*>(input_scale);
@@ -514,17 +628,18 @@ extern "C" int nob200_matmul_int8(int num_tokens, const void* input, const void*
   params.multiply = static_cast<const __nv_bfloat16*>(multiply);
   params.output = static_cast<__nv_bfloat16*>(output);
   params.use_silu = use_silu != 0;
-  return launch_matmul<false>("matmul_int8", num_tokens, input, weight, n, k, params, stream);
+  if (!adapters) return launch_matmul<false, false>(name, num_tokens, input, weight, n, k, params, stream);
+  if (const int rc = check_adapters(name, *adapters)) return rc;
+  return launch_matmul<false, true>(name, num_tokens, input, weight, n, k, params, stream, *adapters);
 }
 
-extern "C" int nob200_matmul_bf16(int num_tokens, const void* input, const void* weight, const void* bias,
-                                  const void* residual, const void* multiply, void* output, float output_scale, int n,
-                                  int k, int use_silu, void* stream) {
-  using namespace nob200;
-  NOB_REQUIRE(num_tokens > 0 && n > 0 && k > 0, "matmul_bf16: sizes must be positive");
-  NOB_REQUIRE(input && weight && output, "matmul_bf16: NULL tensor");
-  NOB_REQUIRE(k % 8 == 0, "matmul_bf16: k (%d) must be a multiple of 8 (row pitch of the TMA tiles)", k);
-  NOB_REQUIRE(n % 8 == 0, "matmul_bf16: n (%d) must be a multiple of 8 (16-byte rows of the bf16 epilogue)", n);
+int matmul_bf16(const char* name, int num_tokens, const void* input, const void* weight, const void* bias,
+                const void* residual, const void* multiply, void* output, float output_scale, int n, int k, int use_silu,
+                const Adapters* adapters, void* stream) {
+  NOB_REQUIRE(num_tokens > 0 && n > 0 && k > 0, "%s: sizes must be positive", name);
+  NOB_REQUIRE(input && weight && output, "%s: NULL tensor", name);
+  NOB_REQUIRE(k % 8 == 0, "%s: k (%d) must be a multiple of 8 (row pitch of the TMA tiles)", name, k);
+  NOB_REQUIRE(n % 8 == 0, "%s: n (%d) must be a multiple of 8 (16-byte rows of the bf16 epilogue)", name, n);
   GemmParams params = {};
   params.bias = static_cast<const __nv_bfloat16*>(bias);
   params.residual = static_cast<const __nv_bfloat16*>(residual);
@@ -532,5 +647,42 @@ extern "C" int nob200_matmul_bf16(int num_tokens, const void* input, const void*
   params.output = static_cast<__nv_bfloat16*>(output);
   params.output_scale = output_scale;
   params.use_silu = use_silu != 0;
-  return launch_matmul<true>("matmul_bf16", num_tokens, input, weight, n, k, params, stream);
+  if (!adapters) return launch_matmul<true, false>(name, num_tokens, input, weight, n, k, params, stream);
+  if (const int rc = check_adapters(name, *adapters)) return rc;
+  return launch_matmul<true, true>(name, num_tokens, input, weight, n, k, params, stream, *adapters);
+}
+}  // namespace
+}  // namespace nob200
+
+extern "C" int nob200_matmul_int8(int num_tokens, const void* input, const void* weight, const void* bias,
+                                  const void* residual, const void* multiply, void* output, const void* weight_scale,
+                                  const void* input_scale, int n, int k, int use_silu, void* stream) {
+  return nob200::matmul_int8("matmul_int8", num_tokens, input, weight, bias, residual, multiply, output, weight_scale,
+                             input_scale, n, k, use_silu, nullptr, stream);
+}
+
+extern "C" int nob200_matmul_int8_adapters(int num_tokens, const void* input, const void* weight, const void* bias,
+                                           const void* residual, const void* multiply, void* output,
+                                           const void* weight_scale, const void* input_scale, int n, int k, int use_silu,
+                                           const void* compressed0, const void* expansion0, int rank0,
+                                           const void* compressed1, const void* expansion1, int rank1, void* stream) {
+  const nob200::Adapters adapters{{compressed0, compressed1}, {expansion0, expansion1}, {rank0, rank1}};
+  return nob200::matmul_int8("matmul_int8_adapters", num_tokens, input, weight, bias, residual, multiply, output,
+                             weight_scale, input_scale, n, k, use_silu, &adapters, stream);
+}
+
+extern "C" int nob200_matmul_bf16(int num_tokens, const void* input, const void* weight, const void* bias,
+                                  const void* residual, const void* multiply, void* output, float output_scale, int n,
+                                  int k, int use_silu, void* stream) {
+  return nob200::matmul_bf16("matmul_bf16", num_tokens, input, weight, bias, residual, multiply, output, output_scale, n, k,
+                             use_silu, nullptr, stream);
+}
+
+extern "C" int nob200_matmul_bf16_adapters(int num_tokens, const void* input, const void* weight, const void* bias,
+                                           const void* residual, const void* multiply, void* output, int n, int k,
+                                           int use_silu, const void* compressed0, const void* expansion0, int rank0,
+                                           const void* compressed1, const void* expansion1, int rank1, void* stream) {
+  const nob200::Adapters adapters{{compressed0, compressed1}, {expansion0, expansion1}, {rank0, rank1}};
+  return nob200::matmul_bf16("matmul_bf16_adapters", num_tokens, input, weight, bias, residual, multiply, output, 1.0f, n, k,
+                             use_silu, &adapters, stream);
 }

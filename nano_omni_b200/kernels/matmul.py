@@ -19,6 +19,36 @@ from nano_omni_b200 import _lib
 from nano_omni_b200.core import Arguments, Config, DType, Kernel, MmaType, TensorDesc, Workload
 
 
+MAX_ADAPTERS = 2
+
+
+def _adapter_ranks(arguments, num_tokens: int, n: int) -> tuple[int, ...]:
+    """Ranks of the low-rank adapters multiplied inside the GEMM: (compressed [tokens, rank], expansion [n, rank]) pairs."""
+    assert len(arguments.adapters) <= MAX_ADAPTERS, f"at most {MAX_ADAPTERS} adapters"
+    for compressed, expansion in arguments.adapters:
+        assert compressed.dtype == expansion.dtype == DType.BF16
+        assert len(compressed.shape) == len(expansion.shape) == 2
+        rank = compressed.shape[1]
+        assert compressed.shape == (num_tokens, rank) and expansion.shape == (n, rank)
+        assert rank % 64 == 0, "adapter ranks must be multiples of 64"
+    return tuple(compressed.shape[1] for compressed, _ in arguments.adapters)
+
+
+def _adapter_arguments(workload) -> tuple[tuple[TensorDesc, TensorDesc], ...]:
+    return tuple(
+        (TensorDesc.empty(DType.BF16, (workload.num_tokens, rank)), TensorDesc.empty(DType.BF16, (workload.n, rank)))
+        for rank in workload.adapter_ranks
+    )
+
+
+def _adapter_operands(adapters) -> tuple:
+    """(compressed, expansion, rank) of every slot; rank 0 marks an empty one."""
+    operands = []
+    for compressed, expansion in (*adapters, *[(None, None)] * (MAX_ADAPTERS - len(adapters))):
+        operands += _lib.ptr(compressed), _lib.ptr(expansion), ctypes.c_int(0 if compressed is None else compressed.shape[1])
+    return tuple(operands)
+
+
 class MatmulInt8Workload(Workload):
     num_tokens: int = Field(gt=0)
     n: int = Field(gt=0)
@@ -27,6 +57,7 @@ class MatmulInt8Workload(Workload):
     use_residual: bool = False
     use_multiply: bool = False
     use_silu: bool = False
+    adapter_ranks: tuple[int, ...] = ()
 
 
 class MatmulInt8Config(Config):
@@ -51,6 +82,7 @@ class MatmulInt8Arguments(Arguments):
     weight_scale: TensorDesc
     input_scale: TensorDesc
     use_silu: bool
+    adapters: tuple[tuple[TensorDesc, TensorDesc], ...] = ()
 
     def dynamic_parameters(self) -> tuple[tuple[str, int], ...]:
         return (("num_tokens", self.input.shape[0]),)
@@ -59,6 +91,10 @@ class MatmulInt8Arguments(Arguments):
 class MatmulInt8Kernel(Kernel[MatmulInt8Arguments, MatmulInt8Workload, MatmulInt8Config]):
     name = "matmul_int8"
     symbol = "nob200_matmul_int8"
+
+    @classmethod
+    def bound_symbol(cls):
+        return _lib.symbol(cls.symbol), _lib.symbol(cls.symbol + "_adapters")
 
     @classmethod
     def make_arguments(cls, workload: MatmulInt8Workload) -> MatmulInt8Arguments:
@@ -73,6 +109,7 @@ class MatmulInt8Kernel(Kernel[MatmulInt8Arguments, MatmulInt8Workload, MatmulInt
             TensorDesc.empty(DType.F32, (workload.n, 1)),
             TensorDesc.empty(DType.F32, (workload.num_tokens,)),
             workload.use_silu,
+            _adapter_arguments(workload),
         )
 
     @classmethod
@@ -104,20 +141,27 @@ class MatmulInt8Kernel(Kernel[MatmulInt8Arguments, MatmulInt8Workload, MatmulInt
             use_residual=arguments.residual is not None,
             use_multiply=arguments.multiply is not None,
             use_silu=arguments.use_silu,
+            adapter_ranks=_adapter_ranks(arguments, num_tokens, n),
         )
 
     @classmethod
     def tops(cls, arguments: MatmulInt8Arguments) -> dict[MmaType, int]:
         workload = cls.make_workload(arguments)
-        return {MmaType.I8I8I32: 2 * workload.num_tokens * workload.n * workload.k}
+        work = {MmaType.I8I8I32: 2 * workload.num_tokens * workload.n * workload.k}
+        if workload.adapter_ranks:
+            work[MmaType.BF16BF16F32] = 2 * workload.num_tokens * workload.n * sum(workload.adapter_ranks)
+        return work
 
     def _launch(self, function, stream: int) -> int:
         a, w = self.arguments, self.workload
-        return function(
+        common = (
             ctypes.c_int(w.num_tokens), _lib.ptr(a.input), _lib.ptr(a.weight), _lib.ptr(a.bias), _lib.ptr(a.residual),
             _lib.ptr(a.multiply), _lib.ptr(a.output), _lib.ptr(a.weight_scale), _lib.ptr(a.input_scale),
-            ctypes.c_int(w.n), ctypes.c_int(w.k), ctypes.c_int(int(a.use_silu)), ctypes.c_void_p(stream),
+            ctypes.c_int(w.n), ctypes.c_int(w.k), ctypes.c_int(int(a.use_silu)),
         )  # fmt: skip
+        if not a.adapters:
+            return function[0](*common, ctypes.c_void_p(stream))
+        return function[1](*common, *_adapter_operands(a.adapters), ctypes.c_void_p(stream))
 
 
 # ------------------------------------------------------------------ bf16 GEMM (bf16 projections, LoRA products)
@@ -130,6 +174,7 @@ class MatmulBf16Workload(Workload):
     use_multiply: bool = False
     use_silu: bool = False
     output_scale: float = Field(default=1.0, allow_inf_nan=False)
+    adapter_ranks: tuple[int, ...] = ()
 
 
 @dataclasses.dataclass(frozen=True, slots=True)
@@ -142,6 +187,7 @@ class MatmulBf16Arguments(Arguments):
     output: TensorDesc
     output_scale: float | int
     use_silu: bool
+    adapters: tuple[tuple[TensorDesc, TensorDesc], ...] = ()
 
     def dynamic_parameters(self) -> tuple[tuple[str, int], ...]:
         return (("num_tokens", self.input.shape[0]),)
@@ -152,6 +198,10 @@ class MatmulBf16Kernel(Kernel[MatmulBf16Arguments, MatmulBf16Workload, MatmulInt
 
     name = "matmul_bf16"
     symbol = "nob200_matmul_bf16"
+
+    @classmethod
+    def bound_symbol(cls):
+        return _lib.symbol(cls.symbol), _lib.symbol(cls.symbol + "_adapters")
 
     @classmethod
     def make_arguments(cls, workload: MatmulBf16Workload) -> MatmulBf16Arguments:
@@ -165,6 +215,7 @@ class MatmulBf16Kernel(Kernel[MatmulBf16Arguments, MatmulBf16Workload, MatmulInt
             TensorDesc.empty(DType.BF16, wide),
             workload.output_scale,
             workload.use_silu,
+            _adapter_arguments(workload),
         )
 
     @classmethod
@@ -186,6 +237,8 @@ class MatmulBf16Kernel(Kernel[MatmulBf16Arguments, MatmulBf16Workload, MatmulInt
             if operand is not None:
                 assert operand.dtype == DType.BF16 and operand.shape == (num_tokens, n)
         assert k % 8 == 0 and n % 8 == 0, "k and n must be multiples of 8"
+        ranks = _adapter_ranks(arguments, num_tokens, n)
+        assert not ranks or arguments.output_scale == 1, "adapters come with an output scale of one"
         return MatmulBf16Workload(
             num_tokens=num_tokens,
             n=n,
@@ -195,20 +248,24 @@ class MatmulBf16Kernel(Kernel[MatmulBf16Arguments, MatmulBf16Workload, MatmulInt
             use_multiply=arguments.multiply is not None,
             use_silu=arguments.use_silu,
             output_scale=float(arguments.output_scale),
+            adapter_ranks=ranks,
         )
 
     @classmethod
     def tops(cls, arguments: MatmulBf16Arguments) -> dict[MmaType, int]:
         workload = cls.make_workload(arguments)
-        return {MmaType.BF16BF16F32: 2 * workload.num_tokens * workload.n * workload.k}
+        return {MmaType.BF16BF16F32: 2 * workload.num_tokens * workload.n * (workload.k + sum(workload.adapter_ranks))}
 
     def _launch(self, function, stream: int) -> int:
         a, w = self.arguments, self.workload
-        return function(
+        common = (
             ctypes.c_int(w.num_tokens), _lib.ptr(a.input), _lib.ptr(a.weight), _lib.ptr(a.bias), _lib.ptr(a.residual),
-            _lib.ptr(a.multiply), _lib.ptr(a.output), ctypes.c_float(w.output_scale), ctypes.c_int(w.n),
-            ctypes.c_int(w.k), ctypes.c_int(int(a.use_silu)), ctypes.c_void_p(stream),
+            _lib.ptr(a.multiply), _lib.ptr(a.output),
         )  # fmt: skip
+        shape = ctypes.c_int(w.n), ctypes.c_int(w.k), ctypes.c_int(int(a.use_silu))
+        if not a.adapters:
+            return function[0](*common, ctypes.c_float(w.output_scale), *shape, ctypes.c_void_p(stream))
+        return function[1](*common, *shape, *_adapter_operands(a.adapters), ctypes.c_void_p(stream))
 
 
 # ------------------------------------------------------------------ row-wise int8 activations

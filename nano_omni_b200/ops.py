@@ -47,6 +47,7 @@ from nano_omni_b200.kernels.dense_int8_fp8 import (
 )
 from nano_omni_b200.kernels.dense_nvfp4 import DenseNvfp4Arguments, DenseNvfp4Config, DenseNvfp4Kernel
 from nano_omni_b200.kernels.matmul import (
+    MAX_ADAPTERS,
     ConvRotInt8Arguments,
     ConvRotInt8Kernel,
     Int8RowwiseArguments,
@@ -111,12 +112,13 @@ class PreparedInput:
     _quantized: dict = dataclasses.field(default_factory=dict, init=False, repr=False)
     _compressed: dict = dataclasses.field(default_factory=dict, init=False, repr=False)
 
-    def compress(self, name: str, weight: TensorDesc) -> TensorDesc:
-        if weight not in self._compressed:
+    def compress(self, name: str, weight: TensorDesc, scale: float = 1.0) -> TensorDesc:
+        key = weight, scale
+        if key not in self._compressed:
             output = self.sequence.temporary(f"{name}.down", DType.BF16, (self.input.shape[0], weight.shape[0]))
-            self.sequence.emit(MatmulBf16Kernel, MatmulBf16Arguments(self.input, weight, None, None, None, output, 1.0, False))
-            self._compressed[weight] = output
-        return self._compressed[weight]
+            self.sequence.emit(MatmulBf16Kernel, MatmulBf16Arguments(self.input, weight, None, None, None, output, scale, False))
+            self._compressed[key] = output
+        return self._compressed[key]
 
     def quantize(self, name: str, dtype: DType, input_scale: TensorDesc | None, rotation_group: int):
         if dtype != DType.I8:
@@ -159,8 +161,13 @@ class KernelSequence:
                use_silu: bool = False, loras: tuple[tuple[TensorDesc, TensorDesc, float], ...] = (),
                rotation_group: int = 0) -> None:  # fmt: skip
         """Emit a projection (ops/matmul/sequence.py:141-235): every LoRA pair adds
-        ``strength * (input x down^T) x up^T`` through the residual chain, in order, before the main GEMM;
-        bf16 and int8 weights (int8 needs a weight-scale tensor; the activations are quantised once per input)."""
+        ``strength * (input x down^T) x up^T``; bf16 and int8 weights (int8 needs a weight-scale tensor; the activations
+        are quantised once per input).
+
+        The last two pairs of a rank that is a multiple of 64 (a 128-byte chunk of the GEMM's K loop) are multiplied inside
+        the main GEMM, with the strength in the compressed activations; the others update the residual, in order, in
+        GEMMs of their own: a rank-64 update reads and writes the whole output (95 us at 15104 x 5376; the
+        projection with its pair 664 us so, 604 with the pair inside)."""
         prepared = input if isinstance(input, PreparedInput) else self.prepare(input)
         if prepared.sequence is not self:
             raise ValueError("prepared input belongs to a different kernel sequence")
@@ -171,18 +178,28 @@ class KernelSequence:
             raise ValueError("linear output shape or dtype mismatch")
         if weight.dtype == DType.I8 and not isinstance(weight_scale, TensorDesc):
             raise TypeError("INT8 linear requires a weight_scale buffer")
+        inside = [index for index, (down, _, _) in enumerate(loras) if down.shape[0] % 64 == 0][-MAX_ADAPTERS:]
+        adapters = []
         for index, (down, up, strength) in enumerate(loras):
+            if index in inside:
+                adapters.append((prepared.compress(f"{name}.lora{index}", down, strength), up))
+                continue
             compressed = prepared.compress(f"{name}.lora{index}", down)
             update = self.temporary(f"{name}.lora{index}.up", DType.BF16, output.shape)
             self.emit(MatmulBf16Kernel, MatmulBf16Arguments(compressed, up, None, residual, None, update, strength, False))
             residual = update
         if weight.dtype == DType.BF16:
-            self.emit(MatmulBf16Kernel, MatmulBf16Arguments(source, weight, bias, residual, multiply, output, 1.0, use_silu))
+            self.emit(
+                MatmulBf16Kernel,
+                MatmulBf16Arguments(source, weight, bias, residual, multiply, output, 1.0, use_silu, tuple(adapters)),
+            )
         elif weight.dtype == DType.I8:
             quantized, scales = prepared.quantize(name, DType.I8, None, rotation_group)
             self.emit(
                 MatmulInt8Kernel,
-                MatmulInt8Arguments(quantized, weight, bias, residual, multiply, output, weight_scale, scales, use_silu),
+                MatmulInt8Arguments(
+                    quantized, weight, bias, residual, multiply, output, weight_scale, scales, use_silu, tuple(adapters)
+                ),
             )
         else:
             raise ValueError(f"unsupported linear weight dtype: {weight.dtype}")
