@@ -226,9 +226,8 @@ fa_fwd_sol_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       }
     } else if (warp == kMmaWarp || warp == kMmaWarp + 1) {
       // ---------------------------------------------------------- tcgen05 issuer
-      // All 32 lanes run the warp-uniform control flow; one elected lane issues (see elect_one()).  The waits on the
-      // probabilities are on every entry's chain (P stored -> PV -> next QK of the stream -> scores complete) and
-      // poll; K / V tiles were loaded long before and their waits may sleep.
+      // All 32 lanes run the warp-uniform control flow; one elected lane issues (see elect_one()).  Its waits sleep: K / V tiles
+      // were loaded long before, and scores of the stream's next entry are complete while it waits for probabilities.
       {
         constexpr uint32_t idesc_qk = umma_idesc(kDS32, kFmtS8, kFmtS8, 0, 0, kTile, kBlock);
         constexpr uint32_t idesc_pv = umma_idesc(kDF32, kFmtE4M3, kFmtE4M3, 0, 0, kTile, 128);
@@ -311,7 +310,9 @@ fa_fwd_sol_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             ok = sk >= 0;
             if (!ok) break;
           }
-          if (!(ok = warp_poll(&S.p_full[t][buffer], (e >> 1) & 1, abort_flag, status, kWaitTimeoutSoftmax))) break;
+          // asleep: the other score buffer of the stream gives it slack (60778 x 14, whole operator, 6.295 ms polling, 6.273 so;
+          // the softmax warps asleep on their scores 6.317)
+          if (!(ok = warp_rest(&S.p_full[t][buffer], (e >> 1) & 1, abort_flag, status, kWaitTimeoutSoftmax))) break;
           tc_fence_after();
           issue_pv(t, buffer, sv, e > 0);
           if (sk >= 0) issue_qk(t, buffer, sk);  // in order behind the PV that read this buffer
