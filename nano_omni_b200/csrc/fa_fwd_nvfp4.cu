@@ -39,7 +39,7 @@
 // groups.  A block that a softmax warp's query block did not select is not exponentiated: its codes are zero.
 // The result is the un-normalised numerator divided by 2688 and the state (running maximum in raw units, sum of p / 2688)
 // that nob200_sol_nvfp4_finalize consumes.
-// 32768 tokens x 24 heads, 18 % selected, whole operator: 4.18 ms with steps of 64 keys, now 3.93.
+// 32768 tokens x 24 heads, 18 % selected, whole operator: 4.18 ms with steps of 64 keys, now 3.90.
 // The maximum that P is rounded against is raised per step, as in the dense form: error of the numerator over the sum against
 // 64 bits, twelve calls of 300 to 2900 tokens, mean .09213 with steps of a block, .09217 so (the grid of e2m1 itself).
 #include <cuda.h>
@@ -346,7 +346,10 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           const int ik = 2 * u, sk = ik % kStages;
           const uint64_t a0 = t ? q_desc[1] : q_desc[0], b0 = kv_desc + sk * (kTileBytes >> 4);
           if (first && !rest(&S.kv_full[sk], full_parity(ik), kWaitTimeoutLoad)) return false;
-          if (taken && !spin(taken, taken_parity, kWaitTimeoutSoftmax)) return false;
+          // polling (dense 20011 x 24 3.571 ms, asleep 3.577) except where each group brings its own keys (sol 32768 x 24
+          // 3.926 ms polling, 3.902 asleep)
+          if (taken && !(kSol ? rest(taken, taken_parity, kWaitTimeoutSoftmax) : spin(taken, taken_parity, kWaitTimeoutSoftmax)))
+            return false;
           tc_fence_after();
           if (kSol) {
             if (elect_one()) {
