@@ -130,10 +130,12 @@ fa_fwd_sol_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     tmem_alloc(&S.tmem_base, kTmemCols);
     tmem_relinquish();
   }
+  pdl_wait();  // launched as a programmatic dependent: the set-up above overlaps the kernel before
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = S.tmem_base;
+  pdl_release();
 
   if (warp >= 8) {
     reg_dealloc<56>();
@@ -584,6 +586,5 @@ extern "C" int nob200_sol_int8_fp8_attention_d128(int num_tokens, int head_offse
     return fail(kCudaError, "sol_int8_fp8_attention_d128: cannot reserve %zu B of shared memory: %s", smem,
                 cudaGetErrorString(err));
   dim3 grid((num_tokens + kTile - 1) / kTile, heads);
-  fa_fwd_sol_i8f8_kernel<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(mq, mk, mv, params);
-  return check_launch("sol_int8_fp8_attention_d128");
+  return launch_pdl("sol_int8_fp8_attention_d128", fa_fwd_sol_i8f8_kernel, grid, kThreads, smem, stream, mq, mk, mv, params);
 }

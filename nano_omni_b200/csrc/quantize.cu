@@ -493,9 +493,11 @@ __device__ __forceinline__ size_t sf_offset(int r, int g, int groups) {
 
 // Q/K orientation: rows are tokens (padded to 128), 8 groups of 16 channels.
 __global__ void __launch_bounds__(256)
-nvfp4_prepare_rows_kernel(const __nv_bfloat16* __restrict__ src, const float* __restrict__ mean,
+nvfp4_prepare_rows_kernel(const __nv_bfloat16* src, const float* mean,
                           uint8_t* __restrict__ packed, uint8_t* __restrict__ scales, int num_tokens, int heads,
                           int padded_tokens, int hadamard, float global_scale) {
+  pdl_wait();
+  pdl_release();
   constexpr int kRows = 4;  // rows per thread: their loads are all in flight before the first is used
   const int head = blockIdx.x;  // heads fastest: CTAs in flight read whole rows of the source
   const int lane16 = threadIdx.x & 15;
@@ -507,7 +509,7 @@ nvfp4_prepare_rows_kernel(const __nv_bfloat16* __restrict__ src, const float* __
   for (int p = 0; p < kRows; ++p) {
     const int row = first_row + 16 * p;
     loaded[p] = row < num_tokens
-                    ? __ldg(reinterpret_cast<const uint4*>(src + static_cast<size_t>(row) * columns + head * 128 + ch))
+                    ? *(reinterpret_cast<const uint4*>(src + static_cast<size_t>(row) * columns + head * 128 + ch))
                     : make_uint4(0u, 0u, 0u, 0u);
   }
   float mu[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -549,9 +551,11 @@ nvfp4_prepare_rows_kernel(const __nv_bfloat16* __restrict__ src, const float* __
 // One CTA per (64-token block, head); the tile is transposed through shared memory.
 template <bool HADAMARD>
 __global__ void __launch_bounds__(256)
-nvfp4_prepare_transposed_kernel(const __nv_bfloat16* __restrict__ src, const float* __restrict__ mean,
+nvfp4_prepare_transposed_kernel(const __nv_bfloat16* src, const float* mean,
                                 uint8_t* __restrict__ packed, uint8_t* __restrict__ scales, int num_tokens, int heads,
                                 int padded_tokens, float global_scale) {
+  pdl_wait();
+  pdl_release();
   // 64 tokens x 128 channels pass through shared memory to change hands from (token, 8 channels) to (channel, 16
   // tokens).  Without the rotation the tile holds the bf16 pieces as loaded (16-byte stores, 2-byte loads, no bank
   // conflicts either way) and the mean is subtracted after the transposition; with it, rows must be centred and
@@ -568,7 +572,7 @@ nvfp4_prepare_transposed_kernel(const __nv_bfloat16* __restrict__ src, const flo
   for (int p = 0; p < 4; ++p) {
     const int token = block * 64 + p * 16 + (threadIdx.x >> 4);
     loaded[p] = token < num_tokens
-                    ? __ldg(reinterpret_cast<const uint4*>(src + static_cast<size_t>(token) * columns + head * 128 + ch))
+                    ? *(reinterpret_cast<const uint4*>(src + static_cast<size_t>(token) * columns + head * 128 + ch))
                     : make_uint4(0u, 0u, 0u, 0u);
   }
 #pragma unroll
@@ -749,22 +753,17 @@ extern "C" int nob200_nvfp4_prepare(int num_tokens, const void* source, const vo
   NOB_REQUIRE(num_tokens <= 65535 * 16, "nvfp4_prepare: %d tokens exceed the grid limit", num_tokens);
   NOB_REQUIRE(global_scale >= 0.f, "nvfp4_prepare: global_scale must be >= 0 (0 selects per-block scales only)");
   const int padded = (num_tokens + 127) / 128 * 128;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (!transpose) {
-    nvfp4_prepare_rows_kernel<<<dim3(heads, padded / 64), 256, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(source), static_cast<const float*>(mean), static_cast<uint8_t*>(quantized),
-        static_cast<uint8_t*>(scales), num_tokens, heads, padded, hadamard, global_scale);
-  } else {
-    if (hadamard)
-      nvfp4_prepare_transposed_kernel<true><<<dim3(heads, padded / 64), 256, 0, s>>>(
-          static_cast<const __nv_bfloat16*>(source), static_cast<const float*>(mean), static_cast<uint8_t*>(quantized),
-          static_cast<uint8_t*>(scales), num_tokens, heads, padded, global_scale);
-    else
-      nvfp4_prepare_transposed_kernel<false><<<dim3(heads, padded / 64), 256, 0, s>>>(
-          static_cast<const __nv_bfloat16*>(source), static_cast<const float*>(mean), static_cast<uint8_t*>(quantized),
-          static_cast<uint8_t*>(scales), num_tokens, heads, padded, global_scale);
+    return launch_pdl("nvfp4_prepare", nvfp4_prepare_rows_kernel, dim3(heads, padded / 64), 256, 0, stream,
+                      static_cast<const __nv_bfloat16*>(source), static_cast<const float*>(mean),
+                      static_cast<uint8_t*>(quantized), static_cast<uint8_t*>(scales), num_tokens, heads, padded, hadamard,
+                      global_scale);
   }
-  return check_launch("nvfp4_prepare");
+  auto* kernel = hadamard ? nvfp4_prepare_transposed_kernel<true> : nvfp4_prepare_transposed_kernel<false>;
+  return launch_pdl("nvfp4_prepare", kernel, dim3(heads, padded / 64), 256, 0, stream,
+                    static_cast<const __nv_bfloat16*>(source), static_cast<const float*>(mean),
+                    static_cast<uint8_t*>(quantized), static_cast<uint8_t*>(scales), num_tokens, heads, padded,
+                    global_scale);
 }
 
 // ------------------------------------------------- column mean, no allocation
