@@ -737,17 +737,9 @@ int launch_nvfp4(bool sol, const char* name, int num_query_tokens, int num_kv_to
   if (err != cudaSuccess)
     return fail(kCudaError, "%s: cannot reserve %zu B of shared memory: %s", name, smem, cudaGetErrorString(err));
   const dim3 grid = sol ? dim3((num_query_tokens + 2 * kTile - 1) / (2 * kTile), heads) : dim3(key_split_blocks(split, heads));
-  // A dependent launch hides the set-up and the launch itself (700 tokens x 8 heads, whole operator, 34.9 -> 27.4 us; 20011 x
-  // 24 unchanged).  A sol call of several waves is launched plainly: its CTAs, of unlike lengths, fill the SMs unevenly
-  // while the router drains (32768 x 24 3.91 ms plainly, 3.95 as a dependent).
-  int device = 0, sms = 148;
-  if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  if (sol && static_cast<long long>(grid.x) * grid.y > sms) {
-    kernel<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(mq, mk, mv, params, split);
-    rc = check_launch(name);
-  } else {
-    rc = launch_pdl(name, kernel, grid, kThreads, smem, stream, mq, mk, mv, params, split);
-  }
+  // A dependent launch hides the set-up and the launch itself: 700 tokens x 8 heads, whole operator, 34.9 -> 27.4 us, sol
+  // 4000 x 14 166.8 -> 163.5 us.  (Sol 32768 x 24 alone 3.935 -> 3.927 ms, back to back 3.92 -> 3.95.)
+  rc = launch_pdl(name, kernel, grid, kThreads, smem, stream, mq, mk, mv, params, split);
   if (rc || !split.tail_rows) return rc;
   OutRoute route = {};
   route.peer[0] = static_cast<__nv_bfloat16*>(output);
