@@ -29,19 +29,19 @@
 //
 // kSol: each query tile visits only the 64-key blocks that one of its two 64-row query blocks selects (mask u8
 // [query blocks, heads, key blocks] of 64-token blocks; key block 0 always attends), so tiles A and B walk lists of
-// their own, a list entry being one key block with a flag per query block.  A step is TWO entries, 128 keys from anywhere:
-// with the waits, hand-overs and votes of a step paid per 64 keys, 64 keys took 2600 cycles for a pair of tiles where the
-// dense form takes 3430 for 128.  Every step's score / value MMA group brings its own K / V through the ring: K as two
-// boxes of 64 rows, with the two scale atoms (channel halves) of the aligned 128-row tile that each block lies in: the
-// score MMAs have N = 64 and read the scales of an odd block two TMEM columns in (key row n of an atom sits in lane n % 32,
-// column n / 32), those of the second block copied over those of the first between their MMAs (one pipe, in order).  V
-// comes as two boxes of [channel][32 bytes] (32-byte swizzle) with the one scale atom of each block's four 16-token
-// groups.  A block that a softmax warp's query block did not select is not exponentiated: its codes are zero.
-// The result is the un-normalised numerator divided by 2688 and the state (running maximum in raw units, sum of p / 2688)
-// that nob200_sol_nvfp4_finalize consumes.
-// 32768 tokens x 24 heads, 18 % selected, whole operator: 4.18 ms with steps of 64 keys, now 3.90.
-// The maximum that P is rounded against is raised per step, as in the dense form: error of the numerator over the sum against
-// 64 bits, twelve calls of 300 to 2900 tokens, mean .09213 with steps of a block, .09217 so (the grid of e2m1 itself).
+// their own, a list entry being one key block with a flag per query block, and every score / value MMA group brings
+// its own K / V tile through the ring.  K data come as the 128-row tile that starts at the block's first token, K
+// scales as the two atoms of the aligned 128-row tile the block lies in: the score MMAs have N = 64 and read the
+// scales of an odd block two TMEM columns in (key row n of an atom sits in lane n % 32, column n / 32).  V comes as
+// [channel][64 bytes] from the block's first token on with the one scale atom of its four 16-token groups: one
+// value MMA of K = 64 per entry.  A softmax warp whose query block did not select the entry stores zero codes.
+// The running maximum is raised per 64-key block, as the reference does: the grid that P is rounded on hangs on it, and
+// raising it once per two blocks makes the error against 64 bits larger (.4 % on lists of two blocks, 1.5 % with scores
+// four times as wide, less the longer the list).  32768 tokens x 24 heads, 18 % selected, whole operator: 4.18 ms; steps of
+// two entries 3.96 ms with one raise each, 4.73 to 4.93 ms with a raise and a value MMA per entry: O moves to a new maximum
+// in between, behind the first entry's value MMA (without any rescaling of O that form takes 3.70).  The result is the un-normalised numerator
+// divided by 2688 and the state (running maximum in raw units, sum of p / 2688) that nob200_sol_nvfp4_finalize
+// consumes.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -78,7 +78,7 @@ struct __align__(1024) Shared {
   uint8_t q[2][kTileBytes];
   uint8_t kv[kStages][kTileBytes];
   uint8_t q_sf[2][kSfBytes];
-  uint8_t kv_sf[kStages][2 * kSfBytes];  // dense: the first half; sol K: the atoms of both blocks' tiles
+  uint8_t kv_sf[kStages][kSfBytes];
   uint64_t q_full;
   uint64_t kv_full[kStages];
   uint64_t kv_empty[kStages];
@@ -166,7 +166,10 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   const int unit_rows = kSol ? 2 * kTile : split.unit_rows;
   const int q0 = share.q_tile * unit_rows;
   const bool two = unit_rows > kTile && q0 + kTile < P.num_query_tokens;
-  constexpr int kKeys = kTile;  // of a step
+  // Dense: a step is a key tile of 128.  Sol: a step is one 64-key routing block of the tile's list, so that no MMA,
+  // load or exponential is spent on a neighbour block nobody selected; K and V still arrive as 128-key tiles that
+  // start at the block's first token, and the block-scaled MMAs read their first 64 keys.
+  constexpr int kKeys = kSol ? 64 : kTile;
   const int q_row_blocks = (P.num_query_tokens + kTile - 1) / kTile;  // 128-row blocks of the padded operands
   volatile uint32_t* abort_flag = &S.abort;
   uint32_t* status = P.status;
@@ -202,13 +205,9 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   const uint32_t tmem = S.tmem_base;
   pdl_release();  // the merge of the shares may be scheduled behind the last CTAs
 
-  // steps of query tile t: the key tiles of the CTA's share (dense; both tiles share each K / V tile), or pairs of entries
-  // of the tile's own list
-  auto tile_count = [&](int t) { return kSol ? (S.list_len[t] + 1) / 2 : share.kv_end - share.kv_begin; };
-  // sol: key block of half `h` of step `i`; an odd list ends with a block twice, the second selected by nobody
-  auto block_at = [&](int t, int i, int h) {
-    return static_cast<int>(S.list[t][2 * i + (h && 2 * i + 1 < S.list_len[t] ? 1 : 0)]);
-  };
+  // key tiles of query tile t: those of the CTA's share (dense; both tiles share each K / V tile), or the tile's own list
+  auto tile_count = [&](int t) { return kSol ? S.list_len[t] : share.kv_end - share.kv_begin; };
+  auto tile_at = [&](int t, int i) { return kSol ? static_cast<int>(S.list[t][i]) : share.kv_begin + i; };
   auto wait_list = [&](uint32_t bit) -> bool {
     if (!kSol) return true;
     return __all_sync(0xffffffffu, mbar_wait(&S.list_ready, 0, abort_flag, status, bit));
@@ -271,12 +270,10 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         int next_a = 0, next_b = 0;
         int issued = 0;
         for (int u = 0; u < units; ++u) {
-          const int kt = share.kv_begin + u;
-          int kb[2] = {0, 0};
+          int kt = share.kv_begin + u;
           if (kSol) {
             const int t = (next_a < n_a && (next_a <= next_b || next_b >= n_b)) ? 0 : 1;
-            const int i = t ? next_b++ : next_a++;
-            kb[0] = block_at(t, i, 0), kb[1] = block_at(t, i, 1);
+            kt = tile_at(t, t ? next_b++ : next_a++);
           }
           bool ok = true;
           for (int part = 0; part < 2 && ok; ++part) {  // K at 2u, V at 2u+1
@@ -284,20 +281,17 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             if (i >= kStages) ok = mbar_wait(&S.kv_empty[st], ((i / kStages) - 1) & 1, abort_flag, status, kWaitTimeoutRing);
             if (!ok) break;
             if (kSol) {
-              mbar_expect_tx(&S.kv_full[st], kTileBytes + (part ? 2 * 512 : 2 * kSfBytes));
-#pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                uint8_t* dst = S.kv[st] + h * (kTileBytes / 2);
-                if (part) {
-                  tma_load_3d(dst, &map_v, &S.kv_full[st], kb[h] * 32, 0, head);  // [channel][32 bytes = 64 tokens]
-                  bulk_load(S.kv_sf[st] + 512 * h, P.v_sf + (static_cast<size_t>(head) * n_kv_total * 2 + kb[h]) * 512, 512,
-                            &S.kv_full[st]);
-                } else {
-                  tma_load_3d(dst, &map_k, &S.kv_full[st], 0, kb[h] * 64, head);  // [token][64 bytes]
-                  bulk_load(S.kv_sf[st] + kSfBytes * h,
-                            P.k_sf + (static_cast<size_t>(head) * n_kv_total + (kb[h] >> 1)) * kSfBytes, kSfBytes,
-                            &S.kv_full[st]);
-                }
+              // kt is a 64-key block: data tiles from its first token on; K scales are the two atoms (channel halves)
+              // of the 128-row tile it lies in, V scales the one atom of its four 16-token groups
+              if (part) {
+                mbar_expect_tx(&S.kv_full[st], kTileBytes + 512);
+                tma_load_3d(S.kv[st], &map_v, &S.kv_full[st], kt * 32, 0, head);  // [channel][64 bytes from token 64 kt]
+                bulk_load(S.kv_sf[st], P.v_sf + (static_cast<size_t>(head) * n_kv_total * 2 + kt) * 512, 512, &S.kv_full[st]);
+              } else {
+                mbar_expect_tx(&S.kv_full[st], kTileBytes + kSfBytes);
+                tma_load_3d(S.kv[st], &map_k, &S.kv_full[st], 0, kt * 64, head);  // [token][64 bytes]
+                bulk_load(S.kv_sf[st], P.k_sf + (static_cast<size_t>(head) * n_kv_total + (kt >> 1)) * kSfBytes, kSfBytes,
+                          &S.kv_full[st]);
               }
             } else {
               mbar_expect_tx(&S.kv_full[st], kTileBytes + kSfBytes);
@@ -343,38 +337,17 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         const uint64_t kv_desc = desc + (smem_u32(S.kv[0]) >> 4);
         // S = Q_t K^T with the K tile of ring unit u; `first` reader waits for the tile and copies its scales,
         // `last` reader releases the stage
-        auto qk = [&](int t, int u, bool first, bool last, uint64_t* taken, uint32_t taken_parity, int kb0, int kb1) -> bool {
+        // `block`: the 64-key block of a sol entry (its K scales are rows 64 (block & 1) .. of the tile's atoms: two
+        // TMEM columns further on); 0 for dense
+        auto qk = [&](int t, int u, bool first, bool last, uint64_t* taken, uint32_t taken_parity, int block) -> bool {
           const int ik = 2 * u, sk = ik % kStages;
           const uint64_t a0 = t ? q_desc[1] : q_desc[0], b0 = kv_desc + sk * (kTileBytes >> 4);
           if (first && !rest(&S.kv_full[sk], full_parity(ik), kWaitTimeoutLoad)) return false;
           // polling (dense 20011 x 24 3.571 ms, asleep 3.577) except where each group brings its own keys (sol 32768 x 24
-          // 3.926 ms polling, 3.902 asleep)
+          // 4.187 ms polling, 4.175 asleep)
           if (taken && !(kSol ? rest(taken, taken_parity, kWaitTimeoutSoftmax) : spin(taken, taken_parity, kWaitTimeoutSoftmax)))
             return false;
           tc_fence_after();
-          if (kSol) {
-            if (elect_one()) {
-#pragma unroll
-              for (int h = 0; h < 2; ++h) {  // the 64 keys of a block, their scales ahead of them (same pipe, in order)
-                const uint64_t bh = b0 + h * (kTileBytes / 2 >> 4);
-                const uint32_t sf = tmem + kColSfK + 2 * ((h ? kb1 : kb0) & 1);
-                cp_scale_atom(tmem + kColSfK, smem_u32(S.kv_sf[sk]) + h * kSfBytes);
-                cp_scale_atom(tmem + kColSfK + 4, smem_u32(S.kv_sf[sk]) + h * kSfBytes + 512);
-                asm volatile(
-                    "{\n\t.reg .pred p0, p1;\n\t"
-                    "setp.ne.b32 p0, 0, 0;\n\tsetp.eq.b32 p1, 0, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], %2, %4, %1, [%6], [%8], p0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], %3, %5, %1, [%7], [%9], p1;\n\t}" ::"r"(
-                        tmem + kColS + 64 * h),
-                    "r"(idesc_for(64)), "l"(a0), "l"(a0 + 2), "l"(bh), "l"(bh + 2), "r"(tmem + kColSfQ + 8 * t),
-                    "r"(tmem + kColSfQ + 8 * t + 4), "r"(sf), "r"(sf + 4)
-                    : "memory");
-              }
-              tc_commit(&S.s_full[t]);
-              tc_commit(&S.kv_empty[sk]);
-            }
-            return true;
-          }
           if (elect_one()) {
             if (first) {  // the key tile's scales, ahead of its first MMA (same pipe, in order)
               cp_scale_atom(tmem + kColSfK, smem_u32(S.kv_sf[sk]));
@@ -386,8 +359,9 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], %2, %4, %1, [%6], [%8], p0;\n\t"
                 "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], %3, %5, %1, [%7], [%9], p1;\n\t}" ::"r"(
                     tmem + kColS),
-                "r"(kIdesc), "l"(a0), "l"(a0 + 2), "l"(b0), "l"(b0 + 2), "r"(tmem + kColSfQ + 8 * t),
-                "r"(tmem + kColSfQ + 8 * t + 4), "r"(tmem + kColSfK), "r"(tmem + kColSfK + 4)
+                "r"(idesc_for(kKeys)), "l"(a0), "l"(a0 + 2), "l"(b0), "l"(b0 + 2), "r"(tmem + kColSfQ + 8 * t),
+                "r"(tmem + kColSfQ + 8 * t + 4), "r"(tmem + kColSfK + 2 * (block & 1)),
+                "r"(tmem + kColSfK + 4 + 2 * (block & 1))
                 : "memory");
             tc_commit(&S.s_full[t]);
             if (last) tc_commit(&S.kv_empty[sk]);
@@ -409,22 +383,19 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           for (int g = 0; ok && g < groups; ++g) {
             int t, i;
             next_group(t, i);
-            ok = qk(t, g, true, true, prev_t < 0 ? nullptr : &S.s_taken[prev_t], prev_i & 1, block_at(t, i, 0),
-                    block_at(t, i, 1));
+            ok = qk(t, g, true, true, prev_t < 0 ? nullptr : &S.s_taken[prev_t], prev_i & 1, tile_at(t, i));
             prev_t = t, prev_i = i;
           }
         } else {
           const bool shared = n_b > 0;
-          ok = ok && qk(0, 0, true, !shared, nullptr, 0, 0, 0);
+          ok = ok && qk(0, 0, true, !shared, nullptr, 0, 0);
           for (int i = 0; ok && i < n_a; ++i) {
-            if (shared && !(ok = qk(1, i, false, true, &S.s_taken[0], i & 1, 0, 0))) break;
-            if (i + 1 < n_a && !(ok = qk(0, i + 1, true, !shared, &S.s_taken[shared ? 1 : 0], i & 1, 0, 0))) break;
+            if (shared && !(ok = qk(1, i, false, true, &S.s_taken[0], i & 1, 0))) break;
+            if (i + 1 < n_a && !(ok = qk(0, i + 1, true, !shared, &S.s_taken[shared ? 1 : 0], i & 1, 0))) break;
           }
         }
       } else {
-        // dense: a channel's 128 tokens are a row of 64 bytes; sol: 32 bytes in each of the two blocks' boxes
-        const uint64_t kv_desc = (kSol ? umma_smem_desc(0, 16, 256, kSwizzle32B) : desc) + (smem_u32(S.kv[0]) >> 4);
-        const uint64_t second = kSol ? kTileBytes / 2 >> 4 : 2;  // keys 64-127
+        const uint64_t kv_desc = desc + (smem_u32(S.kv[0]) >> 4);
         // O_t += P_t(i) V with the V tile of ring unit u: one MMA of K = 64 per 64 keys.  `first` reader waits for the
         // tile and copies its scales ahead of the MMAs (same pipe, in order), `last` reader releases the stage.
         auto pv = [&](int t, int i, int u, bool first, bool last) -> bool {
@@ -439,15 +410,23 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           if (elect_one()) {
             if (first) {
               cp_scale_atom(tmem + kColSfV, smem_u32(S.kv_sf[sv]));
-              cp_scale_atom(tmem + kColSfV + 4, smem_u32(S.kv_sf[sv]) + 512);
+              if (!kSol) cp_scale_atom(tmem + kColSfV + 4, smem_u32(S.kv_sf[sv]) + 512);
             }
-            asm volatile(
-                "{\n\t.reg .pred p0, p1;\n\tsetp.ne.b32 p0, %4, 0;\n\tsetp.eq.b32 p1, 0, 0;\n\t"
-                "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], [%1], %2, %3, [%5], [%6], p0;\n\t"
-                "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], [%7], %8, %3, [%9], [%10], p1;\n\t}" ::"r"(d),
-                "r"(a), "l"(b), "r"(kIdesc), "r"(i > 0 ? 1u : 0u), "r"(sf), "r"(tmem + kColSfV), "r"(a + 8), "l"(b + second),
-                "r"(sf + 4), "r"(tmem + kColSfV + 4)
-                : "memory");
+            if (kSol) {  // an entry is 64 keys: one MMA
+              asm volatile(
+                  "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                  "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], [%1], %2, %3, [%5], [%6], p;\n\t}" ::"r"(d),
+                  "r"(a), "l"(b), "r"(kIdesc), "r"(i > 0 ? 1u : 0u), "r"(sf), "r"(tmem + kColSfV)
+                  : "memory");
+            } else {
+              asm volatile(
+                  "{\n\t.reg .pred p0, p1;\n\tsetp.ne.b32 p0, %4, 0;\n\tsetp.eq.b32 p1, 0, 0;\n\t"
+                  "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], [%1], %2, %3, [%5], [%6], p0;\n\t"
+                  "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], [%7], %8, %3, [%9], [%10], p1;\n\t}" ::"r"(d),
+                  "r"(a), "l"(b), "r"(kIdesc), "r"(i > 0 ? 1u : 0u), "r"(sf), "r"(tmem + kColSfV), "r"(a + 8), "l"(b + 2),
+                  "r"(sf + 4), "r"(tmem + kColSfV + 4)
+                  : "memory");
+            }
             tc_commit(&S.pv_done[t][i & 1]);
             if (last) tc_commit(&S.kv_empty[sv]);
           }
@@ -483,20 +462,8 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       bool ok = wait_list(kWaitTimeoutLoad);
       const int n = ok ? tile_count(t) : 0;
       for (int i = 0; i < n; ++i) {
-        // keys of the step's two halves that exist and, sol, whose block this row's query block selected (warp-uniform: a warp
-        // lies inside one query block)
-        int valid[2];
-        if (kSol) {
-          const int len = S.list_len[t];
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const bool selected = 2 * i + h < len && ((S.flags[t][2 * i + h] >> quarter) & 1u) != 0;
-            valid[h] = selected ? min(64, P.num_kv_tokens - block_at(t, i, h) * 64) : 0;
-          }
-        } else {
-          const int left = P.num_kv_tokens - (share.kv_begin + i) * kKeys;
-          valid[0] = min(64, left), valid[1] = min(64, left - 64);
-        }
+        const int kt = tile_at(t, i);
+        const bool selected = !kSol || ((S.flags[t][i] >> quarter) & 1u) != 0;
         ok = poll(&S.s_full[t], i & 1, kWaitTimeoutMma);
         if (!ok) break;
         tc_fence_after();
@@ -509,18 +476,20 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         if (lane == 0) mbar_arrive(&S.s_taken[t]);
         // PV(i-2) read the P buffer of this tile: looked at early, so that the answer is there when P is stored
         const bool p_free = i < 2 || mbar_test(&S.pv_done[t][i & 1], ((i - 2) >> 1) & 1);
-        if (valid[0] + valid[1] < kKeys) {  // the others count as -inf
+        // keys that do not exist or that this row's query block did not select count as -inf
+        int hi = selected ? kKeys : 0;
+        const int valid = P.num_kv_tokens - kt * kKeys;
+        if (hi > valid) hi = valid;
+        if (hi < kKeys) {
 #pragma unroll
-          for (int e = 0; e < 64; ++e) {
-            if (e >= valid[0]) s[e] = 0xff800000u;
-            if (e >= valid[1]) s[64 + e] = 0xff800000u;
-          }
+          for (int e = 0; e < kKeys; ++e)
+            if (e >= hi) s[e] = 0xff800000u;
         }
         bool raise = false;
         float alpha = 1.f;
         uint32_t pw[kKeys / 8], sfw[kKeys / 64];
-        if (kSol && valid[0] + valid[1] == 0) {
-          // nothing of this step for this warp's rows
+        if (kSol && hi <= 0) {
+          // nothing of this tile for this warp's rows (uniform: a warp lies inside one query block)
 #pragma unroll
           for (int c = 0; c < kKeys / 8; ++c) pw[c] = 0u;
 #pragma unroll
@@ -566,37 +535,20 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
               y[g & 1][e + 1] = ex2(x1);
             }
           };
-          // groups [begin, end), the exponentials of one ahead of the packing of the one before
-          auto quantise = [&](int begin, int end) {
-            exponentials(begin);
+          exponentials(0);
 #pragma unroll
-            for (int g = begin; g < end; ++g) {
-              const float bs = ex2(fmaf(gmax[g], P.scale_log2, bias));
-              if (g + 1 < end) exponentials(g + 1);
-              const float* c = y[g & 1];
-              uint64_t sum = add2(add2(pack2(c[0], c[1]), pack2(c[2], c[3])), add2(pack2(c[4], c[5]), pack2(c[6], c[7])));
-              sum = add2(sum, add2(add2(pack2(c[8], c[9]), pack2(c[10], c[11])), add2(pack2(c[12], c[13]), pack2(c[14], c[15]))));
-              la = fma2(sum, pack2(bs, bs), la);  // the unrounded probabilities' sum: p = code value x unrounded scale
-              pw[2 * g] = pack_e2m1x8(c);
-              pw[2 * g + 1] = pack_e2m1x8(c + 8);
-              const uint32_t byte = pack_e4m3x2(bs, 0.f) & 0xffu;
-              if ((g & 3) == 0) sfw[g >> 2] = 0u;
-              sfw[g >> 2] |= byte << (8 * (g & 3));
-            }
-          };
-          if (!kSol) {
-            quantise(0, 8);
-          } else {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              if (valid[h] > 0) {
-                quantise(4 * h, 4 * h + 4);
-              } else {
-#pragma unroll
-                for (int c = 8 * h; c < 8 * h + 8; ++c) pw[c] = 0u;
-                sfw[h] = 0u;
-              }
-            }
+          for (int g = 0; g < kKeys / 16; ++g) {
+            const float bs = ex2(fmaf(gmax[g], P.scale_log2, bias));
+            if (g + 1 < kKeys / 16) exponentials(g + 1);
+            const float* c = y[g & 1];
+            uint64_t sum = add2(add2(pack2(c[0], c[1]), pack2(c[2], c[3])), add2(pack2(c[4], c[5]), pack2(c[6], c[7])));
+            sum = add2(sum, add2(add2(pack2(c[8], c[9]), pack2(c[10], c[11])), add2(pack2(c[12], c[13]), pack2(c[14], c[15]))));
+            la = fma2(sum, pack2(bs, bs), la);  // the unrounded probabilities' sum: p = code value x unrounded scale
+            pw[2 * g] = pack_e2m1x8(c);
+            pw[2 * g + 1] = pack_e2m1x8(c + 8);
+            const uint32_t byte = pack_e4m3x2(bs, 0.f) & 0xffu;
+            if ((g & 3) == 0) sfw[g >> 2] = 0u;
+            sfw[g >> 2] |= byte << (8 * (g & 3));
           }
         }
         if (!__all_sync(0xffffffffu, p_free)) {
@@ -710,12 +662,11 @@ int launch_nvfp4(bool sol, const char* name, int num_query_tokens, int num_kv_to
   if ((rc = make_tensor_map_3d(&mq, CU_TENSOR_MAP_DATA_TYPE_UINT8, query, 64, q_rows, heads, 64, q_rows * 64, 64, kTile, 1,
                                CU_TENSOR_MAP_SWIZZLE_64B)))
     return rc;
-  if ((rc = make_tensor_map_3d(&mk, CU_TENSOR_MAP_DATA_TYPE_UINT8, key, 64, k_rows, heads, 64, k_rows * 64, 64,
-                               sol ? 64 : kTile, 1, CU_TENSOR_MAP_SWIZZLE_64B)))
+  if ((rc = make_tensor_map_3d(&mk, CU_TENSOR_MAP_DATA_TYPE_UINT8, key, 64, k_rows, heads, 64, k_rows * 64, 64, kTile, 1,
+                               CU_TENSOR_MAP_SWIZZLE_64B)))
     return rc;
   if ((rc = make_tensor_map_3d(&mv, CU_TENSOR_MAP_DATA_TYPE_UINT8, value, k_rows / 2, 128, heads, k_rows / 2,
-                               k_rows / 2 * 128, sol ? 32 : 64, kTile, 1,
-                               sol ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B)))
+                               k_rows / 2 * 128, 64, kTile, 1, CU_TENSOR_MAP_SWIZZLE_64B)))
     return rc;
 
   Params params = {};

@@ -18,6 +18,7 @@ FILES = [
     "tests/test_gpu_attention_nvfp4.py",
     "tests/test_gpu_sol_attention.py",
     "tests/test_gpu_sol_exact.py",
+    "tests/test_gpu_sol_steps.py",
 ]
 
 

@@ -158,9 +158,9 @@ def test_nvfp4_exact_stage_and_finalize_match_oracle(T):
     dk = rm.nvfp4_dequantize(ops[1][0].cpu(), ops[1][1].cpu())[:, :T]
     dv = rm.nvfp4_dequantize(ops[2][0].cpu(), ops[2][1].cpu()).transpose(1, 2)[:, :T]
     # Probabilities are rounded to e2m1 with a ue4m3 scale per 16 keys relative to a running maximum that kernel and
-    # reference both raise per 64-key block; the kernel takes the union of two query blocks' lists and divides by an
-    # approximate reciprocal of the scale, so single codes may round differently.  Both are measured against
-    # unrounded probabilities: the kernel must stay within 1.5x the reference's own error.
+    # reference both raise per 64-key block; the kernel takes codes and scales from the scores, not from p, so single
+    # codes may round differently.  Both are measured against unrounded probabilities: the kernel must stay within
+    # 1.5x the reference's own error.
     want_numerator, want_state = sm.sol_exact_generic(
         dq, dk, dv, selected.cpu(), always_first_block=True, round_probability=sm.round_nvfp4_groups, probability_scale=2688.0
     )
@@ -292,9 +292,8 @@ def test_against_reference_fixtures(golden_sol):
         prepare(flat(v), h, True),
     )
     exact4, state4 = nvfp4_exact(ops4, selected, T, h)
-    # The reference rounds probabilities to e2m1 before the value product and so does the kernel, on another grid
-    # (running maximum per 128-key tile instead of per 64-key block).  Same state; numerator and final output must
-    # lie no further from the unrounded result than 1.5x the reference's.
+    # The reference rounds probabilities to e2m1 before the value product and so does the kernel, on the same schedule.
+    # Same state; numerator and final output must lie no further from the unrounded result than 1.5x the reference's.
     want_state4 = torch.from_numpy(golden_sol[f"f4_state_{tag}"])
     torch.testing.assert_close(state4.cpu(), want_state4, rtol=2e-3, atol=1e-4)
     dq = rm.nvfp4_dequantize(ops4[0][0].cpu(), ops4[0][1].cpu())[:, :T]
