@@ -102,6 +102,11 @@ from nano_omni_b200.kernels.sol_exact import (
 )
 
 
+def _ordinary(strength: float) -> bool:
+    """A strength that leaves bf16 products of the activations their range, so that it may go into them."""
+    return 2.0**-24 <= abs(strength) <= 2.0**24
+
+
 @dataclasses.dataclass(frozen=True, slots=True)
 class PreparedInput:
     """One unchanged projection input whose quantised form and LoRA compressions are shared by sibling projections
@@ -113,12 +118,30 @@ class PreparedInput:
     _compressed: dict = dataclasses.field(default_factory=dict, init=False, repr=False)
 
     def compress(self, name: str, weight: TensorDesc, scale: float = 1.0) -> TensorDesc:
-        key = weight, scale
-        if key not in self._compressed:
+        """``scale * input x weight^T``, once per weight and scale."""
+        known = self._compressed.setdefault(weight, {})
+        if scale not in known:
             output = self.sequence.temporary(f"{name}.down", DType.BF16, (self.input.shape[0], weight.shape[0]))
             self.sequence.emit(MatmulBf16Kernel, MatmulBf16Arguments(self.input, weight, None, None, None, output, scale, False))
-            self._compressed[key] = output
-        return self._compressed[key]
+            known[scale] = output
+        return known[scale]
+
+    def shared_compression(self, name: str, weight: TensorDesc, strength: float) -> tuple[TensorDesc, float]:
+        """A compression and the factor that makes it ``strength * input x weight^T``: of whichever scale is there, else a
+        new one of scale 1."""
+        for scale, output in self._compressed.get(weight, {}).items():
+            if _ordinary(strength) and _ordinary(scale):
+                return output, strength / scale
+        return self.compress(name, weight), strength
+
+    def takes_inside(self, weight: TensorDesc, scale: float, n: int) -> bool:
+        """Whether a pair is multiplied inside a GEMM of ``n`` columns, with ``scale`` in its compression.  Another scale of
+        a weight that is compressed already would read the input (2 k bytes a token) once more; the update outside
+        shares the compression and writes and reads 2 n bytes a token each: worth it where k is above 2 n (at 15104
+        tokens a compression from 7168 columns takes 43 us, an update of 5376 columns 95)."""
+        known = self._compressed.get(weight, {})
+        shared = not known or scale in known
+        return weight.shape[0] % 64 == 0 and _ordinary(scale) and (shared or self.input.shape[1] <= 2 * n)
 
     def quantize(self, name: str, dtype: DType, input_scale: TensorDesc | None, rotation_group: int):
         if dtype != DType.I8:
@@ -167,7 +190,8 @@ class KernelSequence:
         The last two pairs of a rank that is a multiple of 64 (a 128-byte chunk of the GEMM's K loop) are multiplied inside
         the main GEMM, with the strength in the compressed activations; the others update the residual, in order, in
         GEMMs of their own: a rank-64 update reads and writes the whole output (95 us at 15104 x 5376; the
-        projection with its pair 664 us so, 604 with the pair inside)."""
+        projection with its pair 664 us so, 604 with the pair inside).  Sibling projections share a compression; see
+        ``PreparedInput.takes_inside`` for pairs of one down-projection at several strengths."""
         prepared = input if isinstance(input, PreparedInput) else self.prepare(input)
         if prepared.sequence is not self:
             raise ValueError("prepared input belongs to a different kernel sequence")
@@ -178,15 +202,16 @@ class KernelSequence:
             raise ValueError("linear output shape or dtype mismatch")
         if weight.dtype == DType.I8 and not isinstance(weight_scale, TensorDesc):
             raise TypeError("INT8 linear requires a weight_scale buffer")
-        inside = [index for index, (down, _, _) in enumerate(loras) if down.shape[0] % 64 == 0][-MAX_ADAPTERS:]
+        n = weight.shape[0]
+        inside = [i for i, (down, _, strength) in enumerate(loras) if prepared.takes_inside(down, strength, n)][-MAX_ADAPTERS:]
         adapters = []
         for index, (down, up, strength) in enumerate(loras):
             if index in inside:
                 adapters.append((prepared.compress(f"{name}.lora{index}", down, strength), up))
                 continue
-            compressed = prepared.compress(f"{name}.lora{index}", down)
+            compressed, factor = prepared.shared_compression(f"{name}.lora{index}", down, strength)
             update = self.temporary(f"{name}.lora{index}.up", DType.BF16, output.shape)
-            self.emit(MatmulBf16Kernel, MatmulBf16Arguments(compressed, up, None, residual, None, update, strength, False))
+            self.emit(MatmulBf16Kernel, MatmulBf16Arguments(compressed, up, None, residual, None, update, factor, False))
             residual = update
         if weight.dtype == DType.BF16:
             self.emit(
