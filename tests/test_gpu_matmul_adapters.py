@@ -5,8 +5,10 @@ import itertools
 import pytest
 import torch
 
+from nano_omni_b200 import ops
 from nano_omni_b200.core import DType, TensorDesc
 from nano_omni_b200.kernels.matmul import MatmulBf16Arguments, MatmulBf16Kernel, MatmulInt8Arguments, MatmulInt8Kernel
+from oracle import reference_math as rm
 
 pytestmark = pytest.mark.gpu
 
@@ -68,3 +70,92 @@ def test_ranks_are_checked():
         pair = (desc(DType.BF16, (8, rank)), desc(DType.BF16, (16, rank)))
         with pytest.raises(AssertionError):
             MatmulBf16Kernel(MatmulBf16Arguments(x, w, None, None, None, out, 1.0, False, (pair,)))
+
+
+class Siblings(ops.Op):
+    """Projections of one input, each with (weight, weight scale or None, output, pairs)."""
+
+    def __init__(self, x, projections, residual):
+        desc = TensorDesc.from_torch
+        super().__init__(desc(x), outputs=())
+        self.residual = desc(residual)
+        self.projections = [
+            (desc(w), 1.0 if ws is None else desc(ws), desc(out), tuple((desc(a), desc(b), s) for a, b, s in loras))
+            for w, ws, out, loras in projections
+        ]
+
+    def kernels(self, scratch):
+        sequence = ops.KernelSequence(scratch)
+        prepared = sequence.prepare(self.inputs[0])
+        for i, (weight, scale, out, loras) in enumerate(self.projections):
+            sequence.linear(f"p{i}", prepared, weight, out, weight_scale=scale, residual=self.residual, loras=loras)
+        return sequence.calls
+
+
+# ranks and strengths of each sibling's pairs, in order, the last two of whole chunks of 64 inside; whether siblings have their
+# down-projections in common; GEMMs that are expected: compressions, updates outside and the projections themselves
+ADAPTERS = {
+    "one": ([[(64, 0.75)]], 1 + 1),
+    "two strengths": ([[(64, 0.75), (128, -1.5)]], 2 + 1),
+    "three, the last two inside": ([[(64, 2.0), (128, -0.75), (64, 0.5)]], 3 + 1 + 1),
+    "one outside beside one inside": ([[(64, -0.75), (32, 1.5)]], 2 + 1 + 1),
+    "siblings of one strength": ([[(64, 0.75)], [(64, 0.75)]], 1 + 2),
+    "siblings of two strengths": ([[(64, 0.75)], [(64, -1.5)]], 1 + 1 + 2),
+}
+
+
+@pytest.mark.parametrize("int8", [False, True])
+@pytest.mark.parametrize("name", ADAPTERS)
+def test_projections_with_adapters_against_float64(name, int8):
+    m, n, k = 300, 264, 1024
+    siblings, gemms = ADAPTERS[name]
+    g = torch.Generator(device="cuda").manual_seed(len(name))
+
+    def normal(*shape, std=1.0):
+        return (torch.randn(*shape, generator=g, device="cuda") * std).bfloat16()
+
+    x, residual = normal(m, k), normal(m, n)
+    down = {rank: normal(rank, k, std=k**-0.5) for rank in (32, 64, 128)}
+    projections = []
+    for pairs in siblings:
+        first = {rank: True for rank in down}
+        loras = []
+        for rank, strength in pairs:  # a second pair of a rank has a down-projection of its own
+            a = down[rank] if first[rank] else normal(rank, k, std=k**-0.5)
+            first[rank] = False
+            loras.append((a, normal(n, rank, std=rank**-0.5), strength))
+        if int8:
+            w = torch.randint(-127, 128, (n, k), generator=g, device="cuda", dtype=torch.int8)
+            ws = (0.5 + torch.rand(n, 1, generator=g, device="cuda")) / (73 * k**0.5)
+        else:
+            w, ws = normal(n, k, std=k**-0.5), None
+        projections.append((w, ws, torch.full((m, n), float("nan"), dtype=torch.bfloat16, device="cuda"), loras))
+    op = Siblings(x, projections, residual).to()
+    calls, need = op.prepare()
+    assert sum(c.name.startswith("matmul") for c in calls) == gemms, [c.name for c in calls]
+    op.run(torch.empty(max(need, 256), dtype=torch.uint8, device="cuda"))
+    torch.cuda.synchronize()
+    if int8:
+        quantised, scales = rm.int8_rowwise(x.cpu())
+        quantised, scales = quantised.cuda().double(), scales.cuda().double()[:, None]
+    for w, ws, out, loras in projections:
+        if int8:
+            main, size = (
+                (a @ b.T) * scales * ws.double().T for a, b in ((quantised, w.double()), (quantised.abs(), w.double().abs()))
+            )
+        else:
+            main, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+        want, size = main + residual.double(), size + residual.double().abs()
+        bound = torch.zeros_like(want)
+        for a, b, strength in loras:
+            compressed = strength * (x.double() @ a.double().T)
+            want, size = want + compressed @ b.double().T, size + compressed.abs() @ b.double().abs().T
+            # each compressed activation is rounded to bf16 once (at most 2^-8 of it), and an update outside the GEMM
+            # rounds the residual and what was added to it so far
+            bound += 2**-8 * compressed.abs() @ b.double().abs().T
+        outside = max(0, gemms - len(siblings) - len({(a.data_ptr()) for *_, ls in projections for a, _, _ in ls}))
+        bound += 2**-8 * (1.01 * want.abs() + outside * size) + 1e-5 * size
+        error = (out.double() - want).abs()
+        assert (error <= bound).all(), (name, float((error - bound).max()))
+        # typical errors lie far below that bound of the worst case: a strength dropped or taken twice does not
+        assert error.norm() < 0.006 * want.norm(), float(error.norm() / want.norm())
