@@ -152,8 +152,8 @@ __device__ __forceinline__ bool warp_poll(uint64_t* bar, uint32_t parity, volati
   }
   return true;
 }
-// Suspends in mbarrier.try_wait.  For waits with slack: a polling warp takes issue slots from the softmax warps of
-// its scheduler.
+// Suspends in mbarrier.try_wait.  For waits with slack, where a polling warp takes issue slots from the softmax warps of
+// its scheduler, and for the softmax warps' own waits in the bf16 kernels, which run at the power cap.
 __device__ __forceinline__ bool warp_rest(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag,
                                           uint32_t* status, uint32_t bit) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, bit));

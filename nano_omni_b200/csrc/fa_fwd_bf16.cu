@@ -314,8 +314,8 @@ fa_fwd_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       uint64_t la = 0ull, lb = 0ull;  // four partial row sums as two fp32 pairs
       bool ok = true;
       for (int j = 0; j < n_kv; ++j) {
-        // asleep: this kernel runs at the power cap, and a warp that polls while the tensor pipe works on its scores costs
-        // clock (32768 x 24: 11.11 ms polling, 11.02 so; 9461 x 14 from the projections 606 and 603 us)
+        // asleep: this kernel runs at the power cap, where polling costs clock; .4 to .8 % at most, as much as one run differs
+        // from the next on another GPU (32768 x 24 11.1 ms polling, 11.0 so)
         ok = warp_rest(&S.s_full[t], j & 1, abort_flag, status, kWaitTimeoutMma);
         if (!ok) break;
         if (lane == 0) TRACE(4 + warp, j, 0);

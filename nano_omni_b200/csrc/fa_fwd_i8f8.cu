@@ -223,7 +223,7 @@ fa_fwd_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           const uint32_t d = tmem + kColO + t * kTile, a = tmem + kColP + t * 64 + (j & 1) * 32;
           if (t == 0 && !rest(&S.kv_full[sv], full_parity(iv), kWaitTimeoutLoad)) return false;
           // asleep: with two P buffers there is slack, and a polling warp takes issue slots from the softmax warps of its
-          // scheduler (eight slices of 4096 x 30389 x 24 heads 8.37 ms polling, 8.29 so; the score issuer asleep as well 8.34)
+          // scheduler; .7 % (eight slices of 4096 x 30389 x 24 heads), not above what one run differs from the next on another GPU
           if (!rest(&S.p_full[t][j & 1], (j >> 1) & 1, kWaitTimeoutSoftmax)) return false;
           tc_fence_after();
           if (elect_one()) {

@@ -37,11 +37,11 @@
 // value MMA of K = 64 per entry.  A softmax warp whose query block did not select the entry stores zero codes.
 // The running maximum is raised per 64-key block, as the reference does: the grid that P is rounded on hangs on it, and
 // raising it once per two blocks makes the error against 64 bits larger (.4 % on lists of two blocks, 1.5 % with scores
-// four times as wide, less the longer the list).  32768 tokens x 24 heads, 18 % selected, whole operator: 4.18 ms; steps of
-// two entries 3.96 ms with one raise each, 4.73 to 4.93 ms with a raise and a value MMA per entry: O moves to a new maximum
-// in between, behind the first entry's value MMA (without any rescaling of O that form takes 3.70).  The result is the un-normalised numerator
-// divided by 2688 and the state (running maximum in raw units, sum of p / 2688) that nob200_sol_nvfp4_finalize
-// consumes.
+// four times as wide, less the longer the list).  32768 tokens x 24 heads, 18 % selected, whole operator: 4.17 ms; steps of
+// two entries 3.95 ms with one raise each, 4.73 to 4.93 ms with a raise and a value MMA per entry: O moves to a new maximum
+// in between, behind the first entry's value MMA (without any rescaling of O that form takes 3.70).
+// The result is the un-normalised numerator divided by 2688 and the state (running maximum in raw units, sum of p / 2688)
+// that nob200_sol_nvfp4_finalize consumes.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -343,8 +343,7 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           const int ik = 2 * u, sk = ik % kStages;
           const uint64_t a0 = t ? q_desc[1] : q_desc[0], b0 = kv_desc + sk * (kTileBytes >> 4);
           if (first && !rest(&S.kv_full[sk], full_parity(ik), kWaitTimeoutLoad)) return false;
-          // polling (dense 20011 x 24 3.571 ms, asleep 3.577) except where each group brings its own keys (sol 32768 x 24
-          // 4.187 ms polling, 4.175 asleep)
+          // polling, except where each group brings its own keys; either way within .3 % (dense 20011 x 24, sol 32768 x 24)
           if (taken && !(kSol ? rest(taken, taken_parity, kWaitTimeoutSoftmax) : spin(taken, taken_parity, kWaitTimeoutSoftmax)))
             return false;
           tc_fence_after();
@@ -404,7 +403,7 @@ fa_fwd_nvfp4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           const uint32_t d = tmem + kColO + t * kTile, a = tmem + kColP + 32 * t + 16 * (i & 1);
           const uint32_t sf = tmem + kColSfP + 16 * t + 8 * (i & 1);
           if (first && !rest(&S.kv_full[sv], full_parity(iv), kWaitTimeoutLoad)) return false;
-          // asleep: there is slack, and polling takes issue slots from the softmax warps (20011 x 24 3.58 ms polling, 3.57 so)
+          // asleep: there is slack, and polling takes issue slots from the softmax warps; within .3 % (20011 x 24)
           if (!rest(&S.p_full[t][i & 1], (i >> 1) & 1, kWaitTimeoutSoftmax)) return false;
           tc_fence_after();
           if (elect_one()) {
@@ -688,8 +687,9 @@ int launch_nvfp4(bool sol, const char* name, int num_query_tokens, int num_kv_to
   if (err != cudaSuccess)
     return fail(kCudaError, "%s: cannot reserve %zu B of shared memory: %s", name, smem, cudaGetErrorString(err));
   const dim3 grid = sol ? dim3((num_query_tokens + 2 * kTile - 1) / (2 * kTile), heads) : dim3(key_split_blocks(split, heads));
-  // A dependent launch hides the set-up and the launch itself: 700 tokens x 8 heads, whole operator, 34.9 -> 27.4 us, sol
-  // 4000 x 14 166.8 -> 163.5 us.  (Sol 32768 x 24 alone 3.935 -> 3.927 ms, back to back 3.92 -> 3.95.)
+  // A dependent launch hides the set-up and the launch itself.  With this kernel and its quantisers as dependents the
+  // dense operator of 700 tokens x 8 heads went from 34.9 to 27.2 us; with the sol kernel alone 900 x 8 goes from 68.9 to 67.4
+  // and 4000 x 14 from 171.0 to 168.5 us, 32768 x 24 from 4.168 to 4.174 ms back to back: no line between sizes is drawn.
   rc = launch_pdl(name, kernel, grid, kThreads, smem, stream, mq, mk, mv, params, split);
   if (rc || !split.tail_rows) return rc;
   OutRoute route = {};

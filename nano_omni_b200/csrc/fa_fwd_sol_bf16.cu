@@ -407,9 +407,9 @@ fa_fwd_sol_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       // One tile of scores for this row: bit i of valid[i/32] says whether column i counts.
       auto run_tile = [&](const uint32_t (&valid)[4], bool pooled_phase, int last_col) -> bool {
         const bool none_valid = (valid[0] | valid[1] | valid[2] | valid[3]) == 0u;
-        // asleep: polling beside the other stream's softmax costs more issue slots and, at the power cap, clock than the
-        // later resumption does (131072 x 24 54.25 ms polling, 53.90 so, 7310 x 14 240.0 and 238.4 us; the issuer asleep on
-        // its probabilities 55.0 ms)
+        // asleep: polling beside the other stream's softmax costs issue slots and, at the power cap, clock; .2 to .9 %
+        // (131072 x 24, 7310 x 14), hardly above what one run differs from the next (the issuer asleep on its probabilities
+        // loses 2 %)
         if (!warp_rest(&S.s_full[t], done & 1, abort_flag, status, kWaitTimeoutMma)) return false;
         tc_fence_after();
         if (none_valid) {

@@ -312,8 +312,7 @@ fa_fwd_sol_i8f8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             ok = sk >= 0;
             if (!ok) break;
           }
-          // asleep: the other score buffer of the stream gives it slack (60778 x 14, whole operator, 6.295 ms polling, 6.273 so;
-          // the softmax warps asleep on their scores 6.317)
+          // asleep: the other score buffer of the stream gives it slack; either way 6.27-6.29 ms (60778 x 14, whole operator)
           if (!(ok = warp_rest(&S.p_full[t][buffer], (e >> 1) & 1, abort_flag, status, kWaitTimeoutSoftmax))) break;
           tc_fence_after();
           issue_pv(t, buffer, sv, e > 0);

@@ -24,13 +24,14 @@
 //             order with separately rounded fp32 operations.  The residual arrives by TMA two steps ahead and the
 //             result leaves by TMA, both through the warp's own staging tiles of 32 x 32: a thread per row touches 32
 //             different lines per instruction, and that bounded the products with a short K (LoRA updates).
-// int8 15104 x 5376 x 7168 395 -> 347 us (2 N M K at the measured rate: 346), the rank-64 pair beside it 175 -> 144 us,
-// bf16 512 x 7168 x 5376 42 -> 36 us.
+// These kernels by themselves: int8 15104 x 5376 x 7168 395 -> 347 us (2 N M K at the measured rate: 354), the rank-64 pair
+// beside it 175 -> 144 us, bf16 512 x 7168 x 5376 42 -> 36 us (launched back to back; timed call by call 41.5 us).
 // Low-rank adapters (the ADAPTED form) are multiplied inside: sum_r compressed[m, r] * expansion[n, r], one more chunk of
 // K per 64 of the rank.  bf16: behind the main operands' chunks, into the same accumulator.  int8: the epilogue warps first
 // turn the int32 accumulator into scaled fp32 in place, and kind::f16 MMAs add to that, behind the first chunks of the next
 // tile so that the tensor pipe does not wait for them.  As GEMMs of their own the updates are bound by the output they read
-// and write: a rank-64 pair with 15104 x 5376 x 7168 int8 took 664 us, inside it takes 604.
+// and write: the whole operator of 15104 x 5376 x 7168 int8 with a rank-64 pair and a residual took 678 us, with the pair
+// inside it takes 614, at an error against 64 bits that is 13 to 27 % lower (one rounding to bf16 for two).
 // BN is 64 .. 256, chosen per shape by tile_width().  Every wait is bounded.
 #include <cuda.h>
 
@@ -498,8 +499,8 @@ namespace {
 // below 256 columns, the load of its 16 KiB + BN/2 x 128 bytes per SM at 64 bytes per cycle; a tile's start and end
 // count as some chunks' worth.  Wide tiles win on long calls; a call of one short wave is spread over more pairs.
 // All seven widths timed on twelve shapes (int8 and bf16, 256 to 15104 rows, rank-64 products among them): the rule takes
-// the fastest in each (512 x 7168 x 5376 bf16: 44.2 us at 224, 97.3 at 64, 46.1 at 256; 1000 x 5376 x 7168 int8: 52.2 at
-// 160, 58.4 at 256), with any constant from 0 to 4000 in place of the 1000 cycles.
+// the fastest in each (operators of the time of that comparison, 512 x 7168 x 5376 bf16: 44.2 us at 224, 97.3 at 64, 46.1 at
+// 256; 1000 x 5376 x 7168 int8: 52.2 at 160, 58.4 at 256), with any constant from 0 to 4000 in place of the 1000 cycles.
 int tile_width(int m, int n, int k_chunks, int pairs) {
   const long long m_tiles = (m + kBM - 1) / kBM;
   int best = kMaxBN;

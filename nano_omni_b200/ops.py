@@ -190,7 +190,7 @@ class KernelSequence:
         The last two pairs of a rank that is a multiple of 64 (a 128-byte chunk of the GEMM's K loop) are multiplied inside
         the main GEMM, with the strength in the compressed activations; the others update the residual, in order, in
         GEMMs of their own: a rank-64 update reads and writes the whole output (95 us at 15104 x 5376; the
-        projection with its pair 664 us so, 604 with the pair inside).  Sibling projections share a compression; see
+        projection with its pair 678 us so, 614 with the pair inside).  Sibling projections share a compression; see
         ``PreparedInput.takes_inside`` for pairs of one down-projection at several strengths."""
         prepared = input if isinstance(input, PreparedInput) else self.prepare(input)
         if prepared.sequence is not self:
